@@ -38,14 +38,6 @@
 
 namespace dg {
 
-// A tree's schedule state in the merged step (Integrator: max_acti_level, acti_counter, acti_time, and
-// this port's stamp and epoch counters), kept on the device while a run executes.
-struct TreeSched {
-	int max_acti, stamp, epoch, pad;
-	int counter[MAX_ACTI];
-	double time[MAX_ACTI];
-};
-
 // Per-tree arguments of the batched stage kernels: fixed while a run executes, except the list pointers
 // of the running level, which kb_swap exchanges as Solver::substep does, and the halt flag.
 struct TreeArgs {
@@ -261,11 +253,6 @@ __global__ void __launch_bounds__(BLOCK) kb_aux(DG_BATCH_PARAMS, int k) {
 	}
 }
 
-// Epochs of one substep in the tree's own sequence (Solver::substep): update + 1, slope + 2, the four
-// multiphase sweeps + 3 .. + 6, then the estimate, the split and the unsplit.
-template<class M>
-constexpr int EPOCH_EST = M::MULTI ? 7 : 3;
-
 template<class M>
 __global__ void __launch_bounds__(BLOCK) kb_estimate(DG_BATCH_PARAMS) {
 	DG_BATCH_PROLOGUE
@@ -359,7 +346,7 @@ public:
 template<class M>
 class Batch : public BatchBase {
 	static constexpr int D = M::D, NC = 1 << D, NF = 2 * D;
-	static constexpr int EPOCHS = EPOCH_EST<M> + 2;  // epoch numbers one substep uses per tree
+	static constexpr int EPOCHS = SUBSTEP_EPOCHS<M>;  // epoch numbers one substep uses per tree
 	static constexpr int LANES  = NF <= 4 ? 4 : 8;    // lanes per cell of the lane-group stages
 	static constexpr int HEADROOM = 2;  // levels above its finest that a tree may take on within a run
 

@@ -111,7 +111,8 @@ int dg_step_many(dg_solver **s, int n, int threads, int signal, int *force_break
 		for (int j = next++; j < n; j = next++) {
 			const int k    = order[j];
 			force_break[k] = 0;
-			status[k]      = guarded(s[k], [&] { s[k]->impl->step(signal, &force_break[k], &global_dt[k], nullptr, nullptr); });
+			status[k]      = guarded(s[k], [&] { s[k]->impl->step(signal, &force_break[k], &global_dt[k], nullptr, nullptr,
+			                                                                 threads < n ? threads : n); });
 		}
 	};
 	const int nt = threads < n ? threads : (n > 0 ? n : 1);

@@ -3,13 +3,14 @@
 #pragma once
 
 #include "../../include/dacti_gpu.h"
-#include "stages.cuh"
+#include "run.cuh"
 
 #include <cub/cub.cuh>
 
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -32,7 +33,8 @@ struct dg_error : std::runtime_error {
 class SolverBase {
 public:
 	virtual ~SolverBase() = default;
-	virtual void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user) = 0;
+	// `peers`: solvers that step at the same time on streams of their own (1: this one has the GPU)
+	virtual void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user, int peers = 1) = 0;
 	virtual long long cell_count() = 0;
 	virtual long long read_cells(int *levels, double *data, long long max_cells) = 0;
 	virtual long long read_cells_via(int *levels, double *data, long long max_cells, void *scratch, size_t bytes) = 0;
@@ -80,6 +82,9 @@ class Solver : public SolverBase {
 	Lists Ls_{};
 	Counters *d_cnt_ = nullptr;
 	Counters *h_cnt_ = nullptr;  // pinned
+	RunState *d_run_ = nullptr;  // schedule state of device-resident runs, then the grid barrier's counter
+	RunState *h_run_ = nullptr;  // pinned
+	int run_cluster_ = 0;        // blocks of a clustered run on this device (0: not asked yet)
 	void *pool_mem_  = nullptr;
 	void *spare_mem_  = nullptr;  // one field's worth of slots: target of the re-sort and gc permutations
 	size_t spare_bytes_ = 0;
@@ -189,6 +194,8 @@ public:
 		DG_CUDA(cudaMalloc(&d_cnt_, sizeof(Counters)));
 		DG_CUDA(cudaMallocHost(&h_cnt_, sizeof(Counters)));
 		DG_CUDA(cudaMemset(d_cnt_, 0, sizeof(Counters)));
+		DG_CUDA(cudaMalloc(&d_run_, sizeof(RunState) + sizeof(unsigned)));
+		DG_CUDA(cudaMallocHost(&h_run_, sizeof(RunState) + sizeof(unsigned)));
 		upload_tree(c);
 		construct();
 	}
@@ -206,6 +213,8 @@ public:
 		cudaFree(pos_mem_);
 		cudaFree(d_cnt_);
 		cudaFreeHost(h_cnt_);
+		cudaFree(d_run_);
+		cudaFreeHost(h_run_);
 		cudaFree(d_leaves_);
 		cudaFree(d_read_);
 		cudaFree(d_readlv_);
@@ -696,14 +705,16 @@ private:
 
 	void check_status() {
 		uint32_t s = h_cnt_->status & ~ST_NAN;
+		if (s & ST_BARRIER) throw dg_error(DG_ERR_CUDA, "a grid barrier of a device-resident run gave up waiting");
 		if (s & ST_CAPACITY) throw dg_error(DG_ERR_CAPACITY, "device list or pool capacity exceeded");
 		if (s & ST_DEPTH) throw dg_error(DG_ERR_DEPTH, "tree level jump deeper than supported");
 		if (s & ST_MISSING_BC) throw dg_error(DG_ERR_MISSING_BC, "face without neighbour or boundary condition");
 		if (s & ST_SPLIT_UNSPLIT) throw dg_error(DG_ERR_UNSUPPORTED, "cell both split and coarsened in one substep");
 	}
 
-	// One ACTI-level substep: impl/integrate.hpp:277-299 minus the host bookkeeping.
-	void substep(int L) {
+	// One ACTI-level substep: impl/integrate.hpp:277-299 minus the host bookkeeping. The head runs up to
+	// the indicator, the tail regrids and rebuilds the cluster's list.
+	void substep_head(int L) {
 		const int n      = h_cnt_->clu[L];
 		const double dtL = global_dt_ / (double) (1 << L);
 		ensure_scratch(n);
@@ -739,15 +750,25 @@ private:
 		if (tight) {
 			sync_counters();
 			check_status();
-			const long long need = (long long) h_cnt_->top + (long long) NC * h_cnt_->n_split + 16;
-			if (need > P_.cap) {
-				const long long want = growth_target(need, std::max(need + need / 4, (long long) P_.cap * 5 / 4));
-				grow_pool((int) std::min<long long>(want, 2000000000LL));
-				list = Ls_.clu[L];
-				ensure_scratch(n);  // the growth released the list scratch; the reassignment uses its marks
-			}
+			grow_for_splits();
 		}
-		const int gf = grid_for((long long) n * (NC + 1));
+	}
+
+	// A pool with room for the split requests that the host's counters hold.
+	void grow_for_splits() {
+		const long long need = (long long) h_cnt_->top + (long long) NC * h_cnt_->n_split + 16;
+		if (need <= P_.cap) return;
+		const long long want = growth_target(need, std::max(need + need / 4, (long long) P_.cap * 5 / 4));
+		grow_pool((int) std::min<long long>(want, 2000000000LL));
+	}
+
+	void substep_tail(int L, int n) {
+		const double dtL   = global_dt_ / (double) (1 << L);
+		int32_t *list      = Ls_.clu[L];
+		const int counterL = acti_counter_[L];
+		const int g        = grid_for(n);
+		const int gf       = grid_for((long long) n * (NC + 1));
+		ensure_scratch(n);  // a growth of the pool releases the list scratch; the reassignment uses its marks
 		run_k(DG_K_REGRID, n, [&] { k_unsplit_select<M><<<g, BLOCK, 0, st_>>>(P_, list, n, L, Ls_.unsplit, d_cnt_); });
 		run_k(DG_K_REGRID, 0, [&] {
 			k_split<M><<<gf, BLOCK, 0, st_>>>(P_, C_, &d_cnt_->n_split, Ls_.split, L, Ls_.fresh, ++epoch_, d_cnt_);
@@ -792,49 +813,208 @@ private:
 		DG_CUDA(cudaGetLastError());
 	}
 
-public:
-	// Integrator::integrate (impl/integrate.hpp:12-87)
-	void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user) override {
-		C_.signal   = signal;
-		C_.coarsen  = (n_global_ % coarsen_every_) == 0;
-		*force_break = 0;
-		const int top_seq = 1 << (MAX_ACTI - 1);
-		int seq           = 0;
+	// The end of a substep that the host ran (impl/integrate.hpp:56-67). Returns whether a NaN ends the step.
+	bool substep_end(int L) {
+		acti_counter_[L] = (acti_counter_[L] + 1) % 2;
+		acti_time_[L] += global_dt_ / (double) (1 << L);
+		flush(L);
+		sync_counters();
+		check_status();
+		n_split_total_ += h_cnt_->n_split;
+		n_unsplit_total_ += h_cnt_->n_unsplit;
+		n_substeps_++;
+		updates_ += h_cnt_->clu[L];
+		return h_cnt_->status & ST_NAN;
+	}
+
+	// The next substep of the global step (impl/integrate.hpp:25-39): sequence value `seq` and the next level
+	// index `l` to look at in it (MAX_ACTI: the next value is due). Returns the level, -1 at the step's end.
+	int next_substep(int &seq, int &l) {
 		while (true) {
-			int finest = max_acti_;
-			for (int l = MAX_ACTI - 1; l > finest; --l)
-				if (h_cnt_->clu[l] > 0) {
-					finest = l;
-					break;
-				}
-			const int stride = 1 << (MAX_ACTI - 1 - finest);
-			seq              = (seq / stride + 1) * stride;
-			if (seq > top_seq) break;
-			for (int l = 0; l < MAX_ACTI; ++l) {
-				if (seq % (1 << l) != 0) continue;
-				const int L = MAX_ACTI - l - 1;
+			if (l >= MAX_ACTI) {
+				int finest = max_acti_;
+				for (int k = MAX_ACTI - 1; k > finest; --k)
+					if (h_cnt_->clu[k] > 0) {
+						finest = k;
+						break;
+					}
+				const int stride = 1 << (MAX_ACTI - 1 - finest);
+				seq              = (seq / stride + 1) * stride;
+				if (seq > 1 << (MAX_ACTI - 1)) return -1;
+				l = 0;
+			}
+			while (l < MAX_ACTI) {
+				const int k = l++;
+				if (seq % (1 << k) != 0) continue;
+				const int L = MAX_ACTI - k - 1;
 				if (h_cnt_->clu[L] > 0 && L > max_acti_) {
 					max_acti_     = L;
 					acti_time_[L] = acti_time_[L - 1];
 				}
-				if (L > max_acti_) continue;
-				substep(L);
-				acti_counter_[L] = (acti_counter_[L] + 1) % 2;
-				const double dtL = global_dt_ / (double) (1 << L);
-				acti_time_[L] += dtL;
-				flush(L);
-				sync_counters();
-				check_status();
-				n_split_total_ += h_cnt_->n_split;
-				n_unsplit_total_ += h_cnt_->n_unsplit;
-				n_substeps_++;
-				updates_ += h_cnt_->clu[L];
-				if (h_cnt_->status & ST_NAN) {
-					*force_break = 1;
-					*global_dt   = global_dt_;
-					return;
+				if (L <= max_acti_) return L;
+			}
+		}
+	}
+
+	// ---- device-resident runs (run.cuh) ---------------------------------------------------------
+
+	// Largest cluster a run takes. Above it a substep's launches fill the GPU, and each of them has the
+	// registers and block size of its own stage, where a run has one for all: drop3d_large of perf/cases.py
+	// steps in 707 to 711 ms with this limit at 4096 to 32768 cells, 721 at 65536 and 925 at 131072, and
+	// drop3d (17 thousand cells a substep) in 243 ms at 4096, 198 at 32768, 289 without runs.
+	static constexpr int RUN_CELLS = 1 << 15;
+	// Largest cluster for which a run is one thread-block cluster (its barrier is 0.35 us, the grid's 1.3):
+	// up to about here the run of sixteen SMs is as fast as the one of all (drop2d 107 ms against 118,
+	// lax_tiny 23 against 27).
+	static constexpr int RUN_CLUSTER_CELLS = 2048;
+	// Solvers side by side from which each takes one thread-block cluster, whatever its size.
+	static constexpr int RUN_PEERS = 9;
+
+	template<bool V, class S>
+	void launch_run(const RunArgs &a, bool clustered) {
+		auto *fn = k_run<M, V, S>;
+		cudaLaunchConfig_t cfg{};
+		cudaLaunchAttribute at[1];
+		cfg.blockDim = RUN_THREADS;
+		cfg.stream   = st_;
+		cfg.attrs    = at;
+		cfg.numAttrs = 1;
+		if (clustered) {
+			DG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+			if (run_cluster_ == 0) {
+				// sixteen blocks where the device can place such a cluster, else the portable eight
+				at[0].id               = cudaLaunchAttributeClusterDimension;
+				at[0].val.clusterDim.x = 16;
+				at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+				cfg.gridDim            = 16;
+				int fit                = 0;
+				if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess) {
+					cudaGetLastError();
+					fit = 0;
 				}
-				if (fn) fn(user, L, acti_time_[L], (int) n_substeps_, dtL, h_cnt_->clu[L]);
+				run_cluster_ = fit > 0 ? 16 : 8;
+			}
+			at[0].id               = cudaLaunchAttributeClusterDimension;
+			at[0].val.clusterDim.x = run_cluster_;
+			at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+			cfg.gridDim            = run_cluster_;
+		} else {
+			int dev = 0, sms = 0;
+			DG_CUDA(cudaGetDevice(&dev));
+			DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+			at[0].id              = cudaLaunchAttributeCooperative;
+			at[0].val.cooperative = 1;
+			cfg.gridDim           = sms;
+		}
+		DG_CUDA(cudaLaunchKernelEx(&cfg, fn, a));
+		n_launches_++;
+	}
+
+	// Runs substeps from (seq, l) on the device until the global step is done or the host is needed;
+	// `most` is the largest cluster as the run starts. The host's schedule state, lists and counters are
+	// current afterwards. Returns why the run ended (RunStop); `L` is the level of an unfinished substep.
+	int run(int &seq, int &l, int &L, long long most, int peers) {
+		ensure_scratch(std::min<long long>(std::max<long long>(most + most / 2, 4096), RUN_CELLS));
+		RunState &h    = *h_run_;
+		h.sch.max_acti = max_acti_;
+		h.sch.stamp    = stamp_;
+		h.sch.epoch    = epoch_;
+		h.sch.pad      = 0;
+		std::copy(acti_counter_, acti_counter_ + MAX_ACTI, h.sch.counter);
+		std::copy(acti_time_, acti_time_ + MAX_ACTI, h.sch.time);
+		h.seq = seq;
+		h.l   = l;
+		*(unsigned *) (h_run_ + 1) = 0;
+		DG_CUDA(cudaMemcpyAsync(d_run_, h_run_, sizeof(RunState) + sizeof(unsigned), cudaMemcpyHostToDevice, st_));
+		DG_CUDA(cudaMemsetAsync(&d_cnt_->n_recv, 0, (char *) (&d_cnt_->status + 1) - (char *) &d_cnt_->n_recv, st_));
+		const bool clustered = peers >= RUN_PEERS || most <= RUN_CLUSTER_CELLS;
+		// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU
+		static std::mutex whole_gpu;
+		std::unique_lock<std::mutex> hold(whole_gpu, std::defer_lock);
+		if (!clustered) hold.lock();
+		RunArgs a{P_, C_, B_, Ls_, d_cnt_, d_run_, (unsigned *) (d_run_ + 1), global_dt_, limiter_, sigma_ ? 1 : 0,
+		          (int) std::min<long long>(scratch_cap_, RUN_CELLS), clustered ? 1 : 0};
+		if constexpr (!M::VISC) {
+			if (mixed_) launch_run<false, float>(a, clustered);
+			else launch_run<false, double>(a, clustered);
+		} else if constexpr (!M::MULTI) {
+			if (mixed_) launch_run<true, float>(a, clustered);
+			else launch_run<true, double>(a, clustered);
+		} else {
+			if (visc_ && mixed_) launch_run<true, float>(a, clustered);
+			else if (visc_) launch_run<true, double>(a, clustered);
+			else if (mixed_) launch_run<false, float>(a, clustered);
+			else launch_run<false, double>(a, clustered);
+		}
+		DG_CUDA(cudaMemcpyAsync(h_run_, d_run_, sizeof(RunState), cudaMemcpyDeviceToHost, st_));
+		sync_counters();
+		if (h_cnt_->status & ST_BARRIER) check_status();  // the run's state is not complete
+		max_acti_ = h.sch.max_acti;
+		stamp_    = h.sch.stamp;
+		epoch_    = h.sch.epoch;
+		std::copy(h.sch.counter, h.sch.counter + MAX_ACTI, acti_counter_);
+		std::copy(h.sch.time, h.sch.time + MAX_ACTI, acti_time_);
+		seq = h.seq;
+		l   = h.l;
+		L   = h.L;
+		std::copy(h.clu, h.clu + MAX_ACTI, Ls_.clu);
+		Ls_.tmp = h.tmp;
+		n_split_total_ += h.splits;
+		n_unsplit_total_ += h.unsplits;
+		updates_ += h.updates;
+		n_substeps_ += h.substeps;
+		return h.stop;
+	}
+
+public:
+	// Integrator::integrate (impl/integrate.hpp:12-87)
+	void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user, int peers = 1) override {
+		C_.signal   = signal;
+		C_.coarsen  = (n_global_ % coarsen_every_) == 0;
+		*force_break = 0;
+		// Runs on the device serve the default stage choices; the host issues a substep's stages one by one
+		// where a callback or the timing of every stage asks for it, and for clusters that fill the GPU.
+		const bool resident = !fn && !prof_ && opts_ == DG_OPT_DEFAULT;
+		int seq = 0, l = MAX_ACTI;
+		while (true) {
+			int s = seq, k = l;
+			const int next = next_substep(s, k);
+			if (next < 0) break;
+			bool broke = false;
+			if (resident && h_cnt_->clu[next] <= RUN_CELLS) {
+				long long most = 0;
+				for (int c = 0; c < MAX_ACTI; ++c)
+					if (h_cnt_->clu[c] <= RUN_CELLS) most = std::max<long long>(most, h_cnt_->clu[c]);
+				int L          = 0;
+				const int stop = run(seq, l, L, most, peers);
+				if (stop == RUN_DONE) break;
+				if (stop == RUN_LARGE) continue;
+				if (stop == RUN_STATUS) {
+					check_status();
+					broke = h_cnt_->status & ST_NAN;
+				} else {
+					// the run closed before the regrid of substep L
+					check_status();
+					const int n = h_cnt_->clu[L];
+					epoch_ += EPOCH_EST<M>;
+					grow_for_splits();
+					substep_tail(L, n);
+					broke = substep_end(L);
+				}
+			} else {
+				seq         = s;
+				l           = k;
+				const int n = h_cnt_->clu[next];
+				substep_head(next);
+				substep_tail(next, n);
+				broke = substep_end(next);
+				if (!broke && fn)
+					fn(user, next, acti_time_[next], (int) n_substeps_, global_dt_ / (double) (1 << next), h_cnt_->clu[next]);
+			}
+			if (broke) {
+				*force_break = 1;
+				*global_dt   = global_dt_;
+				return;
 			}
 		}
 		n_global_++;

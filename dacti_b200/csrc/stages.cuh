@@ -22,17 +22,21 @@ constexpr int SLOPE_THREADS = 128, SLOPE_MIN_BLOCKS = 5;
 __device__ __forceinline__ int gtid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int gstride() { return gridDim.x * blockDim.x; }
 
-// Thread index and grid stride of the grid-stride loops of the stage bodies: the launch's own grid, or
-// (batched trees) the range of blocks a launch gives one tree.
+// Which warp-sized work items a warp of a stage takes: items [begin, end) in steps of step(). A launch of
+// its own walks the whole grid; a batched launch gives each tree a range of blocks.
 struct PlainGrid {
-	__device__ __forceinline__ int tid() const { return blockIdx.x * blockDim.x + threadIdx.x; }
-	__device__ __forceinline__ int stride() const { return gridDim.x * blockDim.x; }
+	__device__ __forceinline__ int begin(int) const { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
+	__device__ __forceinline__ int end(int items) const { return items; }
+	__device__ __forceinline__ int step() const { return (gridDim.x * blockDim.x) >> 5; }
 };
 struct BlockRange {
 	int first, count;  // blocks [first, first + count) of the launch
-	__device__ __forceinline__ int tid() const { return ((int) blockIdx.x - first) * blockDim.x + threadIdx.x; }
-	__device__ __forceinline__ int stride() const { return count * blockDim.x; }
+	__device__ __forceinline__ int begin(int) const { return (((int) blockIdx.x - first) * blockDim.x + threadIdx.x) >> 5; }
+	__device__ __forceinline__ int end(int items) const { return items; }
+	__device__ __forceinline__ int step() const { return (count * blockDim.x) >> 5; }
 };
+// Items of n cells at `per` cells a warp.
+__device__ __forceinline__ int warp_items(int n, int per) { return (n + per - 1) / per; }
 
 __device__ __forceinline__ void append(int32_t *list, int *count, int value, int cap, uint32_t *status) {
 	int pos = atomicAdd(count, 1);
@@ -60,7 +64,7 @@ __device__ __forceinline__ void load_face_rec(const Pool &P, int i, int dim, S *
 	double a[2 * E];
 #pragma unroll
 	for (int k = 0; k < E; ++k) {
-		const double2 v = __ldg(r + k);
+		const double2 v = r[k];
 		a[2 * k] = v.x, a[2 * k + 1] = v.y;
 	}
 #pragma unroll
@@ -68,13 +72,13 @@ __device__ __forceinline__ void load_face_rec(const Pool &P, int i, int dim, S *
 	const double2 *sr = r + (R::S0 + dim * R::ES) / 2;
 #pragma unroll
 	for (int k = 0; k < R::ES / 2; ++k) {
-		const double2 v = __ldg(sr + k);
+		const double2 v = sr[k];
 		if (2 * k < E) sl[2 * k] = (S) v.x;
 		if (2 * k + 1 < E) sl[2 * k + 1] = (S) v.y;
 	}
 	if constexpr (M::MULTI) {
 		const double *kr = rec_of(P, i, R::W) + R::K0;
-		kap = (S) __ldg(kr);
+		kap = (S) *kr;
 		nrm = (S) pick<0, M::D>(kr + 1, dim);
 	}
 }
@@ -97,7 +101,11 @@ __device__ __forceinline__ void write_rec_k(const Pool &P, int i) {
 
 template<class M, class Grid>
 __device__ __forceinline__ void d_rec_k(const Grid &g, const Pool &P, const int32_t *list, int n) {
-	for (int tid = g.tid(); tid < n; tid += g.stride()) write_rec_k<M>(P, list[tid]);
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid < n) write_rec_k<M>(P, list[tid]);
+	}
 }
 template<class M>
 __global__ void k_rec_k(Pool P, const int32_t *list, int n) {
@@ -324,9 +332,9 @@ __device__ __forceinline__ void d_flux_receive(const Grid &g, const Pool &P, con
 	const int cap    = P.cap;
 	const int lane   = threadIdx.x & 31;
 	const int sub    = lane & (G - 1);
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot = wbase + lane / G;
 		double acc[M::F];
 #pragma unroll
@@ -394,9 +402,9 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
 	const int sub    = lane - grp * G;
 	const int base   = grp * G;
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot    = wbase + grp;
 		const bool active = grp < GW && slot < n;
 		double acc[F];
@@ -687,8 +695,9 @@ __device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Con
 	const int cap  = P.cap;
 	const int lane = threadIdx.x & 31;
 	// warp-uniform loop: the whole warp stamps the updated cells' ancestors together
-	for (int t0 = g.tid() - lane; t0 < n; t0 += g.stride()) {
-		const int tid = t0 + lane;
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + lane;
 		int up        = 0;
 		if (tid < n) {
 			const int i  = list[tid];
@@ -815,9 +824,9 @@ __device__ __forceinline__ void d_slope(const Grid &g, const Pool &P, const Cons
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
 	const int sub    = lane - grp * G;
 	const int base   = grp * G;
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot    = wbase + grp;
 		const bool active = grp < GW && slot < n;
 		const int i       = active ? list[slot] : 0;
@@ -957,9 +966,9 @@ __device__ __forceinline__ void d_estimate(const Grid &g, const Pool &P, const C
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
 	const int sub    = lane - grp * G;
 	const int base   = grp * G;
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot    = wbase + grp;
 		const bool active = grp < GW && slot < n;
 		const int i       = active ? list[slot] : 0;
@@ -1055,25 +1064,32 @@ __global__ void __launch_bounds__(BLOCK) k_estimate(Pool P, Consts C, const int3
 
 // A parent coarsens when all its children are coarsening candidates of this cluster
 // (impl/adaptive_refinement.hpp:198-209); the first child decides.
+template<class M>
+__device__ __forceinline__ bool unsplit_selected(const Pool &P, int i, int L, int &par, Counters *cnt) {
+	const int cap = P.cap;
+	if (!(P.op[i] & OP_UCAND)) return false;
+	par = P.parent[i];
+	if (P.child[par] != i) return false;
+	bool all = true;
+	for (int c = 0; c < (1 << M::D); ++c) {
+		const int ch = P.child[(size_t) c * cap + par];
+		const uint8_t o = P.op[ch];
+		if (P.clu[ch] != L || !(o & OP_UCAND)) all = false;
+		if (P.clu[ch] == L && (o & OP_SPLIT) && (o & OP_UCAND)) {
+			set_status(&cnt->status, ST_SPLIT_UNSPLIT);
+			all = false;
+		}
+	}
+	return all;
+}
 template<class M, class Grid>
 __device__ __forceinline__ void d_unsplit_select(const Grid &g, const Pool &P, const int32_t *list, int n, int L, int32_t *unsplit_list, Counters *cnt) {
-	const int cap = P.cap;
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
-		const int i = list[tid];
-		if (!(P.op[i] & OP_UCAND)) continue;
-		const int par = P.parent[i];
-		if (P.child[par] != i) continue;
-		bool all = true;
-		for (int c = 0; c < (1 << M::D); ++c) {
-			const int ch = P.child[(size_t) c * cap + par];
-			const uint8_t o = P.op[ch];
-			if (P.clu[ch] != L || !(o & OP_UCAND)) all = false;
-			if (P.clu[ch] == L && (o & OP_SPLIT) && (o & OP_UCAND)) {
-				set_status(&cnt->status, ST_SPLIT_UNSPLIT);
-				all = false;
-			}
-		}
-		if (all) append(unsplit_list, &cnt->n_unsplit, par, cap, &cnt->status);
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid >= n) continue;
+		int par;
+		if (unsplit_selected<M>(P, list[tid], L, par, cnt)) append(unsplit_list, &cnt->n_unsplit, par, P.cap, &cnt->status);
 	}
 }
 template<class M>
@@ -1094,10 +1110,10 @@ __device__ __forceinline__ void d_split(const Grid &g, const Pool &P, const Cons
 	const int lane   = threadIdx.x & 31;
 	const int c      = lane & (NC - 1);  // the child this lane sets up
 	const int lead   = lane & ~(NC - 1);
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
+	const int items  = warp_items(n, GW);
 	// one group of 2^D lanes per parent: the group's first lane allocates, every lane builds one child
-	for (int base = warp * GW; base < n; base += nwarps * GW) {
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int base    = it * GW;
 		const int slot    = base + lane / NC;
 		const bool active = slot < n;
 		const int par     = active ? split_list[slot] : 0;
@@ -1188,62 +1204,81 @@ __global__ void k_split(Pool P, Consts C, const int *n_ptr, const int32_t *split
 // Domain::unsplit with interpolated_cell (integrator/domain.hpp:150-180, 296-325): the parent takes
 // the children's mean t, u, k, t_slope and gradient (the gradient sum starts from the parent's own
 // stale gradient, as interpolated_cell does not reset it) and keeps its old slope and rhs.
+template<class M>
+__device__ __forceinline__ void unsplit_cell(const Pool &P, const Consts &C, int par, int L, int32_t *fresh, int epoch, Counters *cnt) {
+	constexpr int E = M::E, D = M::D, NC = 1 << D, G = M::G;
+	const int cap = P.cap;
+	double t = 0.0, u[E], kk[M::P > 0 ? M::P : 1], ts[G > 0 ? G : 1], gr[D * G > 0 ? D * G : 1];
+	for (int q = 0; q < E; ++q) u[q] = 0.0;
+	for (int q = 0; q < M::P; ++q) kk[q] = 0.0;
+	for (int q = 0; q < G; ++q) ts[q] = 0.0;
+	for (int q = 0; q < D * G; ++q) gr[q] = C.visc ? at(P.grad, cap, q, par) : 0.0;
+	double error = 0.0;
+	for (int c = 0; c < NC; ++c) {
+		const int ch = P.child[(size_t) c * cap + par];
+		t += P.t[ch];
+		for (int q = 0; q < E; ++q) u[q] = u[q] + at(P.u, cap, q, ch);
+		for (int q = 0; q < M::P; ++q) kk[q] = kk[q] + at(P.k, cap, q, ch);
+		if (C.visc) {
+			for (int q = 0; q < D * G; ++q) gr[q] = gr[q] + at(P.grad, cap, q, ch);
+			for (int q = 0; q < G; ++q) ts[q] = ts[q] + at(P.tslope, cap, q, ch);
+		}
+	}
+	for (int c = 0; c < NC; ++c) {
+		const int ch = P.child[(size_t) c * cap + par];
+		error += P.err[ch];
+		P.flags[ch] |= F_GARBAGE | F_LEAF;
+	}
+	t = t / (double) NC;
+	for (int q = 0; q < G; ++q) ts[q] = ts[q] / (double) NC;
+	for (int q = 0; q < E; ++q) u[q] = u[q] / (double) NC;
+	double p[E];
+	prim_from_cons<M>(C.m, u, p);
+	for (int q = 0; q < M::P; ++q) kk[q] = kk[q] / (double) NC;
+	for (int q = 0; q < D * G; ++q) gr[q] = gr[q] / (double) NC;
+	P.t[par] = t;
+	double *rpar = rec_of(P, par, Rec<M>::W);
+	for (int q = 0; q < E; ++q) {
+		P.u[(size_t) q * cap + par] = u[q];
+		P.p[(size_t) q * cap + par] = p[q];
+		rpar[Rec<M>::P0 + q]        = p[q];
+	}
+	for (int q = 0; q < M::P; ++q) P.k[(size_t) q * cap + par] = kk[q];
+	write_rec_k<M>(P, par);
+	if (C.visc) {
+		for (int q = 0; q < G; ++q) P.tslope[(size_t) q * cap + par] = ts[q];
+		for (int q = 0; q < D * G; ++q) P.grad[(size_t) q * cap + par] = gr[q];
+	}
+	for (int q = 0; q < M::F; ++q) P.flux[(size_t) q * cap + par] = 0.0;
+	for (int f = 0; f < 2 * D; ++f) P.nbr[(size_t) f * cap + par] = 0;
+	P.err[par]   = error;
+	P.flags[par] = (P.flags[par] | F_LEAF | F_ACTIVE | F_CAN_SPLIT) & ~F_GARBAGE;
+	P.acti[par]  = (int8_t) L;
+	P.clu[par]   = (int8_t) L;
+	append(fresh, &cnt->n_new, par, cap, &cnt->status);
+	mark_up(P, P.parent[par], epoch);
+}
 template<class M, class Grid>
 __device__ __forceinline__ void d_unsplit(const Grid &g, const Pool &P, const Consts &C, const int *n_ptr, const int32_t *unsplit_list, int L, int32_t *fresh, int epoch, Counters *cnt) {
-	constexpr int E = M::E, D = M::D, NC = 1 << D, G = M::G;
-	const int n   = *n_ptr;
-	const int cap = P.cap;
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
-		const int par = unsplit_list[tid];
-		double t = 0.0, u[E], kk[M::P > 0 ? M::P : 1], ts[G > 0 ? G : 1], gr[D * G > 0 ? D * G : 1];
-		for (int q = 0; q < E; ++q) u[q] = 0.0;
-		for (int q = 0; q < M::P; ++q) kk[q] = 0.0;
-		for (int q = 0; q < G; ++q) ts[q] = 0.0;
-		for (int q = 0; q < D * G; ++q) gr[q] = C.visc ? at(P.grad, cap, q, par) : 0.0;
-		double error = 0.0;
-		for (int c = 0; c < NC; ++c) {
-			const int ch = P.child[(size_t) c * cap + par];
-			t += P.t[ch];
-			for (int q = 0; q < E; ++q) u[q] = u[q] + at(P.u, cap, q, ch);
-			for (int q = 0; q < M::P; ++q) kk[q] = kk[q] + at(P.k, cap, q, ch);
-			if (C.visc) {
-				for (int q = 0; q < D * G; ++q) gr[q] = gr[q] + at(P.grad, cap, q, ch);
-				for (int q = 0; q < G; ++q) ts[q] = ts[q] + at(P.tslope, cap, q, ch);
-			}
+	const int n     = *n_ptr;
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid < n) unsplit_cell<M>(P, C, unsplit_list[tid], L, fresh, epoch, cnt);
+	}
+}
+// Selection and coarsening in one pass over the cluster's cells, as one stage of a fused substep: a
+// family's decision reads only its own cells, and coarsening it writes nothing another family reads.
+template<class M, class Grid>
+__device__ __forceinline__ void d_coarsen(const Grid &g, const Pool &P, const Consts &C, const int32_t *list, int n, int L, int32_t *fresh, int epoch, Counters *cnt) {
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		int par;
+		if (tid < n && unsplit_selected<M>(P, list[tid], L, par, cnt)) {
+			atomicAdd(&cnt->n_unsplit, 1);
+			unsplit_cell<M>(P, C, par, L, fresh, epoch, cnt);
 		}
-		for (int c = 0; c < NC; ++c) {
-			const int ch = P.child[(size_t) c * cap + par];
-			error += P.err[ch];
-			P.flags[ch] |= F_GARBAGE | F_LEAF;
-		}
-		t = t / (double) NC;
-		for (int q = 0; q < G; ++q) ts[q] = ts[q] / (double) NC;
-		for (int q = 0; q < E; ++q) u[q] = u[q] / (double) NC;
-		double p[E];
-		prim_from_cons<M>(C.m, u, p);
-		for (int q = 0; q < M::P; ++q) kk[q] = kk[q] / (double) NC;
-		for (int q = 0; q < D * G; ++q) gr[q] = gr[q] / (double) NC;
-		P.t[par] = t;
-		double *rpar = rec_of(P, par, Rec<M>::W);
-		for (int q = 0; q < E; ++q) {
-			P.u[(size_t) q * cap + par] = u[q];
-			P.p[(size_t) q * cap + par] = p[q];
-			rpar[Rec<M>::P0 + q]        = p[q];
-		}
-		for (int q = 0; q < M::P; ++q) P.k[(size_t) q * cap + par] = kk[q];
-		write_rec_k<M>(P, par);
-		if (C.visc) {
-			for (int q = 0; q < G; ++q) P.tslope[(size_t) q * cap + par] = ts[q];
-			for (int q = 0; q < D * G; ++q) P.grad[(size_t) q * cap + par] = gr[q];
-		}
-		for (int q = 0; q < M::F; ++q) P.flux[(size_t) q * cap + par] = 0.0;
-		for (int f = 0; f < 2 * D; ++f) P.nbr[(size_t) f * cap + par] = 0;
-		P.err[par]   = error;
-		P.flags[par] = (P.flags[par] | F_LEAF | F_ACTIVE | F_CAN_SPLIT) & ~F_GARBAGE;
-		P.acti[par]  = (int8_t) L;
-		P.clu[par]   = (int8_t) L;
-		append(fresh, &cnt->n_new, par, cap, &cnt->status);
-		mark_up(P, P.parent[par], epoch);
 	}
 }
 template<class M>
@@ -1342,15 +1377,15 @@ __device__ __forceinline__ void d_nbr_fresh(const Grid &g, const Pool &P, const 
 	const int cap    = P.cap;
 	const int lane   = threadIdx.x & 31;
 	const int sub    = lane & (G - 1);
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
+	const int items  = warp_items(n, GW);
 	auto queue = [&](int i, int f) {
 		const int nb = P.nbr[(size_t) f * cap + i];
 		if (nb != 0 && ((P.flags[nb] & F_ACTIVE) || !(P.flags[nb] & F_LEAF))) {
 			if (atomicOr(&P.fmask[nb], 1u << (f ^ 1)) == 0) append(upd, &cnt->n_upd, nb, cap, &cnt->status);
 		}
 	};
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot = wbase + lane / G;
 		if (slot >= n || sub >= NF) continue;
 		const int i       = fresh[slot];
@@ -1377,9 +1412,9 @@ __device__ __forceinline__ void d_nbr_list(const Grid &g, const Pool &P, const C
 	const int n      = *n_ptr;
 	const int lane   = threadIdx.x & 31;
 	const int sub    = lane & (G - 1);
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot = wbase + lane / G;
 		const bool act = slot < n && sub < NF;
 		const int x      = act ? list[slot] : 0;
@@ -1402,44 +1437,51 @@ __global__ void k_nbr_list(Pool P, Consts C, const int *n_ptr, const int32_t *li
 // the rebuilt list with an atomic counter (which leaves them in the order the warps reach the counter),
 // mark them, so that an order-keeping compaction can rebuild the list in the old list's order. After the
 // Morton re-sort that keeps each cluster list in Morton order through the whole global step.
+template<class M>
+__device__ __forceinline__ bool reassign_cell(const Pool &P, const Consts &C, int i, int L, double dtL, int counter_L, const Lists &Ls, Counters *cnt) {
+	const int cap = P.cap;
+	double p[M::E];
+	load_p<M>(P, i, p);
+	const double mdt = max_delta_time<M>(C.m, p, C.size[P.level[i]]);
+	P.maxdt[i]       = mdt;
+	double cfl       = dtL / mdt;
+	const uint32_t fl = P.flags[i];
+	bool stays        = false;
+	if (!(fl & F_LEAF) || (fl & F_GARBAGE)) {
+		P.clu[i] = CLU_NONE;
+		P.op[i]  = OP_NONE;  // a node that is no leaf never looks like a coarsening candidate
+	} else if (cfl < 0.5 * C.max_cfl && counter_L == 1 && L > 0) {
+		append(Ls.buf[L - 1], &cnt->buf[L - 1], i, cap, &cnt->status);
+		cfl *= 2;
+		P.clu[i] = (int8_t) (BUF_BASE + L - 1);
+	} else if (cfl > C.max_cfl && L < MAX_ACTI - 1) {
+		const int raise = (int) log2(cfl / C.max_cfl) + 1;
+		if (L + raise < MAX_ACTI) {
+			append(Ls.clu[L + raise], &cnt->clu[L + raise], i, cap, &cnt->status);
+			P.acti[i] = (int8_t) (L + raise);
+			cfl /= (double) (1 << raise);
+			P.clu[i] = (int8_t) (L + raise);
+		} else {
+			P.clu[i] = CLU_NONE;
+		}
+	} else {
+		stays    = true;
+		P.clu[i] = (int8_t) L;
+	}
+	P.cfl[i] = cfl;
+	return stays;
+}
 template<class M, class Grid>
 __device__ __forceinline__ void d_reassign(const Grid &g, const Pool &P, const Consts &C, const int32_t *list, const int *n_ptr, int n_host, int L, double dtL, int counter_L, const Lists &Ls, Counters *cnt, uint8_t *stay = nullptr) {
-	const int n   = n_ptr ? *n_ptr : n_host;
-	const int cap = P.cap;
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
-		const int i = list[tid];
-		double p[M::E];
-		load_p<M>(P, i, p);
-		const double mdt = max_delta_time<M>(C.m, p, C.size[P.level[i]]);
-		P.maxdt[i]       = mdt;
-		double cfl       = dtL / mdt;
-		const uint32_t fl = P.flags[i];
-		if (stay) stay[tid] = 0;
-		if (!(fl & F_LEAF) || (fl & F_GARBAGE)) {
-			P.cfl[i] = cfl;
-			P.clu[i] = CLU_NONE;
-			continue;
-		}
-		if (cfl < 0.5 * C.max_cfl && counter_L == 1 && L > 0) {
-			append(Ls.buf[L - 1], &cnt->buf[L - 1], i, cap, &cnt->status);
-			cfl *= 2;
-			P.clu[i] = (int8_t) (BUF_BASE + L - 1);
-		} else if (cfl > C.max_cfl && L < MAX_ACTI - 1) {
-			const int raise = (int) log2(cfl / C.max_cfl) + 1;
-			if (L + raise < MAX_ACTI) {
-				append(Ls.clu[L + raise], &cnt->clu[L + raise], i, cap, &cnt->status);
-				P.acti[i] = (int8_t) (L + raise);
-				cfl /= (double) (1 << raise);
-				P.clu[i] = (int8_t) (L + raise);
-			} else {
-				P.clu[i] = CLU_NONE;
-			}
-		} else {
-			if (stay) stay[tid] = 1;
-			else append(Ls.tmp, &cnt->n_tmp, i, cap, &cnt->status);
-			P.clu[i] = (int8_t) L;
-		}
-		P.cfl[i] = cfl;
+	const int n     = n_ptr ? *n_ptr : n_host;
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid >= n) continue;
+		const int i      = list[tid];
+		const bool stays = reassign_cell<M>(P, C, i, L, dtL, counter_L, Ls, cnt);
+		if (stay) stay[tid] = stays;
+		else if (stays) append(Ls.tmp, &cnt->n_tmp, i, P.cap, &cnt->status);
 	}
 }
 template<class M>
@@ -1452,7 +1494,10 @@ __global__ void k_reassign(Pool P, Consts C, const int32_t *list, const int *n_p
 template<class Grid>
 __device__ __forceinline__ void d_flush(const Grid &g, const Pool &P, const int32_t *buf, const int *n_ptr, int32_t *clu_list, int *clu_count, int L, Counters *cnt) {
 	const int n = *n_ptr;
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid >= n) continue;
 		const int i = buf[tid];
 		append(clu_list, clu_count, i, P.cap, &cnt->status);
 		P.acti[i] = (int8_t) L;
@@ -1716,9 +1761,9 @@ __device__ __forceinline__ void d_smooth_alpha(const Grid &g, const Pool &P, con
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
 	const int sub    = lane - grp * G;
 	const int base   = grp * G;
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot    = wbase + grp;
 		const bool active = grp < GW && slot < n;
 		const int i       = active ? list[slot] : 0;
@@ -1749,7 +1794,10 @@ __global__ void __launch_bounds__(BLOCK) k_smooth_alpha(Pool P, Consts C, BcTabl
 
 template<class Grid>
 __device__ __forceinline__ void d_store_tmp(const Grid &g, const Pool &P, const int32_t *list, int n, int comp, const double *src) {
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid >= n) continue;
 		const int i = list[tid];
 		P.k[(size_t) comp * P.cap + i] = src[i];
 	}
@@ -1770,9 +1818,9 @@ __device__ __forceinline__ void d_normal(const Grid &g, const Pool &P, const Con
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
 	const int sub    = lane - grp * G;
 	const int base   = grp * G;
-	const int warp   = g.tid() >> 5;
-	const int nwarps = g.stride() >> 5;
-	for (int wbase = warp * GW; wbase < n; wbase += nwarps * GW) {
+	const int items  = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int wbase = it * GW;
 		const int slot    = wbase + grp;
 		const bool active = grp < GW && slot < n;
 		const int i       = active ? list[slot] : 0;
@@ -1807,7 +1855,10 @@ __global__ void __launch_bounds__(BLOCK) k_normal(Pool P, Consts C, BcTable B, c
 template<class M, class Grid>
 __device__ __forceinline__ void d_curvature(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, Counters *cnt) {
 	const int cap = P.cap;
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid >= n) continue;
 		const int i  = list[tid];
 		double kappa = 0.0;
 		for (int dim = 0; dim < M::D; ++dim) {
@@ -1828,7 +1879,10 @@ __global__ void k_curvature(Pool P, Consts C, BcTable B, const int32_t *list, in
 template<class M, class Grid>
 __device__ __forceinline__ void d_smooth_kappa(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, Counters *cnt) {
 	const int cap = P.cap;
-	for (int tid = g.tid(); tid < n; tid += g.stride()) {
+	const int items = warp_items(n, 32);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		if (tid >= n) continue;
 		const int i     = list[tid];
 		const double kc = at(P.k, cap, M::KAPPA, i);
 		const double as = at(P.k, cap, M::ALPHAS, i);
