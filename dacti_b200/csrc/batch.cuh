@@ -181,7 +181,7 @@ static __global__ void __launch_bounds__(256) kb_begin(TreeArgs *A, int n_trees,
 				s.stamp    = ++z.stamp;
 				s.epoch0   = z.epoch;
 				z.epoch += a.epochs;
-				c->n_recv = c->n_split = c->n_unsplit = c->n_new = c->n_upd = c->n_tmp = 0;
+				c->n_recv = c->n_defer = c->n_split = c->n_unsplit = c->n_new = c->n_upd = c->n_tmp = 0;
 				c->status                                                        = 0;
 			}
 		}
@@ -211,13 +211,14 @@ static __global__ void __launch_bounds__(256) kb_split_check(const TreeArgs *A, 
 template<class M, bool V, class R>
 __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS) kb_face_sum(DG_BATCH_PARAMS) {
 	DG_BATCH_PROLOGUE
-	d_face_sum<M, V, R>(g, a.P, cst, a.B, a.Ls.clu[s.L], s.n, s.L, s.dtL, s.stamp, a.Ls.recv, a.cnt);
+	d_face_sum<M, V, R>(g, a.P, cst, a.B, a.Ls.clu[s.L], s.n, s.L, s.dtL, s.stamp, a.Ls.recv, a.Ls.fresh, a.cnt);
 }
 
 template<class M, class R>
 __global__ void __launch_bounds__(BLOCK) kb_flux_receive(DG_BATCH_PARAMS) {
 	DG_BATCH_PROLOGUE_NC
 	d_flux_receive<M, R>(g, a.P, a.Ls.recv, &a.cnt->n_recv, s.L, a.cnt);
+	d_deferred<M, R>(g, a.P, a.Ls.clu[s.L], a.Ls.fresh, &a.cnt->n_defer, s.L, a.cnt);
 }
 
 template<class M, bool V>

@@ -121,6 +121,7 @@ struct Pool {
 	// Per-substep scratch outside the permuted fields:
 	double *ff;       // [slot][2D][F] flux of each owned face next to a receiver (by the owner's list position)
 	double *du;       // [slot][F] face-flux sum of each running-cluster cell (by list position)
+	int32_t *dmask;   // [slot] what a deferred cell's faces left in its slots, two bits a face (DF_*)
 	int32_t *pos;     // [cap] list position of each running-cluster cell, written by the face-sum stage
 };
 
@@ -130,6 +131,7 @@ struct Counters {
 	int buf[MAX_ACTI];
 	int top;          // next free node slot (== reference tree.size())
 	int n_recv;
+	int n_defer;      // cells with a finer neighbour, whose face sums d_deferred completes
 	int n_split;
 	int n_unsplit;
 	int n_new;        // new cluster members (children + coarsened parents)

@@ -221,14 +221,18 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 		const int32_t *list = s_ls.clu[L];
 		const int e_upd     = epoch0 + 1;
 
-		d_face_sum<M, V, S>(g, P, C, a.B, list, n, L, dtL, stamp, s_ls.recv, cnt);
+		// the list of new cells, not in use before the regrid, holds the deferred cells' positions
+		d_face_sum<M, V, S>(g, P, C, a.B, list, n, L, dtL, stamp, s_ls.recv, s_ls.fresh, cnt);
 		if (!run_barrier(a, arrivals, &s_ok)) return;
 		// the receivers are cells of slower clusters, the updated cells those of this one
+		const bool deferred = __ldcg(&cnt->n_defer) > 0;
+		if (deferred) d_deferred<M, S>(g, P, list, s_ls.fresh, &cnt->n_defer, L, cnt);
+		if (__ldcg(&cnt->n_recv) > 0) d_flux_receive<M, S>(r, P, s_ls.recv, &cnt->n_recv, L, cnt);
+		if (deferred && !run_barrier(a, arrivals, &s_ok)) return;
 		d_update<M, V>(g, P, C, list, n, dtL, e_upd, cnt);
-		d_flux_receive<M, S>(r, P, s_ls.recv, &cnt->n_recv, L, cnt);
 		if (lead && blockIdx.x == 0) cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_upd = cnt->n_tmp = 0;
 		if (!run_barrier(a, arrivals, &s_ok)) return;
-		if (lead && blockIdx.x == 0) cnt->n_recv = 0;
+		if (lead && blockIdx.x == 0) cnt->n_recv = cnt->n_defer = 0;
 		d_slope<M, V>(g, P, C, a.B, list, n, a.limiter, epoch0 + 2, cnt);
 		if constexpr (M::MULTI) {
 			// the sweeps read and write the volume fractions only, which neither slopes nor indicator touch

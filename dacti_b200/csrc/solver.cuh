@@ -412,7 +412,7 @@ public:
 		sel_mem_     = nullptr;
 		scratch_cap_ = 0;
 		DG_CUDA(cudaMalloc(&ff_mem_, sizeof(double) * M::F * NF * (size_t) want));
-		DG_CUDA(cudaMalloc(&du_mem_, sizeof(double) * M::F * (size_t) want));
+		DG_CUDA(cudaMalloc(&du_mem_, (sizeof(double) * M::F + sizeof(int32_t)) * (size_t) want));
 		// stay marks (one byte per list position, rounded to 256) followed by the temp storage of the
 		// order-keeping compaction of `want` items
 		sel_tmp_bytes_ = 0;
@@ -428,7 +428,8 @@ public:
 
 	void attach_derived() {
 		P_.ff   = ff_mem_;
-		P_.du   = du_mem_;
+		P_.du    = du_mem_;
+		P_.dmask = (int32_t *) (du_mem_ + (size_t) M::F * (size_t) scratch_cap_);
 		P_.pos  = pos_mem_;
 	}
 
@@ -671,21 +672,21 @@ private:
 			constexpr int TC = FaceTile<M>::TC;
 			const int gt = (int) std::max<long long>(1, ((long long) n + TC - 1) / TC);
 			if (mixed_) {
-				if (visc_) k_face_tile<M, true, float><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
-				else k_face_tile<M, false, float><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
+				if (visc_) k_face_tile<M, true, float><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
+				else k_face_tile<M, false, float><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
 			} else {
-				if (visc_) k_face_tile<M, true, double><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
-				else k_face_tile<M, false, double><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
+				if (visc_) k_face_tile<M, true, double><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
+				else k_face_tile<M, false, double><<<gt, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
 			}
 			return;
 		}
 		const int g = grid_threads((long long) n * G, T);
 		if (mixed_) {
-			if (visc_) k_face_sum<M, true, float><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
-			else k_face_sum<M, false, float><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
+			if (visc_) k_face_sum<M, true, float><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
+			else k_face_sum<M, false, float><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
 		} else {
-			if (visc_) k_face_sum<M, true, double><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
-			else k_face_sum<M, false, double><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, d_cnt_);
+			if (visc_) k_face_sum<M, true, double><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
+			else k_face_sum<M, false, double><<<g, T, 0, st_>>>(P_, C_, B_, list, n, L, dtL, stamp, Ls_.recv, Ls_.fresh, d_cnt_);
 		}
 	}
 
@@ -732,8 +733,8 @@ private:
 		int e_upd = 0;                       // epoch of this substep's cell update
 		run_k(DG_K_FLUX, n, [&] { launch_face_sum(list, n, L, dtL, stamp_recv); });
 		run_k(DG_K_RECV, 0, [&] {
-			if (mixed_) k_flux_receive<M, float><<<grid_for((long long) n * LPC), BLOCK, 0, st_>>>(P_, Ls_.recv, &d_cnt_->n_recv, L, d_cnt_);
-			else k_flux_receive<M, double><<<grid_for((long long) n * LPC), BLOCK, 0, st_>>>(P_, Ls_.recv, &d_cnt_->n_recv, L, d_cnt_);
+			if (mixed_) k_flux_receive<M, float><<<grid_for((long long) n * LPC), BLOCK, 0, st_>>>(P_, Ls_.recv, list, Ls_.fresh, L, d_cnt_);
+			else k_flux_receive<M, double><<<grid_for((long long) n * LPC), BLOCK, 0, st_>>>(P_, Ls_.recv, list, Ls_.fresh, L, d_cnt_);
 		});
 		run_k(DG_K_UPDATE, n, [&] {
 			e_upd = ++epoch_;

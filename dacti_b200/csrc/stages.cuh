@@ -263,59 +263,61 @@ __device__ __forceinline__ void boundary_flux(const Pool &P, const Consts &C, co
 	for (int q = 0; q < M::F; ++q) Fout[q] = (double) F[q] * area * (t1 - t0) * dirn;
 }
 
-// The c-th owner of a flux across face (dim, dir) of cell i at this substep (impl/flux.hpp:58-59 seen
-// from either side). c = 0: the cell itself (cluster_mode) or its same-level neighbour; c >= 1: the
-// finer cells behind a non-leaf neighbour, adjacent child a and, when that child is split, its
-// adjacent child b - 1 (c - 1 = a (2^(D-1) + 1) + b). Returns the owner or -1; `dn` is the owner's
-// direction towards the other cell and `plus` whether cell i adds the flux.
-template<class M>
-__device__ __forceinline__ int face_owner(const Pool &P, uint32_t *status, int i, int nb, int dim, int dir, int L, int li,
-                                          int ai, int c, bool cluster_mode, int &dn, bool &plus) {
-	constexpr int NSUB = 1 << (M::D - 1);
-	const int cap = P.cap;
-	if (c == 0) {
-		const uint32_t fn = P.flags[nb];
-		if (!(fn & F_LEAF)) return -1;
-		const int ln = P.level[nb], an = P.acti[nb];
-		if (cluster_mode && an <= ai && (ln < li || (ln == li && (dir == 1 || an < ai)))) {
-			dn   = dir;
-			plus = dir == 0;
-			return i;
-		}
-		if (ln == li && P.clu[nb] == L && ai <= an && ((1 - dir) == 1 || ai < an)) {
-			dn   = 1 - dir;
-			plus = dn == 1;
-			return nb;
-		}
-		return -1;
-	}
-	dn   = 1 - dir;
-	plus = dn == 1;
-	const int k = c - 1, a = k / (NSUB + 1), b = k % (NSUB + 1);
-	const int mask = (1 << dim) - 1;
-	const int ca   = (a & mask) | (dn << dim) | ((a >> dim) << (dim + 1));
-	const int ch   = P.child[(size_t) ca * cap + nb];
-	if (ch == 0) return -1;  // left out by the host: an inactive leaf or subtree, which owns no flux
-	const bool ch_leaf = P.flags[ch] & F_LEAF;
-	if (b == 0) return (ch_leaf && P.clu[ch] == L && ai <= P.acti[ch]) ? ch : -1;
-	if (ch_leaf) return -1;
-	const int gb = b - 1;
-	const int cg = (gb & mask) | (dn << dim) | ((gb >> dim) << (dim + 1));
-	const int gc = P.child[(size_t) cg * cap + ch];
-	if (gc == 0) return -1;
-	if (!(P.flags[gc] & F_LEAF)) {
-		set_status(status, ST_DEPTH);
-		return -1;
-	}
-	return (P.clu[gc] == L && ai <= P.acti[gc]) ? gc : -1;
-}
-
 // Face-flux slot of face f of the cell at list position `slot`, written for owned faces next to a receiver. The slots hold FP64
 // values in the FP64 form and FP32 values in the mixed form (T = float: the same array read with a
 // compact FP32 stride).
 template<class T = double>
 __device__ __forceinline__ T *face_flux(const Pool &P, int slot, int f, int nflux, int nfaces) {
 	return reinterpret_cast<T *>(P.ff) + ((size_t) slot * nfaces + f) * nflux;
+}
+
+// Adds to (`plus`) or takes from `acc` the fluxes across face (dim, 1 - dn) of a cell whose neighbour there is
+// the non-leaf nb: those of the finer cells of the running cluster behind the face that are not slower than
+// the cell (ACTI level ai; impl/flux.hpp:58-59 seen from the coarse side), in the order of the adjacent
+// children, a split child's own adjacent children in its place. dn is the finer cells' direction towards
+// the cell. The children's links, facts and list positions are read side by side, not child after child:
+// the walk is a chain of four dependent loads instead of four per child.
+template<class M, class T>
+__device__ __forceinline__ void hanging_fluxes(const Pool &P, uint32_t *status, int nb, int dim, int dn, int L, int ai, bool plus, double *acc) {
+	constexpr int NS = 1 << (M::D - 1), NF = 2 * M::D, F = M::F;
+	const int cap  = P.cap, mask = (1 << dim) - 1;
+	const int fo   = 2 * dim + dn;
+	auto add       = [&](int pos) {
+		const T *v = face_flux<T>(P, pos, fo, F, NF);
+		if (plus) {
+#pragma unroll
+			for (int q = 0; q < F; ++q) acc[q] += v[q];
+		} else {
+#pragma unroll
+			for (int q = 0; q < F; ++q) acc[q] -= v[q];
+		}
+	};
+	int ch[NS], pos[NS];
+	uint32_t fl[NS];
+	bool own[NS];
+#pragma unroll
+	for (int a = 0; a < NS; ++a) ch[a] = P.child[(size_t) ((a & mask) | (dn << dim) | ((a >> dim) << (dim + 1))) * cap + nb];
+#pragma unroll
+	for (int a = 0; a < NS; ++a) {
+		// a child left out by the host (slot 0) is an inactive leaf or subtree, which owns no flux
+		fl[a]  = P.flags[ch[a]];
+		own[a] = P.clu[ch[a]] == L && ai <= P.acti[ch[a]];
+		pos[a] = P.pos[ch[a]];
+	}
+#pragma unroll
+	for (int a = 0; a < NS; ++a) {
+		if (ch[a] == 0) continue;
+		if (fl[a] & F_LEAF) {
+			if (own[a]) add(pos[a]);
+			continue;
+		}
+		for (int g = 0; g < NS; ++g) {
+			const int gc = P.child[(size_t) ((g & mask) | (dn << dim) | ((g >> dim) << (dim + 1))) * cap + ch[a]];
+			if (gc == 0) continue;
+			if (!(P.flags[gc] & F_LEAF)) set_status(status, ST_DEPTH);
+			else if (P.clu[gc] == L && ai <= P.acti[gc]) add(P.pos[gc]);
+		}
+	}
 }
 
 // flux_update, receiving side: each queued receiver sums, in a fixed face order, the fluxes that
@@ -327,7 +329,6 @@ __device__ __forceinline__ void d_flux_receive(const Grid &g, const Pool &P, con
 	constexpr int NF   = 2 * M::D;
 	constexpr int G    = NF <= 4 ? 4 : 8;
 	constexpr int GW   = 32 / G;
-	constexpr int NSUB = 1 << (M::D - 1);
 	const int n      = *n_ptr;
 	const int cap    = P.cap;
 	const int lane   = threadIdx.x & 31;
@@ -345,20 +346,12 @@ __device__ __forceinline__ void d_flux_receive(const Grid &g, const Pool &P, con
 			const int li = P.level[i], ai = P.acti[i];
 			const int nb = P.nbr[(size_t) sub * cap + i];
 			if (nb != 0) {
-				const int ncand = (P.flags[nb] & F_LEAF) ? 1 : 1 + NSUB * (NSUB + 1);
-				for (int c = 0; c < ncand; ++c) {
-					int dn;
-					bool plus;
-					const int owner = face_owner<M>(P, &cnt->status, i, nb, dim, dir, L, li, ai, c, false, dn, plus);
-					if (owner < 0) continue;
-					const T *F = face_flux<T>(P, P.pos[owner], 2 * dim + dn, M::F, NF);
-					if (plus) {
+				if (!(P.flags[nb] & F_LEAF)) {
+					hanging_fluxes<M, T>(P, &cnt->status, nb, dim, 1 - dir, L, ai, dir == 0, acc);
+				} else if (P.level[nb] == li && P.clu[nb] == L && ai <= P.acti[nb] && (dir == 0 || ai < P.acti[nb])) {
+					const T *F = face_flux<T>(P, P.pos[nb], sub ^ 1, M::F, NF);
 #pragma unroll
-						for (int q = 0; q < M::F; ++q) acc[q] += F[q];
-					} else {
-#pragma unroll
-						for (int q = 0; q < M::F; ++q) acc[q] -= F[q];
-					}
+					for (int q = 0; q < M::F; ++q) acc[q] = dir == 0 ? acc[q] + F[q] : acc[q] - F[q];
 				}
 			}
 		}
@@ -376,27 +369,33 @@ __device__ __forceinline__ void d_flux_receive(const Grid &g, const Pool &P, con
 		}
 	}
 }
-template<class M, class T = double>
-__global__ void __launch_bounds__(BLOCK) k_flux_receive(Pool P, const int32_t *list, const int *n_ptr, int L,
-                                                        Counters *cnt) {
-	d_flux_receive<M, T>(PlainGrid{}, P, list, n_ptr, L, cnt);
+// What a lane or incidence of a deferred cell left for d_deferred, two bits a face (Pool::dmask, low bits in
+// the low byte): nothing, the raw flux of an owned face, the signed term, or a hanging face to be gathered.
+enum : int { DF_NONE = 0, DF_RAW = 1, DF_TERM = 2, DF_HANG = 3 };
+
+// The six (four) face terms of a cell in their fixed pairing order.
+template<int NF>
+__device__ __forceinline__ double pair_terms(const double *f) {
+	if constexpr (NF == 4) return (f[0] + f[2]) + (f[1] + f[3]);
+	else return ((f[0] + f[4]) + (f[2] + 0.0)) + ((f[1] + f[5]) + (f[3] + 0.0));
 }
 
 // flux_update (impl/flux.hpp:11-97) seen from each running-cluster cell: the signed sum of the fluxes
 // that cross its faces in this substep, one lane per face (groups of 4 lanes in 2D, 8 cells a warp; of
-// 6 lanes in 3D, 5 cells a warp, the warp's last two lanes idle). Lane f evaluates the flux across face f: the cell's own when it owns the face (the finer
-// side, at equal levels the slower cell or the cell on the left), the same-level neighbour's when the
-// neighbour owns it, the boundary flux, or the sum over the finer owners behind a non-leaf neighbour in
-// candidate order. Every interior flux is evaluated with the owner's arguments (owner, the owner's
-// neighbour, the owner's direction), so the two cells of a face obtain identical bits and the update
-// stays conservative without a face-flux array or atomics. The lane terms combine in a fixed butterfly,
-// ((f0 + f4) + (f2 + 0)) + ((f1 + f5) + (f3 + 0)) in 3D, into du[slot]. An owned face next to a cell of
-// a slower cluster (the coarse-time side of the LTS coupling, impl/flux.hpp:82-91) also goes to the
-// owner's face-flux slot, and that cell joins the receiver list. In the mixed form every flux is rounded
-// to FP32 once, as both sides read it; sums stay FP64.
+// 6 lanes in 3D, 5 cells a warp, the warp's last two lanes idle). Lane f evaluates the flux across face f:
+// the cell's own when it owns the face (the finer side, at equal levels the slower cell or the cell on the
+// left), the same-level neighbour's when the neighbour owns it, or the boundary flux. Every interior flux
+// is evaluated with the owner's arguments (owner, the owner's neighbour, the owner's direction), so the
+// two cells of a face obtain identical bits and the update stays conservative without atomics. The lane
+// terms combine in a fixed order into du[slot]. An owned face next to a cell of a slower cluster (the
+// coarse-time side of the LTS coupling, impl/flux.hpp:82-91) also goes to the owner's face-flux slot, and
+// that cell joins the receiver list; so does an owned face towards a coarser cell. A cell with a finer
+// neighbour is deferred: its other terms are stored, and d_deferred adds the finer owners' fluxes from
+// their slots, instead of evaluating up to 2^(D-1) fluxes again in one lane while the warp waits.
+// In the mixed form every flux is rounded to FP32 once, as both sides read it; sums stay FP64.
 template<class M, bool V, class S = double, class Grid>
-__device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, int L, double dtL, int stamp, int32_t *recv, Counters *cnt) {
-	constexpr int NF = 2 * M::D, G = NF, GW = 32 / G, NSUB = 1 << (M::D - 1), F = M::F;
+__device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, int L, double dtL, int stamp, int32_t *recv, int32_t *defer, Counters *cnt) {
+	constexpr int NF = 2 * M::D, G = NF, GW = 32 / G, F = M::F;
 	const int cap    = P.cap;
 	const int lane   = threadIdx.x & 31;
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
@@ -404,10 +403,10 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 	const int base   = grp * G;
 	const int items  = warp_items(n, GW);
 	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
-		const int wbase = it * GW;
-		const int slot    = wbase + grp;
+		const int slot    = it * GW + grp;
 		const bool active = grp < GW && slot < n;
 		double acc[F];
+		int code = DF_NONE;
 #pragma unroll
 		for (int q = 0; q < F; ++q) acc[q] = 0.0;
 		if (active) {
@@ -424,30 +423,10 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 					boundary_flux<M, V, S>(P, C, B, i, b, dim, dir, dtL, Fb);
 #pragma unroll
 					for (int q = 0; q < F; ++q) acc[q] = 0.0 - (double) (S) Fb[q];
+					code = DF_TERM;
 				}
 			} else if (!(P.flags[nb] & F_LEAF)) {
-				const int li = P.level[i], ai = P.acti[i];
-				double w[F];
-#pragma unroll
-				for (int q = 0; q < F; ++q) w[q] = 0.0;
-				for (int c = 1; c < 1 + NSUB * (NSUB + 1); ++c) {
-					int dn;
-					bool plus;
-					const int owner = face_owner<M>(P, &cnt->status, i, nb, dim, dir, L, li, ai, c, true, dn, plus);
-					if (owner < 0) continue;
-					const int fo = 2 * dim + dn;
-					double Fw[F];
-					interior_flux<M, V, S>(P, C, owner, P.nbr[(size_t) fo * cap + owner], dim, dn, dtL, Fw);
-					if (plus) {
-#pragma unroll
-						for (int q = 0; q < F; ++q) w[q] += (double) (S) Fw[q];
-					} else {
-#pragma unroll
-						for (int q = 0; q < F; ++q) w[q] -= (double) (S) Fw[q];
-					}
-				}
-#pragma unroll
-				for (int q = 0; q < F; ++q) acc[q] = 0.0 + (double) (S) w[q];
+				code = DF_HANG;
 			} else {
 				const int li = P.level[i], ai = P.acti[i], ln = P.level[nb], an = P.acti[nb];
 				int own = -1, fo = f;
@@ -461,11 +440,14 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 					const int other = own == i ? nb : P.nbr[(size_t) fo * cap + nb];
 					double Fi[F];
 					interior_flux<M, V, S>(P, C, own, other, dim, fo & 1, dtL, Fi);
-					if (own == i && P.clu[nb] != L) {
+					code = DF_TERM;
+					if (own == i && (ln < li || P.clu[nb] != L)) {
+						code   = DF_RAW;
 						S *dst = face_flux<S>(P, slot, f, F, NF);
 #pragma unroll
 						for (int q = 0; q < F; ++q) dst[q] = (S) Fi[q];
-						if (atomicExch(&P.stamp[nb], stamp) != stamp) append(recv, &cnt->n_recv, nb, cap, &cnt->status);
+						if (P.clu[nb] != L && atomicExch(&P.stamp[nb], stamp) != stamp)
+							append(recv, &cnt->n_recv, nb, cap, &cnt->status);
 					}
 #pragma unroll
 					for (int q = 0; q < F; ++q) {
@@ -473,6 +455,20 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 						acc[q] = dir ? 0.0 - v : 0.0 + v;
 					}
 				}
+			}
+		}
+		const unsigned lo = __ballot_sync(0xffffffffu, code & 1), hi = __ballot_sync(0xffffffffu, code & 2);
+		const unsigned gm = (1u << G) - 1u;
+		const bool deferred = ((lo & hi) >> base) & gm;
+		if (active && deferred) {
+			if (code == DF_TERM) {
+				S *dst = face_flux<S>(P, slot, sub, F, NF);
+#pragma unroll
+				for (int q = 0; q < F; ++q) dst[q] = (S) acc[q];
+			}
+			if (sub == 0) {
+				P.dmask[slot] = (int) (((lo >> base) & gm) | (((hi >> base) & gm) << 8));
+				append(defer, &cnt->n_defer, slot, cap, &cnt->status);
 			}
 		}
 		// the group's face terms in the fixed pairing order, on every lane of the group
@@ -485,16 +481,15 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 				sum[q]   = v + __shfl_xor_sync(0xffffffffu, v, 1);
 			}
 		} else {
-			// ((f0 + f4) + (f2 + 0)) + ((f1 + f5) + (f3 + 0))
 #pragma unroll
 			for (int q = 0; q < F; ++q) {
 				double f[6];
 #pragma unroll
 				for (int k = 0; k < 6; ++k) f[k] = __shfl_sync(0xffffffffu, acc[q], min(base + k, 31));
-				sum[q] = ((f[0] + f[4]) + (f[2] + 0.0)) + ((f[1] + f[5]) + (f[3] + 0.0));
+				sum[q] = pair_terms<6>(f);
 			}
 		}
-		if (active) {
+		if (active && !deferred) {
 			double *dst = P.du + (size_t) slot * F;
 #pragma unroll
 			for (int q = 0; q < F; ++q)
@@ -502,10 +497,71 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 		}
 	}
 }
+
+// The face sums of the deferred cells: lane f of a cell's group takes its stored term, or the sum of the
+// finer owners' fluxes behind a hanging face, and the group combines them in d_face_sum's order into du.
+template<class M, class S, class Grid>
+__device__ __forceinline__ void d_deferred(const Grid &g, const Pool &P, const int32_t *list, const int32_t *defer, const int *n_ptr, int L, Counters *cnt) {
+	constexpr int NF = 2 * M::D, G = NF, GW = 32 / G, F = M::F;
+	const int n     = *n_ptr;
+	const int cap   = P.cap;
+	const int lane  = threadIdx.x & 31;
+	const int grp   = lane / G;
+	const int sub   = lane - grp * G;
+	const int base  = grp * G;
+	const int items = warp_items(n, GW);
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int k       = it * GW + grp;
+		const bool active = grp < GW && k < n;
+		double acc[F];
+#pragma unroll
+		for (int q = 0; q < F; ++q) acc[q] = 0.0;
+		int slot = 0;
+		if (active) {
+			slot           = defer[k];
+			const int m    = P.dmask[slot];
+			const int code = ((m >> sub) & 1) | (((m >> (8 + sub)) & 1) << 1);
+			const int dir  = sub & 1;
+			if (code == DF_HANG) {
+				const int i = list[slot];
+				double w[F];
+#pragma unroll
+				for (int q = 0; q < F; ++q) w[q] = 0.0;
+				hanging_fluxes<M, S>(P, &cnt->status, P.nbr[(size_t) sub * cap + i], sub >> 1, 1 - dir, L, P.acti[i], dir == 0, w);
+#pragma unroll
+				for (int q = 0; q < F; ++q) acc[q] = 0.0 + (double) (S) w[q];
+			} else if (code != DF_NONE) {
+				const S *src = face_flux<S>(P, slot, sub, F, NF);
+#pragma unroll
+				for (int q = 0; q < F; ++q) {
+					const double v = (double) src[q];
+					acc[q]         = code == DF_TERM ? v : dir ? 0.0 - v : 0.0 + v;
+				}
+			}
+		}
+		double *dst = P.du + (size_t) slot * F;
+#pragma unroll
+		for (int q = 0; q < F; ++q) {
+			double f[NF];
+#pragma unroll
+			for (int j = 0; j < NF; ++j) f[j] = __shfl_sync(0xffffffffu, acc[q], min(base + j, 31));
+			if (active && q % G == sub) dst[q] = pair_terms<NF>(f);
+		}
+	}
+}
 template<class M, bool V, class S = double>
 __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS) k_face_sum(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L,
-                                                    double dtL, int stamp, int32_t *recv, Counters *cnt) {
-	d_face_sum<M, V, S>(PlainGrid{}, P, C, B, list, n, L, dtL, stamp, recv, cnt);
+                                                    double dtL, int stamp, int32_t *recv, int32_t *defer, Counters *cnt) {
+	d_face_sum<M, V, S>(PlainGrid{}, P, C, B, list, n, L, dtL, stamp, recv, defer, cnt);
+}
+
+// The receivers' sums and the deferred cells' face sums: both gather face-flux slots of the running cluster
+// and neither reads what the other writes.
+template<class M, class T = double>
+__global__ void __launch_bounds__(BLOCK) k_flux_receive(Pool P, const int32_t *recv, const int32_t *list, const int32_t *defer,
+                                                        int L, Counters *cnt) {
+	d_flux_receive<M, T>(PlainGrid{}, P, recv, &cnt->n_recv, L, cnt);
+	d_deferred<M, T>(PlainGrid{}, P, list, defer, &cnt->n_defer, L, cnt);
 }
 
 // The same face sums over tiles of TC consecutive list positions, one 128-thread block per tile. After
@@ -513,14 +569,14 @@ __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS) k_face_sum(Pool
 // most faces have both cells in it; such a face is evaluated once, by the task of its owner, instead of
 // once by each of its cells. Per tile:
 //   1. every (cell, face) incidence is classified as d_face_sum classifies its lane: boundary, non-leaf
-//      neighbour (the sum over the finer owners), a flux owned by the cell, a flux owned by the
-//      same-level neighbour, or none. A flux owned by the neighbour becomes a reference to the
-//      neighbour's own incidence when the neighbour is in the tile (it then evaluates that face as its
-//      own), else a task of this cell; every other flux is a task;
+//      neighbour (which defers the cell), a flux owned by the cell, a flux owned by the same-level
+//      neighbour, or none. A flux owned by the neighbour becomes a reference to the neighbour's own
+//      incidence when the neighbour is in the tile (it then evaluates that face as its own), else a task
+//      of this cell; every other flux is a task;
 //   2. the block's threads run the tasks, interior fluxes first (compacted at the low end of the task
-//      list, boundary and non-leaf sums at the high end, so that warps diverge less), into shared memory;
+//      list, boundary fluxes at the high end, so that warps diverge less), into shared memory;
 //   3. each (cell, component) thread combines the cell's face terms in d_face_sum's fixed pairing order
-//      and writes du.
+//      and writes du, or leaves a deferred cell's terms in its face-flux slots.
 // Every flux is the same call with the same arguments as in d_face_sum (the owner's), and the terms are
 // combined in the same order with the same signs, so du is the same bit for bit.
 template<class M>
@@ -536,14 +592,15 @@ enum : uint8_t { FT_NONE = 0, FT_BND = 1, FT_HANG = 2, FT_INT = 3, FT_INT_FF = 4
 template<class M, bool V, class S>
 __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS)
 k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, double dtL, int stamp, int32_t *recv,
-            Counters *cnt) {
+            int32_t *defer, Counters *cnt) {
 	using T = FaceTile<M>;
-	constexpr int NF = T::NF, F = T::F, TC = T::TC, NI = T::NI, NSUB = 1 << (M::D - 1);
+	constexpr int NF = T::NF, F = T::F, TC = T::TC, NI = T::NI;
 	__shared__ double s_res[NI * F];  // face results by incidence
 	__shared__ int32_t s_a[NI];       // owner of a task, or the partner incidence of a reference
 	__shared__ int32_t s_b[NI];       // the task's other cell, boundary id or non-leaf neighbour
 	__shared__ int16_t s_task[NI];
 	__shared__ int32_t s_cell[TC];
+	__shared__ uint8_t s_defer[TC];
 	__shared__ uint8_t s_kind[NI];
 	__shared__ int s_lo, s_hi;
 	const int cap = P.cap;
@@ -555,7 +612,8 @@ k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, doub
 				i        = list[slot];
 				P.pos[i] = slot;
 			}
-			s_cell[c] = i;
+			s_cell[c]  = i;
+			s_defer[c] = 0;
 		}
 		if (threadIdx.x == 0) s_lo = 0, s_hi = 0;
 		__syncthreads();
@@ -573,14 +631,14 @@ k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, doub
 					if (b < 0) set_status(&cnt->status, ST_MISSING_BC);
 					else kind = FT_BND, low = false;
 				} else if (!(P.flags[nb] & F_LEAF)) {
-					kind = FT_HANG, b = nb, low = false;
+					kind = FT_HANG, s_defer[c] = 1;
 				} else {
 					const int li = P.level[i], ai = P.acti[i], ln = P.level[nb], an = P.acti[nb];
 					if (an <= ai && (ln < li || (ln == li && (dir == 1 || an < ai)))) {
 						kind = FT_INT, a = i, b = nb;
-						if (P.clu[nb] != L) {
+						if (ln < li || P.clu[nb] != L) {
 							kind = FT_INT_FF;
-							if (atomicExch(&P.stamp[nb], stamp) != stamp) append(recv, &cnt->n_recv, nb, cap, &cnt->status);
+							if (P.clu[nb] != L && atomicExch(&P.stamp[nb], stamp) != stamp) append(recv, &cnt->n_recv, nb, cap, &cnt->status);
 						}
 					} else if (ln == li && P.clu[nb] == L && ai <= an && (dir == 0 || ai < an)) {
 						// pos of a cell of this tile was written above, before the barrier; pos of any
@@ -599,7 +657,7 @@ k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, doub
 			s_kind[inc] = kind;
 			s_a[inc]    = a;
 			s_b[inc]    = b;
-			if (kind != FT_NONE && kind != FT_REF) {
+			if (kind != FT_NONE && kind != FT_HANG && kind != FT_REF) {
 				if (low) s_task[atomicAdd(&s_lo, 1)] = (int16_t) inc;
 				else s_task[NI - 1 - atomicAdd(&s_hi, 1)] = (int16_t) inc;
 			}
@@ -618,30 +676,6 @@ k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, doub
 				boundary_flux<M, V, S>(P, C, B, i, s_b[inc], dim, dir, dtL, Fb);
 #pragma unroll
 				for (int q = 0; q < F; ++q) res[q] = 0.0 - (double) (S) Fb[q];
-			} else if (kind == FT_HANG) {
-				const int nb = s_b[inc];
-				const int li = P.level[i], ai = P.acti[i];
-				double w[F];
-#pragma unroll
-				for (int q = 0; q < F; ++q) w[q] = 0.0;
-				for (int cc = 1; cc < 1 + NSUB * (NSUB + 1); ++cc) {
-					int dn;
-					bool plus;
-					const int owner = face_owner<M>(P, &cnt->status, i, nb, dim, dir, L, li, ai, cc, true, dn, plus);
-					if (owner < 0) continue;
-					const int fo = 2 * dim + dn;
-					double Fw[F];
-					interior_flux<M, V, S>(P, C, owner, P.nbr[(size_t) fo * cap + owner], dim, dn, dtL, Fw);
-					if (plus) {
-#pragma unroll
-						for (int q = 0; q < F; ++q) w[q] += (double) (S) Fw[q];
-					} else {
-#pragma unroll
-						for (int q = 0; q < F; ++q) w[q] -= (double) (S) Fw[q];
-					}
-				}
-#pragma unroll
-				for (int q = 0; q < F; ++q) res[q] = 0.0 + (double) (S) w[q];
 			} else {
 				const int own = s_a[inc];
 				const int dir_o = own == i ? dir : 1 - dir;
@@ -662,23 +696,33 @@ k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, doub
 			const int c = idx / F, q = idx - c * F;
 			if (t0 + c >= n) continue;
 			double fv[NF];
+			int mask = 0;
 #pragma unroll
 			for (int k = 0; k < NF; ++k) {
 				const int inc = c * NF + k;
 				const uint8_t kind = s_kind[inc];
 				double v = 0.0;
-				if (kind == FT_BND || kind == FT_HANG) {
+				if (kind == FT_BND) {
 					v = s_res[inc * F + q];
-				} else if (kind != FT_NONE) {
+				} else if (kind != FT_NONE && kind != FT_HANG) {
 					const double raw = s_res[(kind == FT_REF ? s_a[inc] : inc) * F + q];
 					v = (k & 1) ? 0.0 - raw : 0.0 + raw;
 				}
 				fv[k] = v;
+				const int code = kind == FT_NONE ? DF_NONE : kind == FT_HANG ? DF_HANG : kind == FT_INT_FF ? DF_RAW : DF_TERM;
+				mask |= (code & 1) << k | (code >> 1) << (8 + k);
 			}
-			double sum;
-			if constexpr (NF == 4) sum = (fv[0] + fv[2]) + (fv[1] + fv[3]);
-			else sum = ((fv[0] + fv[4]) + (fv[2] + 0.0)) + ((fv[1] + fv[5]) + (fv[3] + 0.0));
-			P.du[(size_t) (t0 + c) * F + q] = sum;
+			if (!s_defer[c]) {
+				P.du[(size_t) (t0 + c) * F + q] = pair_terms<NF>(fv);
+				continue;
+			}
+#pragma unroll
+			for (int k = 0; k < NF; ++k)
+				if ((mask >> k & 1) == 0 && (mask >> (8 + k) & 1)) face_flux<S>(P, t0 + c, k, F, NF)[q] = (S) fv[k];
+			if (q == 0) {
+				P.dmask[t0 + c] = mask;
+				append(defer, &cnt->n_defer, t0 + c, cap, &cnt->status);
+			}
 		}
 		__syncthreads();
 	}

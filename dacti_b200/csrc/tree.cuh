@@ -118,6 +118,39 @@ __device__ void interp_pt(const Pool &P, uint32_t *status, int n, int epoch, dou
 		for (int q = 0; q <= E; ++q) out[q] = __ldcg(P.avg + (size_t) n * AW + q);
 		return;
 	}
+	// Nearly every node asked for has leaves only below it: their links, flags and records are read side by
+	// side (slot 0, an inactive leaf, stands in for a missing child) and added in slot order.
+	int ch[NC];
+	uint32_t fl[NC];
+	bool flat = true;
+#pragma unroll
+	for (int k = 0; k < NC; ++k) ch[k] = P.child[(size_t) k * P.cap + n];
+#pragma unroll
+	for (int k = 0; k < NC; ++k) fl[k] = P.flags[ch[k]];
+#pragma unroll
+	for (int k = 0; k < NC; ++k) flat = flat && (fl[k] & (F_ACTIVE | F_LEAF)) != F_ACTIVE;
+	if (flat) {
+		int cnt = 0;
+		double f[E + 1];
+#pragma unroll
+		for (int q = 0; q <= E; ++q) f[q] = 0.0;
+#pragma unroll
+		for (int k = 0; k < NC; ++k) {
+			double pc[E];
+			load_p_rec<M>(P, ch[k], pc);
+			const double tc = P.t[ch[k]];
+			const bool act  = fl[k] & F_ACTIVE;
+			cnt += act;
+#pragma unroll
+			for (int q = 0; q < E; ++q) f[q] = act ? f[q] + pc[q] : f[q];
+			f[E] = act ? f[E] + tc : f[E];
+		}
+		double *memo = P.avg + (size_t) n * AW;
+#pragma unroll
+		for (int q = 0; q <= E; ++q) memo[q] = out[q] = f[q] / (double) cnt;
+		P.cst[n] = epoch;
+		return;
+	}
 	struct Frame {
 		int node, next, cnt;
 		double f[E + 1];
@@ -254,6 +287,33 @@ __device__ double interp_alpha(const Pool &P, uint32_t *status, int n, Val val, 
 	};
 	if (P.flags[n] & F_LEAF) return val(n);
 	if (ok(n)) return __ldcg(P.avga + n);
+	// leaves only below the node, read side by side (interp_pt)
+	int ch[NC];
+	uint32_t fls[NC];
+	bool flat = true;
+#pragma unroll
+	for (int k = 0; k < NC; ++k) ch[k] = P.child[(size_t) k * P.cap + n];
+#pragma unroll
+	for (int k = 0; k < NC; ++k) fls[k] = P.flags[ch[k]];
+#pragma unroll
+	for (int k = 0; k < NC; ++k) flat = flat && (fls[k] & (F_ACTIVE | F_LEAF)) != F_ACTIVE;
+	if (flat) {
+		int c    = 0;
+		double a = 0.0;
+#pragma unroll
+		for (int k = 0; k < NC; ++k) {
+			const double v = val(ch[k]);
+			const bool act = fls[k] & F_ACTIVE;
+			c += act;
+			a = act ? a + v : a;
+		}
+		const double r = a / (double) c;
+		if (__ldcg(P.mod + n) < e_upd) {
+			P.avga[n] = r;
+			P.csta[n] = epoch;
+		}
+		return r;
+	}
 	int node[MAX_TREE], next[MAX_TREE], cnt[MAX_TREE];
 	double f[MAX_TREE];
 	int sp  = 1;
