@@ -835,7 +835,7 @@ private:
 			Solver<M> *s         = s_[p.sel[k]];
 			const long long need = (long long) s->h_cnt_->top + (long long) NC * s->h_cnt_->n_split + 16;
 			if (need > s->P_.cap) {
-				const long long want = s->growth_target(need, std::max(need + need / 4, (long long) s->P_.cap * 5 / 4));
+				const long long want = s->growth_target(need, s->grown(need));
 				s->grow_pool((int) std::min<long long>(want, 2000000000LL));
 				grown = true;
 			}

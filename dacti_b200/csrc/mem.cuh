@@ -1,0 +1,142 @@
+// Device memory of the solvers: one stream-ordered pool per device, owned by the library.
+//
+// cudaMalloc and cudaFree wait for the whole device. A solver makes about fifteen allocations, a growing
+// tree replaces its pool, lists and scratch every few steps, and while many solvers step side by side each
+// such call waits for every other solver's kernels. Allocations from the pool are ordered with the solver's
+// own stream instead. While solvers live the pool keeps up to KEEP bytes that nothing uses; when the last
+// one is gone it gives back all but KEEP_IDLE.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <mutex>
+#include <vector>
+
+namespace dg {
+
+struct DeviceMemory {
+	static constexpr size_t KEEP      = size_t(4) << 30;
+	static constexpr size_t KEEP_IDLE = size_t(1) << 30;
+
+	cudaMemPool_t pool  = nullptr;
+	cudaStream_t stream = nullptr;  // of frees whose last use the host has waited for
+	int users           = 0;
+
+	static std::mutex &lock() {
+		static std::mutex m;
+		return m;
+	}
+
+	// The current device's memory, made at its first use; null with the error in `e`.
+	static DeviceMemory *of_device(cudaError_t &e) {
+		static DeviceMemory all[64];
+		int dev = 0;
+		if ((e = cudaGetDevice(&dev)) != cudaSuccess) return nullptr;
+		if (dev < 0 || dev >= 64) {
+			e = cudaErrorInvalidDevice;
+			return nullptr;
+		}
+		DeviceMemory &d = all[dev];
+		std::lock_guard<std::mutex> l(lock());
+		if (!d.pool) {
+			cudaMemPoolProps p{};
+			p.allocType     = cudaMemAllocationTypePinned;
+			p.handleTypes   = cudaMemHandleTypeNone;
+			p.location.type = cudaMemLocationTypeDevice;
+			p.location.id   = dev;
+			cudaMemPool_t pool  = nullptr;
+			cudaStream_t stream = nullptr;
+			if ((e = cudaMemPoolCreate(&pool, &p)) != cudaSuccess) return nullptr;
+			unsigned long long keep = KEEP;
+			e                       = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+			if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+			if (e != cudaSuccess) {
+				cudaMemPoolDestroy(pool);
+				return nullptr;
+			}
+			d.pool   = pool;
+			d.stream = stream;
+		}
+		return &d;
+	}
+};
+
+// `bytes` of device memory for work on stream `st`, from its order on.
+inline cudaError_t mem_alloc(void **p, size_t bytes, cudaStream_t st) {
+	cudaError_t e;
+	DeviceMemory *d = DeviceMemory::of_device(e);
+	return d ? cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st) : e;
+}
+// Gives memory back once the work queued on `st` so far is done with it.
+inline void mem_free(void *p, cudaStream_t st) {
+	if (p) cudaFreeAsync(p, st);
+}
+// Gives back memory that nothing queued uses any more, whatever became of the stream it was used on.
+inline void mem_free_idle(void *p) {
+	cudaError_t e;
+	DeviceMemory *d = p ? DeviceMemory::of_device(e) : nullptr;
+	if (d) cudaFreeAsync(p, d->stream);
+}
+// Bytes that the pool holds and nothing uses.
+inline size_t mem_unused() {
+	cudaError_t e;
+	DeviceMemory *d             = DeviceMemory::of_device(e);
+	unsigned long long reserved = 0, used = 0;
+	if (!d || cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+	    cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+		return 0;
+	return reserved > used ? (size_t) (reserved - used) : 0;
+}
+// A user of the current device's pool, as long as it lives.
+class MemoryUser {
+	DeviceMemory *d_;
+
+public:
+	MemoryUser() {
+		cudaError_t e;
+		d_ = DeviceMemory::of_device(e);
+		std::lock_guard<std::mutex> l(DeviceMemory::lock());
+		if (d_) ++d_->users;
+	}
+	MemoryUser(const MemoryUser &)            = delete;
+	MemoryUser &operator=(const MemoryUser &) = delete;
+	~MemoryUser() {
+		std::lock_guard<std::mutex> l(DeviceMemory::lock());
+		if (!d_ || --d_->users > 0) return;
+		cudaStreamSynchronize(d_->stream);
+		cudaMemPoolTrimTo(d_->pool, DeviceMemory::KEEP_IDLE);
+	}
+};
+
+// A pinned host block of PINNED_BYTES; up to PINNED_KEEP of them wait for the next solver, since pinning a page
+// costs as much as building a small one.
+constexpr size_t PINNED_BYTES = 2048;
+constexpr size_t PINNED_KEEP  = 64;
+inline std::vector<void *> &pinned_free() {
+	static std::vector<void *> v;
+	return v;
+}
+inline cudaError_t pinned_alloc(void **p) {
+	{
+		std::lock_guard<std::mutex> l(DeviceMemory::lock());
+		if (!pinned_free().empty()) {
+			*p = pinned_free().back();
+			pinned_free().pop_back();
+			return cudaSuccess;
+		}
+	}
+	return cudaHostAlloc(p, PINNED_BYTES, cudaHostAllocPortable);
+}
+inline void pinned_release(void *p) {
+	if (!p) return;
+	{
+		std::lock_guard<std::mutex> l(DeviceMemory::lock());
+		if (pinned_free().size() < PINNED_KEEP) {
+			pinned_free().push_back(p);
+			return;
+		}
+	}
+	cudaFreeHost(p);
+}
+
+}  // namespace dg

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "../../include/dacti_gpu.h"
+#include "mem.cuh"
 #include "run.cuh"
 
 #include <cub/cub.cuh>
@@ -75,13 +76,14 @@ class Solver : public SolverBase {
 	static constexpr int D = M::D, E = M::E, NC = 1 << D, NF = 2 * D;
 	friend class Batch<M>;
 
+	MemoryUser memory_;
 	cudaStream_t st_ = 0;
 	Consts C_{};
 	BcTable B_{};
 	Pool P_{};
 	Lists Ls_{};
 	Counters *d_cnt_ = nullptr;
-	Counters *h_cnt_ = nullptr;  // pinned
+	Counters *h_cnt_ = nullptr;  // pinned, behind h_run_ unless a batch holds the counters
 	RunState *d_run_ = nullptr;  // schedule state of device-resident runs, then the grid barrier's counter
 	RunState *h_run_ = nullptr;  // pinned
 	int run_cluster_ = 0;        // blocks of a clustered run on this device (0: not asked yet)
@@ -191,33 +193,33 @@ public:
 		if (cap > 2000000000LL) throw dg_error(DG_ERR_CAPACITY, "node pool capacity above 2e9 slots");
 		alloc_pool((int) cap);
 		alloc_lists(cap);
-		DG_CUDA(cudaMalloc(&d_cnt_, sizeof(Counters)));
-		DG_CUDA(cudaMallocHost(&h_cnt_, sizeof(Counters)));
+		DG_CUDA(mem_alloc((void **) &d_cnt_, sizeof(Counters), st_));
+		static_assert(sizeof(RunState) + 16 + sizeof(Counters) <= PINNED_BYTES, "run state and counters share a pinned block");
+		DG_CUDA(pinned_alloc((void **) &h_run_));
+		h_cnt_ = (Counters *) ((char *) h_run_ + (sizeof(RunState) + sizeof(unsigned) + 7) / 8 * 8);
 		DG_CUDA(cudaMemset(d_cnt_, 0, sizeof(Counters)));
-		DG_CUDA(cudaMalloc(&d_run_, sizeof(RunState) + sizeof(unsigned)));
-		DG_CUDA(cudaMallocHost(&h_run_, sizeof(RunState) + sizeof(unsigned)));
+		DG_CUDA(mem_alloc((void **) &d_run_, sizeof(RunState) + sizeof(unsigned), st_));
 		upload_tree(c);
 		construct();
 	}
 
 	~Solver() override {
 		cudaStreamSynchronize(st_);
-		cudaFree(pool_mem_);
-		cudaFree(spare_mem_);
-		cudaFree(sort_mem_);
-		cudaFree(list_mem_);
-		cudaFree(bc_mem_);
-		cudaFree(ff_mem_);
-		cudaFree(du_mem_);
-		cudaFree(sel_mem_);
-		cudaFree(pos_mem_);
-		cudaFree(d_cnt_);
-		cudaFreeHost(h_cnt_);
-		cudaFree(d_run_);
-		cudaFreeHost(h_run_);
-		cudaFree(d_leaves_);
-		cudaFree(d_read_);
-		cudaFree(d_readlv_);
+		mem_free_idle(pool_mem_);
+		mem_free_idle(spare_mem_);
+		mem_free_idle(sort_mem_);
+		mem_free_idle(list_mem_);
+		mem_free_idle(bc_mem_);
+		mem_free_idle(ff_mem_);
+		mem_free_idle(du_mem_);
+		mem_free_idle(sel_mem_);
+		mem_free_idle(pos_mem_);
+		mem_free_idle(d_cnt_);
+		mem_free_idle(d_run_);
+		pinned_release(h_run_);
+		mem_free_idle(d_leaves_);
+		mem_free_idle(d_read_);
+		mem_free_idle(d_readlv_);
 		if (owned_stream_) cudaStreamDestroy(owned_stream_);
 		for (auto e: ev_free_) cudaEventDestroy(e);
 		for (auto &p: pending_) {
@@ -310,7 +312,7 @@ public:
 	void upload_bcs(const dg_case &c) {
 		int n        = c.n_bc > 0 ? c.n_bc : 1;
 		size_t bytes = sizeof(int) * n + sizeof(double) * n * (E + D + 1) + 1024;
-		DG_CUDA(cudaMalloc(&bc_mem_, bytes));
+		DG_CUDA(mem_alloc((void **) &bc_mem_, bytes, st_));
 		char *b   = (char *) bc_mem_;
 		int *type = (int *) b;
 		b += ((sizeof(int) * n + 255) / 256) * 256;
@@ -332,35 +334,49 @@ public:
 		void **ptr;
 		size_t elem;
 		int comps;
+		int link = 0;  // holds slot numbers
+		int stay = 0;  // scratch of one substep, or marks that no later value equals: need not follow their slots
 	};
 
 	std::vector<Field> fields(Pool &P) {
 		return {
-		    {(void **) &P.parent, 4, 1}, {(void **) &P.child, 4, NC}, {(void **) &P.level, 1, 1},
+		    {(void **) &P.parent, 4, 1, 1}, {(void **) &P.child, 4, NC, 1}, {(void **) &P.level, 1, 1},
 		    {(void **) &P.acti, 1, 1}, {(void **) &P.clu, 1, 1}, {(void **) &P.flags, 4, 1},
-		    {(void **) &P.coord, 4, D}, {(void **) &P.nbr, 4, NF}, {(void **) &P.bc, 2, NF},
+		    {(void **) &P.coord, 4, D}, {(void **) &P.nbr, 4, NF, 1}, {(void **) &P.bc, 2, NF},
 		    {(void **) &P.center, 8, D}, {(void **) &P.t, 8, 1}, {(void **) &P.u, 8, E},
 		    {(void **) &P.p, 8, E}, {(void **) &P.rec, 8 * Rec<M>::W, 1}, {(void **) &P.avg, 8 * Avg<M>::W, 1},
 		    {(void **) &P.mod, 4, 1}, {(void **) &P.cst, 4, 1}, {(void **) &P.avga, 8, 1}, {(void **) &P.csta, 4, 1},
 		    {(void **) &P.k, 8, M::P}, {(void **) &P.tslope, 8, visc_ ? M::G : -1},
 		    {(void **) &P.grad, 8, visc_ ? D * M::G : -1},
 		    {(void **) &P.flux, 8, M::F}, {(void **) &P.err, 8, 1}, {(void **) &P.maxdt, 8, 1},
-		    {(void **) &P.cfl, 8, 1}, {(void **) &P.stamp, 4, 1}, {(void **) &P.fmask, 4, 1}, {(void **) &P.op, 1, 1},
-		    {(void **) &P.tmp, 8, 1}, {(void **) &P.tmp2, 8, 1},
+		    {(void **) &P.cfl, 8, 1}, {(void **) &P.stamp, 4, 1, 0, 1}, {(void **) &P.fmask, 4, 1, 0, 1}, {(void **) &P.op, 1, 1},
+		    {(void **) &P.tmp, 8, 1, 0, 1}, {(void **) &P.tmp2, 8, 1, 0, 1},
 		};
 	}
 
 	static size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
-	// The spare buffer holds the largest field of the pool (the reconstruction records, in practice).
+	// The spare buffer of the re-sort and gc holds the largest field of the pool (the reconstruction records,
+	// in practice), or a second pool where that is small enough: a re-sort then writes every field once, in
+	// three launches, and the two change places.
+	static constexpr size_t SECOND_POOL_MAX = size_t(4) << 30;
+	bool spare_dirty_ = true;  // the spare buffer holds something else than an earlier state of the pool
+	size_t pool_bytes(Pool &P) {
+		size_t total = 0;
+		for (auto &f: fields(P)) total += field_bytes(f, P.cap);
+		return total;
+	}
+	bool second_pool() { return pool_bytes(P_) <= SECOND_POOL_MAX; }
 	void ensure_spare() {
 		size_t need = 0;
 		for (auto &f: fields(P_)) need = std::max(need, field_bytes(f, P_.cap));
+		if (second_pool()) need = pool_bytes(P_);
 		if (spare_mem_ && spare_bytes_ >= need) return;
-		cudaFree(spare_mem_);
+		mem_free(spare_mem_, st_);
 		spare_mem_ = nullptr;
-		DG_CUDA(cudaMalloc(&spare_mem_, need));
+		DG_CUDA(mem_alloc((void **) &spare_mem_, need, st_));
 		spare_bytes_ = need;
+		spare_dirty_ = true;
 	}
 
 	// Bytes of one field: comps < 0 marks a field this case does not store (no storage, null pointer);
@@ -369,19 +385,21 @@ public:
 		return f.comps < 0 ? 0 : align_up(f.elem * (size_t) cap * (f.comps > 0 ? f.comps : 1));
 	}
 
-	void *carve_pool(Pool &P, int cap) {
-		P.cap        = cap;
-		auto fs      = fields(P);
-		size_t total = 0;
-		for (auto &f: fs) total += field_bytes(f, cap);
-		void *mem = nullptr;
-		DG_CUDA(cudaMalloc(&mem, total));
-		DG_CUDA(cudaMemsetAsync(mem, 0, total, st_));
+	void place_fields(Pool &P, void *mem) {
 		char *b = (char *) mem;
-		for (auto &f: fs) {
+		for (auto &f: fields(P)) {
 			*f.ptr = f.comps < 0 ? nullptr : b;
-			b += field_bytes(f, cap);
+			b += field_bytes(f, P.cap);
 		}
+	}
+
+	void *carve_pool(Pool &P, int cap) {
+		P.cap              = cap;
+		const size_t total = pool_bytes(P);
+		void *mem          = nullptr;
+		DG_CUDA(mem_alloc((void **) &mem, total, st_));
+		DG_CUDA(cudaMemsetAsync(mem, 0, total, st_));
+		place_fields(P, mem);
 		return mem;
 	}
 
@@ -394,9 +412,9 @@ public:
 	// sized to the largest list a substep has run so far (grown by a quarter when a larger one comes):
 	// receiver face fluxes and face-flux sums.
 	void alloc_derived(int cap) {
-		cudaFree(pos_mem_);
+		mem_free(pos_mem_, st_);
 		pos_mem_ = nullptr;
-		DG_CUDA(cudaMalloc(&pos_mem_, sizeof(int32_t) * (size_t) cap));
+		DG_CUDA(mem_alloc((void **) &pos_mem_, sizeof(int32_t) * (size_t) cap, st_));
 		attach_derived();
 	}
 
@@ -404,21 +422,21 @@ public:
 	void ensure_scratch(long long n) {
 		if (n <= scratch_cap_) return;
 		const long long want = std::max(std::max(n, scratch_cap_ + scratch_cap_ / 4), 1024LL);
-		cudaFree(ff_mem_);
-		cudaFree(du_mem_);
-		cudaFree(sel_mem_);
+		mem_free(ff_mem_, st_);
+		mem_free(du_mem_, st_);
+		mem_free(sel_mem_, st_);
 		ff_mem_      = nullptr;
 		du_mem_      = nullptr;
 		sel_mem_     = nullptr;
 		scratch_cap_ = 0;
-		DG_CUDA(cudaMalloc(&ff_mem_, sizeof(double) * M::F * NF * (size_t) want));
-		DG_CUDA(cudaMalloc(&du_mem_, (sizeof(double) * M::F + sizeof(int32_t)) * (size_t) want));
+		DG_CUDA(mem_alloc((void **) &ff_mem_, sizeof(double) * M::F * NF * (size_t) want, st_));
+		DG_CUDA(mem_alloc((void **) &du_mem_, (sizeof(double) * M::F + sizeof(int32_t)) * (size_t) want, st_));
 		// stay marks (one byte per list position, rounded to 256) followed by the temp storage of the
 		// order-keeping compaction of `want` items
 		sel_tmp_bytes_ = 0;
 		DG_CUDA(cub::DeviceSelect::Flagged(nullptr, sel_tmp_bytes_, (const int32_t *) nullptr, (const uint8_t *) nullptr,
 		                                   (int32_t *) nullptr, (int *) nullptr, (int) want, st_));
-		DG_CUDA(cudaMalloc(&sel_mem_, stay_bytes(want) + sel_tmp_bytes_));
+		DG_CUDA(mem_alloc((void **) &sel_mem_, stay_bytes(want) + sel_tmp_bytes_, st_));
 		scratch_cap_ = want;
 		attach_derived();
 	}
@@ -443,9 +461,16 @@ public:
 		size_t per_slot = sizeof(int32_t) * (2 * MAX_ACTI + 6);
 		for (auto &f: fields(P_))
 			if (f.comps >= 0) per_slot += f.elem * (size_t) (f.comps > 0 ? f.comps : 1);
-		const long long avail = (long long) (free_b + released) - (1LL << 30);
+		const long long avail = (long long) (free_b + mem_unused() + released) - (1LL << 30);
 		const long long fit   = avail > 0 ? avail / (long long) per_slot : 0;
 		return std::max(need, std::min(want, fit));
+	}
+
+	// The rows of field f from `src` (component stride src_cap) to `dst`.
+	static void add_rows(RowTable &t, const Field &f, const void *src, int src_cap, void *dst, int dst_cap, bool relink) {
+		for (int c = 0; c < f.comps; ++c)
+			t.r[t.n++] = {(const char *) src + f.elem * (size_t) src_cap * c, (char *) dst + f.elem * (size_t) dst_cap * c,
+			              (int) f.elem, relink && f.link};
 	}
 
 	// Grows the node pool: a new pool of new_cap slots takes every field, then the old one goes. Grows
@@ -454,15 +479,16 @@ public:
 	// their next use) and the peak holds the two pools and the lists only.
 	void grow_pool(int new_cap) {
 		DG_CUDA(cudaStreamSynchronize(st_));
-		cudaFree(spare_mem_);
+		mem_free(spare_mem_, st_);
 		spare_mem_   = nullptr;
 		spare_bytes_ = 0;
-		cudaFree(sort_mem_);
+		spare_dirty_ = true;
+		mem_free(sort_mem_, st_);
 		sort_mem_   = nullptr;
 		sort_bytes_ = 0;
-		cudaFree(ff_mem_);
-		cudaFree(du_mem_);
-		cudaFree(sel_mem_);
+		mem_free(ff_mem_, st_);
+		mem_free(du_mem_, st_);
+		mem_free(sel_mem_, st_);
 		ff_mem_      = nullptr;
 		du_mem_      = nullptr;
 		sel_mem_     = nullptr;
@@ -470,15 +496,20 @@ public:
 		attach_derived();
 		Pool NP{};
 		void *mem = carve_pool(NP, new_cap);
+		// the slots in use; the rest of the new pool is zero, as it was in the old one
 		auto fo = fields(P_), fn = fields(NP);
+		const int used = std::min(h_cnt_->top, P_.cap);
+		RowTable t{};
 		for (size_t k = 0; k < fo.size(); ++k) {
 			if (fo[k].comps <= 0) continue;
-			DG_CUDA(cudaMemcpy2DAsync(*fn[k].ptr, fn[k].elem * (size_t) new_cap, *fo[k].ptr,
-			                          fo[k].elem * (size_t) P_.cap, fo[k].elem * (size_t) P_.cap, fo[k].comps,
-			                          cudaMemcpyDeviceToDevice, st_));
+			if (fo[k].elem > 8)
+				DG_CUDA(cudaMemcpyAsync(*fn[k].ptr, *fo[k].ptr, fo[k].elem * (size_t) used, cudaMemcpyDeviceToDevice, st_));
+			else
+				add_rows(t, fo[k], *fo[k].ptr, P_.cap, *fn[k].ptr, new_cap, false);
 		}
-		DG_CUDA(cudaStreamSynchronize(st_));
-		cudaFree(pool_mem_);
+		k_rows<<<dim3(grid_for(used, 148 * 4), t.n), BLOCK, 0, st_>>>(t, used, nullptr, nullptr);
+		DG_CUDA(cudaGetLastError());
+		mem_free(pool_mem_, st_);
 		pool_mem_ = mem;
 		P_        = NP;
 		alloc_derived(new_cap);
@@ -487,25 +518,24 @@ public:
 		void *old_mem = list_mem_;
 		int old_cap   = list_cap_;
 		alloc_lists(new_cap);
-		const size_t bytes = sizeof(int32_t) * old_cap;
+		auto keep = [&](int32_t *dst, const int32_t *src, int n) {
+			if (n > 0) DG_CUDA(cudaMemcpyAsync(dst, src, sizeof(int32_t) * std::min(n, old_cap), cudaMemcpyDeviceToDevice, st_));
+		};
 		for (int l = 0; l < MAX_ACTI; ++l) {
-			DG_CUDA(cudaMemcpyAsync(Ls_.clu[l], old.clu[l], bytes, cudaMemcpyDeviceToDevice, st_));
-			DG_CUDA(cudaMemcpyAsync(Ls_.buf[l], old.buf[l], bytes, cudaMemcpyDeviceToDevice, st_));
+			keep(Ls_.clu[l], old.clu[l], h_cnt_->clu[l]);
+			keep(Ls_.buf[l], old.buf[l], h_cnt_->buf[l]);
 		}
-		// the per-substep lists too: the pool can grow between the indicator and the split
-		for (auto pr: {std::make_pair(Ls_.tmp, old.tmp), std::make_pair(Ls_.recv, old.recv),
-		               std::make_pair(Ls_.split, old.split), std::make_pair(Ls_.unsplit, old.unsplit),
-		               std::make_pair(Ls_.fresh, old.fresh), std::make_pair(Ls_.upd, old.upd)})
-			DG_CUDA(cudaMemcpyAsync(pr.first, pr.second, bytes, cudaMemcpyDeviceToDevice, st_));
-		DG_CUDA(cudaStreamSynchronize(st_));
-		cudaFree(old_mem);
+		// the pool can grow between the indicator and the split, whose requests are the only list of a
+		// substep in use there
+		keep(Ls_.split, old.split, h_cnt_->n_split);
+		mem_free(old_mem, st_);
 	}
 
 	int list_cap_ = 0;
 	void alloc_lists(int cap) {
 		const int nlists = 2 * MAX_ACTI + 6;
 		size_t one       = align_up(sizeof(int32_t) * (size_t) cap);
-		DG_CUDA(cudaMalloc(&list_mem_, one * nlists));
+		DG_CUDA(mem_alloc((void **) &list_mem_, one * nlists, st_));
 		char *b = (char *) list_mem_;
 		for (int l = 0; l < MAX_ACTI; ++l) {
 			Ls_.clu[l] = (int32_t *) b;
@@ -592,7 +622,7 @@ public:
 	// Integrator constructor body (integrator/integrator.hpp:100-160).
 	void construct() {
 		const int n = (int) active_leaves_.size();
-		DG_CUDA(cudaMalloc(&d_leaves_, sizeof(int32_t) * (n > 0 ? n : 1)));
+		DG_CUDA(mem_alloc((void **) &d_leaves_, sizeof(int32_t) * (n > 0 ? n : 1), st_));
 		DG_CUDA(cudaMemcpy(d_leaves_, active_leaves_.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
 		const int g = grid_for(n);
 		k_init_cells<M><<<g, BLOCK, 0, st_>>>(P_, C_, d_leaves_, n, d_cnt_);
@@ -611,7 +641,7 @@ public:
 		DG_CUDA(cudaGetLastError());
 		sync_counters();
 		check_status();
-		cudaFree(d_leaves_);  // the constructor's list of every leaf is not used again
+		mem_free(d_leaves_, st_);  // the constructor's list of every leaf is not used again
 		d_leaves_ = nullptr;
 		max_acti_ = 0;
 		for (int l = 0; l < MAX_ACTI; ++l)
@@ -759,8 +789,16 @@ private:
 	void grow_for_splits() {
 		const long long need = (long long) h_cnt_->top + (long long) NC * h_cnt_->n_split + 16;
 		if (need <= P_.cap) return;
-		const long long want = growth_target(need, std::max(need + need / 4, (long long) P_.cap * 5 / 4));
+		const long long want = growth_target(need, grown(need));
 		grow_pool((int) std::min<long long>(want, 2000000000LL));
+	}
+
+	// The capacity wanted when `need` slots must fit: a quarter more, and twice the old one while that is small
+	// (a growth costs about 0.3 ms whatever the size, and a tree that refines from a coarse grid grows ten times
+	// its size within a few steps).
+	long long grown(long long need) {
+		const long long cap = P_.cap;
+		return std::max(need + need / 4, pool_bytes(P_) < SECOND_POOL_MAX / 8 ? cap * 2 : cap * 5 / 4);
 	}
 
 	void substep_tail(int L, int n) {
@@ -1036,15 +1074,20 @@ public:
 		const int n   = top - 1;
 		if (n <= 0) return;
 		ensure_spare();
+		int bits = D * max_tree_level_;
+		while (bits < 31 && (1 << bits) <= top) ++bits;
+		const int end_bit = bits + SORT_CODE_BITS;
 		size_t temp = 0;
 		DG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp, (uint64_t *) nullptr, (uint64_t *) nullptr,
-		                                        (int32_t *) nullptr, (int32_t *) nullptr, n, 0, 64, st_));
+		                                        (int32_t *) nullptr, (int32_t *) nullptr, n, 0, end_bit, st_));
 		const size_t need = align_up(sizeof(uint64_t) * n) * 2 + align_up(sizeof(int32_t) * n) * 2 +
 		                    align_up(sizeof(int32_t) * (top + 1)) + align_up(temp);
 		if (need > sort_bytes_) {
-			cudaFree(sort_mem_);
-			DG_CUDA(cudaMalloc(&sort_mem_, need));
-			sort_bytes_ = need;
+			mem_free(sort_mem_, st_);
+			sort_mem_   = nullptr;
+			sort_bytes_ = 0;
+			DG_CUDA(mem_alloc((void **) &sort_mem_, need + need / 2, st_));
+			sort_bytes_ = need + need / 2;
 		}
 		char *b          = (char *) sort_mem_;
 		uint64_t *k_in   = (uint64_t *) b;
@@ -1059,38 +1102,61 @@ public:
 		b += align_up(sizeof(int32_t) * (top + 1));
 		void *tmp = b;
 		const int g = grid_for(n);
-		run_k(DG_K_OTHER, 0, [&] { k_sort_keys<D><<<g, BLOCK, 0, st_>>>(P_, top, k_in, v_in); });
-		DG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, temp, k_in, k_out, v_in, v_out, n, 0, 64, st_));
+		run_k(DG_K_OTHER, 0, [&] { k_sort_keys<D><<<g, BLOCK, 0, st_>>>(P_, top, max_tree_level_, bits, k_in, v_in); });
+		DG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, temp, k_in, k_out, v_in, v_out, n, 0, end_bit, st_));
 		run_k(DG_K_OTHER, 0, [&] { k_sort_inverse<<<g, BLOCK, 0, st_>>>(v_out, n, newidx); });
-		// each field in turn: permuted into the spare buffer, then copied back over slots [1, top)
-		auto fo = fields(P_);
-		for (size_t k = 0; k < fo.size(); ++k) {
-			const int comps = fo[k].comps;
-			if (comps <= 0) continue;
-			const size_t elem = fo[k].elem;
-			void *src = *fo[k].ptr, *dst = spare_mem_;
+		auto rows = [&](const RowTable &t) {
+			run_k(DG_K_OTHER, 0, [&] { k_rows<<<dim3(grid_for(top, 148 * 4), t.n), BLOCK, 0, st_>>>(t, top, v_out, newidx); });
+		};
+		auto words = [&](const Field &f, const void *src, void *dst) {
 			run_k(DG_K_OTHER, 0, [&] {
-				switch (elem) {
-					case 1: k_permute<int8_t><<<g, BLOCK, 0, st_>>>((const int8_t *) src, (int8_t *) dst, comps, P_.cap, n, v_out); break;
-					case 2: k_permute<int16_t><<<g, BLOCK, 0, st_>>>((const int16_t *) src, (int16_t *) dst, comps, P_.cap, n, v_out); break;
-					case 4: k_permute<int32_t><<<g, BLOCK, 0, st_>>>((const int32_t *) src, (int32_t *) dst, comps, P_.cap, n, v_out); break;
-					case 8: k_permute<double><<<g, BLOCK, 0, st_>>>((const double *) src, (double *) dst, comps, P_.cap, n, v_out); break;
-					default:  // one record of elem bytes per node
-						k_permute_words<<<grid_for((long long) n * (elem / 8)), BLOCK, 0, st_>>>(
-						    (const double *) src, (double *) dst, (int) (elem / 8), n, v_out);
-						break;
-				}
+				k_row_words<<<grid_for((long long) top * (f.elem / 8)), BLOCK, 0, st_>>>((const double *) src, (double *) dst,
+				                                                                        (int) (f.elem / 8), top, v_out);
 			});
-			DG_CUDA(cudaMemcpy2DAsync((char *) src + elem, elem * (size_t) P_.cap, (const char *) dst + elem,
-			                          elem * (size_t) P_.cap, elem * (size_t) n, comps, cudaMemcpyDeviceToDevice, st_));
+		};
+		auto fo = fields(P_);
+		if (second_pool()) {
+			if (spare_dirty_) DG_CUDA(cudaMemsetAsync(spare_mem_, 0, pool_bytes(P_), st_));
+			spare_dirty_ = false;
+			Pool NP      = P_;
+			place_fields(NP, spare_mem_);
+			auto fn = fields(NP);
+			RowTable t{};
+			for (size_t k = 0; k < fo.size(); ++k) {
+				if (fo[k].comps <= 0 || fo[k].stay) continue;
+				if (fo[k].elem > 8) words(fo[k], *fo[k].ptr, *fn[k].ptr);
+				else add_rows(t, fo[k], *fo[k].ptr, P_.cap, *fn[k].ptr, P_.cap, true);
+			}
+			rows(t);
+			std::swap(pool_mem_, spare_mem_);
+			spare_bytes_ = pool_bytes(P_);
+			P_           = NP;
+		} else {
+			// each field in turn: permuted into the spare buffer, then copied back over slots [1, top)
+			for (size_t k = 0; k < fo.size(); ++k) {
+				const int comps   = fo[k].comps;
+				const size_t elem = fo[k].elem;
+				if (comps <= 0 || fo[k].stay) continue;
+				if (elem > 8) {
+					words(fo[k], *fo[k].ptr, spare_mem_);
+				} else {
+					RowTable t{};
+					add_rows(t, fo[k], *fo[k].ptr, P_.cap, spare_mem_, P_.cap, true);
+					rows(t);
+				}
+				DG_CUDA(cudaMemcpy2DAsync((char *) *fo[k].ptr + elem, elem * (size_t) P_.cap, (const char *) spare_mem_ + elem,
+				                          elem * (size_t) P_.cap, elem * (size_t) n, comps, cudaMemcpyDeviceToDevice, st_));
+			}
 		}
-		run_k(DG_K_OTHER, 0, [&] { k_remap_links<D><<<grid_for(top), BLOCK, 0, st_>>>(P_, top, newidx); });
-		int first = 1;
+		LevelRanges r{};
+		int most   = 0;
+		r.first[0] = 1;
 		for (int l = 0; l < MAX_ACTI; ++l) {
-			const int cnt = h_cnt_->clu[l];
-			if (cnt > 0) run_k(DG_K_OTHER, 0, [&] { k_fill_range<<<grid_for(cnt), BLOCK, 0, st_>>>(Ls_.clu[l], first, cnt); });
-			first += cnt;
+			r.list[l]      = Ls_.clu[l];
+			r.first[l + 1] = r.first[l] + h_cnt_->clu[l];
+			most           = std::max(most, h_cnt_->clu[l]);
 		}
+		run_k(DG_K_OTHER, 0, [&] { k_fill_ranges<<<dim3(grid_for(most), MAX_ACTI), BLOCK, 0, st_>>>(r); });
 		DG_CUDA(cudaGetLastError());
 		sync_counters();
 	}
@@ -1103,14 +1169,14 @@ private:
 		for (int l = 0; l < MAX_ACTI; ++l)
 			if (h_cnt_->buf[l] != 0) throw dg_error(DG_ERR_UNSUPPORTED, "garbage collection with non-empty ACTI buffers");
 		int32_t *keep = nullptr, *newidx = nullptr;
-		DG_CUDA(cudaMalloc(&keep, sizeof(int32_t) * (top + 1)));
-		DG_CUDA(cudaMalloc(&newidx, sizeof(int32_t) * (top + 1)));
+		DG_CUDA(mem_alloc((void **) &keep, sizeof(int32_t) * (top + 1), st_));
+		DG_CUDA(mem_alloc((void **) &newidx, sizeof(int32_t) * (top + 1), st_));
 		const int g = grid_for(top);
 		k_gc_keep<<<g, BLOCK, 0, st_>>>(P_, top, keep);
 		size_t tmp_bytes = 0;
 		DG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, keep, newidx, top + 1, st_));
 		void *tmp = nullptr;
-		DG_CUDA(cudaMalloc(&tmp, tmp_bytes));
+		DG_CUDA(mem_alloc((void **) &tmp, tmp_bytes, st_));
 		DG_CUDA(cudaMemsetAsync(keep + top, 0, sizeof(int32_t), st_));
 		DG_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, keep, newidx, top + 1, st_));
 		int new_top = 0;
@@ -1118,6 +1184,7 @@ private:
 		// each field in turn: kept slots compacted into the zeroed spare buffer, which is then copied back
 		// whole (slots from new_top on end up zero)
 		ensure_spare();
+		spare_dirty_ = true;
 		auto fo = fields(P_);
 		for (size_t k = 0; k < fo.size(); ++k) {
 			if (fo[k].comps <= 0) continue;
@@ -1148,9 +1215,9 @@ private:
 		DG_CUDA(cudaGetLastError());
 		sync_counters();
 		check_status();
-		cudaFree(tmp);
-		cudaFree(keep);
-		cudaFree(newidx);
+		mem_free(tmp, st_);
+		mem_free(keep, st_);
+		mem_free(newidx, st_);
 		n_gc_++;
 	}
 
@@ -1166,10 +1233,10 @@ public:
 		long long n = cell_count();
 		if (n > max_cells) throw dg_error(DG_ERR_ARG, "read buffer too small");
 		if (n > read_cap_) {
-			cudaFree(d_read_);
-			cudaFree(d_readlv_);
-			DG_CUDA(cudaMalloc(&d_read_, sizeof(double) * W * n));
-			DG_CUDA(cudaMalloc(&d_readlv_, sizeof(int32_t) * 2 * n));
+			mem_free(d_read_, st_);
+			mem_free(d_readlv_, st_);
+			DG_CUDA(mem_alloc((void **) &d_read_, sizeof(double) * W * n, st_));
+			DG_CUDA(mem_alloc((void **) &d_readlv_, sizeof(int32_t) * 2 * n, st_));
 			read_cap_ = n;
 		}
 		long long base = 0;
@@ -1195,7 +1262,7 @@ public:
 		const long long n = cell_count();
 		if (n > max_cells) throw dg_error(DG_ERR_ARG, "read buffer too small");
 		double *d_out = nullptr;
-		DG_CUDA(cudaMalloc(&d_out, sizeof(double) * width * (n > 0 ? n : 1)));
+		DG_CUDA(mem_alloc((void **) &d_out, sizeof(double) * width * (n > 0 ? n : 1), st_));
 		long long base = 0;
 		for (int pass = 0; pass < 2; ++pass) {
 			for (int l = 0; l < MAX_ACTI; ++l) {
@@ -1208,7 +1275,7 @@ public:
 		cudaError_t e = cudaGetLastError();
 		if (e == cudaSuccess && n > 0) e = cudaMemcpyAsync(data, d_out, sizeof(double) * width * n, cudaMemcpyDeviceToHost, st_);
 		if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-		cudaFree(d_out);
+		mem_free(d_out, st_);
 		if (e != cudaSuccess) throw dg_error(DG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 		return n;
 	}
@@ -1266,7 +1333,7 @@ public:
 	void set_hold(const uint8_t *hold, long long n) override {
 		if (n != cell_count()) throw dg_error(DG_ERR_ARG, "dg_set_hold: one entry per active cell expected");
 		uint8_t *d = nullptr;
-		DG_CUDA(cudaMalloc(&d, n > 0 ? n : 1));
+		DG_CUDA(mem_alloc((void **) &d, n > 0 ? n : 1, st_));
 		cudaError_t e = n > 0 ? cudaMemcpyAsync(d, hold, n, cudaMemcpyHostToDevice, st_) : cudaSuccess;
 		long long base = 0;
 		for (int pass = 0; e == cudaSuccess && pass < 2; ++pass) {
@@ -1279,7 +1346,7 @@ public:
 		}
 		if (e == cudaSuccess) e = cudaGetLastError();
 		if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-		cudaFree(d);
+		mem_free(d, st_);
 		if (e != cudaSuccess) throw dg_error(DG_ERR_CUDA, std::string("set_hold: ") + cudaGetErrorString(e));
 	}
 	void set_coarsen_interval(int k) override {

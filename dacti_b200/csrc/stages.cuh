@@ -2047,26 +2047,28 @@ __device__ __forceinline__ uint64_t spread3(uint64_t x) {  // 19 bits -> every t
 	return x;
 }
 
+constexpr int SORT_OTHERS = MAX_ACTI;  // sort code of the slots that are in no cluster
+constexpr int SORT_CODE_BITS = 5;      // of the codes 0 .. SORT_OTHERS
+
+// Keys of `bits` low bits under the cluster: the Morton code of the cell's corner at tree level `top_level`
+// (D * top_level <= bits), or, for a slot in no cluster, its number, behind all clusters. A sort over the
+// bits in use takes half the passes of one over 64 (29 bits instead of 64 for 3D trees of 8 levels).
 template<int D>
-__global__ void k_sort_keys(Pool P, int top, uint64_t *keys, int32_t *vals) {
-	constexpr int LMAX = D == 2 ? 29 : 19;
+__global__ void k_sort_keys(Pool P, int top, int top_level, int bits, uint64_t *keys, int32_t *vals) {
 	for (int j = gtid(); j < top - 1; j += gstride()) {
 		const int i     = j + 1;
 		const int8_t cl = P.clu[i];
-		uint64_t code   = cl >= 0 ? (uint64_t) cl : 63ull;
-		uint64_t m      = 0;
+		uint64_t code   = cl >= 0 ? (uint64_t) cl : (uint64_t) SORT_OTHERS;
+		uint64_t m      = (uint64_t) i;
 		if (cl >= 0) {
-			const int l  = P.level[i];
-			const int sh = LMAX - l;
+			const int sh = max(top_level - P.level[i], 0);
+			m            = 0;
 			for (int d = 0; d < D; ++d) {
-				uint64_t c = (uint64_t) P.coord[(size_t) d * P.cap + i];
-				c          = sh >= 0 ? (c << sh) : (c >> (-sh));
+				const uint64_t c = (uint64_t) P.coord[(size_t) d * P.cap + i] << sh;
 				m |= (D == 2 ? spread2(c) : spread3(c)) << d;
 			}
-		} else {
-			m = (uint64_t) i;
 		}
-		keys[j] = (code << 58) | (m & ((1ull << 58) - 1));
+		keys[j] = (code << bits) | m;
 		vals[j] = i;
 	}
 }
@@ -2076,34 +2078,46 @@ static __global__ void k_sort_inverse(const int32_t *sorted_vals, int n, int32_t
 	if (gtid() == 0) newidx[0] = 0;
 }
 
-template<typename T>
-__global__ void k_permute(const T *__restrict__ src, T *__restrict__ dst, int comps, int cap, int n,
-                          const int32_t *__restrict__ perm) {
+// Rows of pool slots copied together: one entry per stored component, `link` for a component that holds
+// slot numbers.
+struct RowTable {
+	static constexpr int MAX = 120;
+	struct Row {
+		const char *src;
+		char *dst;
+		int elem, link;
+	} r[MAX];
+	int n;
+};
+
+// Every row of the table in one launch, one row per blockIdx.y, slots [0, n): slot 0, the null node, stays, and
+// slot j takes slot perm[j - 1] of src (without perm, slot j); links go through newidx (old slot -> new slot).
+// A field at a time, with a copy back, was some seventy launches a re-sort, which small trees notice.
+static __global__ void k_rows(const __grid_constant__ RowTable t, int n, const int32_t *__restrict__ perm,
+                              const int32_t *__restrict__ newidx) {
+	const RowTable::Row &r = t.r[blockIdx.y];
 	for (int j = gtid(); j < n; j += gstride()) {
-		const int o = perm[j];
-		for (int c = 0; c < comps; ++c) dst[(size_t) c * cap + j + 1] = src[(size_t) c * cap + o];
+		const size_t o = perm && j > 0 ? perm[j - 1] : j, d = j;
+		if (r.elem == 8) {
+			reinterpret_cast<double *>(r.dst)[d] = reinterpret_cast<const double *>(r.src)[o];
+		} else if (r.elem == 4) {
+			const int32_t v = reinterpret_cast<const int32_t *>(r.src)[o];
+			reinterpret_cast<int32_t *>(r.dst)[d] = r.link ? newidx[v] : v;
+		} else if (r.elem == 2) {
+			reinterpret_cast<int16_t *>(r.dst)[d] = reinterpret_cast<const int16_t *>(r.src)[o];
+		} else {
+			r.dst[d] = r.src[o];
+		}
 	}
 }
 
-// Permutation of a field holding one record of w 8-byte words per node: word-parallel copies.
-static __global__ void k_permute_words(const double *__restrict__ src, double *__restrict__ dst, int w, int n,
-                                       const int32_t *__restrict__ perm) {
+// A field holding one record of w 8-byte words per node, in the same order: word-parallel copies.
+static __global__ void k_row_words(const double *__restrict__ src, double *__restrict__ dst, int w, int n,
+                                   const int32_t *__restrict__ perm) {
 	const long long total = (long long) n * w;
 	for (long long t = gtid(); t < total; t += gstride()) {
 		const int j = (int) (t / w), k = (int) (t % w);
-		dst[(size_t) (j + 1) * w + k] = src[(size_t) perm[j] * w + k];
-	}
-}
-
-template<int D>
-__global__ void k_remap_links(Pool P, int top, const int32_t *newidx) {
-	constexpr int NC = 1 << D, NF = 2 * D;
-	const int cap = P.cap;
-	for (int j = gtid(); j < top; j += gstride()) {
-		if (j == 0) continue;
-		P.parent[j] = newidx[P.parent[j]];
-		for (int c = 0; c < NC; ++c) P.child[(size_t) c * cap + j] = newidx[P.child[(size_t) c * cap + j]];
-		for (int f = 0; f < NF; ++f) P.nbr[(size_t) f * cap + j] = newidx[P.nbr[(size_t) f * cap + j]];
+		dst[t] = src[(size_t) (j > 0 ? perm[j - 1] : 0) * w + k];
 	}
 }
 
@@ -2111,8 +2125,14 @@ static __global__ void k_fill_i32(int32_t *a, int v, int n) {
 	for (int j = gtid(); j < n; j += gstride()) a[j] = v;
 }
 
-static __global__ void k_fill_range(int32_t *list, int first, int n) {
-	for (int j = gtid(); j < n; j += gstride()) list[j] = first + j;
+// The level lists after a re-sort: list l is the slots first[l] .. first[l + 1], one level per blockIdx.y.
+struct LevelRanges {
+	int32_t *list[MAX_ACTI];
+	int first[MAX_ACTI + 1];
+};
+static __global__ void k_fill_ranges(const __grid_constant__ LevelRanges r) {
+	const int l = blockIdx.y, n = r.first[l + 1] - r.first[l];
+	for (int j = gtid(); j < n; j += gstride()) r.list[l][j] = r.first[l] + j;
 }
 
 }  // namespace dg
