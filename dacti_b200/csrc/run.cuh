@@ -60,19 +60,21 @@ struct RunArgs {
 
 constexpr int RUN_THREADS = 512;
 
-// The chunk of warp items of one block of a run: block b of nb takes the b-th of nb equal ranges, so that
-// any item count spreads over all blocks and a block's cells are neighbours in the list. `rev` hands the
-// items to the block's warps from the last one on, for the second of two stages that share a barrier: with
+// The warp items of a run: dealt out over the blocks one by one, so that few items spread over all SMs and the
+// cells with long walks (hanging faces, subtree means), which lie side by side in the list, do not meet in one
+// block: the slowest block ends a stage (2 to 3% on the small cases against contiguous chunks). `rev` hands
+// the items to the blocks' warps from the last one on, for the second of two stages that share a barrier: with
 // few items the two then run on different warps instead of one after the other.
-struct ChunkGrid {
+struct DealtGrid {
+	static constexpr bool DEEP = true;
 	int block, blocks;
 	bool rev;
-	__device__ __forceinline__ int begin(int items) const {
+	__device__ __forceinline__ int begin(int) const {
 		const int w = threadIdx.x >> 5;
-		return (int) ((long long) items * block / blocks) + (rev ? RUN_THREADS / 32 - 1 - w : w);
+		return (rev ? RUN_THREADS / 32 - 1 - w : w) * blocks + block;
 	}
-	__device__ __forceinline__ int end(int items) const { return (int) ((long long) items * (block + 1) / blocks); }
-	__device__ __forceinline__ int step() const { return RUN_THREADS / 32; }
+	__device__ __forceinline__ int end(int items) const { return items; }
+	__device__ __forceinline__ int step() const { return blocks * (RUN_THREADS / 32); }
 };
 
 // A wait longer than this many polls (seconds) gives up, marks the status and ends the run.
@@ -104,14 +106,14 @@ __device__ __forceinline__ bool run_barrier(const RunArgs &a, unsigned &arrivals
 	return *s_ok;
 }
 
-// The cluster's reassignment for a run: the cells that stay are listed block by block in their list order
-// (one reservation per block of RUN_THREADS cells), so that neighbours in the list stay neighbours.
+// The cluster's reassignment for a run: the cells that stay are listed chunk by chunk in their list order
+// (a contiguous chunk per block, one reservation per block of RUN_THREADS cells), so that neighbours in the list stay neighbours.
 template<class M>
-__device__ __forceinline__ void run_reassign(const ChunkGrid &g, const Pool &P, const Consts &C, const int32_t *list, int n, int L,
+__device__ __forceinline__ void run_reassign(const DealtGrid &g, const Pool &P, const Consts &C, const int32_t *list, int n, int L,
                                              double dtL, int counter_L, const Lists &Ls, Counters *cnt, int *s_warp /*[33]*/) {
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = RUN_THREADS / 32;
 	const int items = warp_items(n, 32);
-	const int first = (int) ((long long) items * g.block / g.blocks), last = g.end(items);
+	const int first = (int) ((long long) items * g.block / g.blocks), last = (int) ((long long) items * (g.block + 1) / g.blocks);
 	for (int base = first; base < last; base += nw) {
 		const int tid  = (base + w) * 32 + lane;
 		const bool in  = base + w < last && tid < n;
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 	const int top_seq = 1 << (MAX_ACTI - 1);
 	unsigned arrivals = 0;
 	const bool lead   = threadIdx.x == 0;
-	const ChunkGrid g{(int) blockIdx.x, (int) gridDim.x, false}, r{(int) blockIdx.x, (int) gridDim.x, true};
+	const DealtGrid g{(int) blockIdx.x, (int) gridDim.x, false}, r{(int) blockIdx.x, (int) gridDim.x, true};
 
 	if (lead) {
 		s     = a.state->sch;
@@ -266,10 +268,13 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 			__syncthreads();
 			break;
 		}
-		// a split cell and the family of a coarsened one have no cell in common
-		d_split<M>(g, P, C, &cnt->n_split, s_ls.split, L, s_ls.fresh, epoch0 + EX + 1, cnt);
-		d_coarsen<M>(r, P, C, list, n, L, s_ls.fresh, epoch0 + EX + 2, cnt);
-		if (!run_barrier(a, arrivals, &s_ok)) return;
+		const bool cand = counter_L == 1 && C.coarsen;  // when d_estimate may make candidates
+		if (n_split > 0 || cand) {
+			// a split cell and the family of a coarsened one have no cell in common
+			d_split<M>(g, P, C, &cnt->n_split, s_ls.split, L, s_ls.fresh, epoch0 + EX + 1, cnt);
+			if (cand) d_coarsen<M>(r, P, C, list, n, L, s_ls.fresh, epoch0 + EX + 2, cnt);
+			if (!run_barrier(a, arrivals, &s_ok)) return;
+		}
 		// the neighbour repair reads no time level and the reassignment no neighbour
 		const int n_new = __ldcg(&cnt->n_new);
 		d_nbr_fresh<M>(r, P, C, &cnt->n_new, s_ls.fresh, s_ls.upd, cnt);

@@ -615,8 +615,12 @@ public:
 		active_leaves_.clear();
 		for (int i = 1; i < n; ++i)
 			if ((c.flags[i] & DG_F_LEAF) && (c.flags[i] & DG_F_ACTIVE)) active_leaves_.push_back(i);
-		h_cnt_->top = n;
+		int coarsest = MAX_TREE;
+		for (int i: active_leaves_) coarsest = std::min(coarsest, (int) c.level[i]);
+		h_cnt_->top      = n;
+		h_cnt_->coarsest = coarsest;
 		DG_CUDA(cudaMemcpy(&d_cnt_->top, &n, sizeof(int), cudaMemcpyHostToDevice));
+		DG_CUDA(cudaMemcpy(&d_cnt_->coarsest, &coarsest, sizeof(int), cudaMemcpyHostToDevice));
 	}
 
 	// Integrator constructor body (integrator/integrator.hpp:100-160).
@@ -1200,6 +1204,7 @@ private:
 		Counters z{};
 		z.top    = new_top;
 		z.status = 0;
+		z.coarsest = h_cnt_->coarsest;
 		// the running totals that a batched step keeps on the device carry over (the host copy is current:
 		// gc runs after the step's last read-back)
 		z.n_split_total    = h_cnt_->n_split_total;

@@ -25,11 +25,13 @@ __device__ __forceinline__ int gstride() { return gridDim.x * blockDim.x; }
 // Which warp-sized work items a warp of a stage takes: items [begin, end) in steps of step(). A launch of
 // its own walks the whole grid; a batched launch gives each tree a range of blocks.
 struct PlainGrid {
+	static constexpr bool DEEP = false;  // interp_pt's
 	__device__ __forceinline__ int begin(int) const { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
 	__device__ __forceinline__ int end(int items) const { return items; }
 	__device__ __forceinline__ int step() const { return (gridDim.x * blockDim.x) >> 5; }
 };
 struct BlockRange {
+	static constexpr bool DEEP = false;
 	int first, count;  // blocks [first, first + count) of the launch
 	__device__ __forceinline__ int begin(int) const { return (((int) blockIdx.x - first) * blockDim.x + threadIdx.x) >> 5; }
 	__device__ __forceinline__ int end(int items) const { return items; }
@@ -738,6 +740,7 @@ __device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Con
 	constexpr int E = M::E;
 	const int cap  = P.cap;
 	const int lane = threadIdx.x & 31;
+	const int coarsest = __ldcg(&cnt->coarsest);
 	// warp-uniform loop: the whole warp stamps the updated cells' ancestors together
 	const int items = warp_items(n, 32);
 	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
@@ -806,7 +809,7 @@ __device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Con
 			P.t[i] = P.t[i] + dtL;
 			up     = P.parent[i];
 		}
-		mark_up_warp(P, up, epoch);
+		mark_up_warp(P, up, epoch, coarsest);
 	}
 }
 template<class M, bool V>
@@ -828,7 +831,7 @@ __device__ __forceinline__ int nb_acti(int32_t code) { return ((code >> 16) & 0x
 // impl/adaptive_refinement.hpp:16-60): the neighbour's primitive state and time (its own, or the mean
 // over a non-leaf neighbour's subtree, integrator/domain.hpp:84-148) and the centre distance
 // 0.5 (h + h_n); returns the neighbour facts, 0 when the face has no neighbour.
-template<class M>
+template<class M, bool DEEP>
 __device__ __forceinline__ int32_t neighbour_value(const Pool &P, const Consts &C, uint32_t *status, int i, int f, int epoch,
                                                    double *v /*[E]*/, double &tv, double &dist) {
 	constexpr int E = M::E;
@@ -838,7 +841,7 @@ __device__ __forceinline__ int32_t neighbour_value(const Pool &P, const Consts &
 	const int ln      = P.level[nb];
 	double w[E + 1];
 	if (!(fl & F_LEAF)) {
-		interp_pt<M>(P, status, nb, epoch, w);
+		interp_pt<M, DEEP>(P, status, nb, epoch, w);
 	} else {
 		load_p_rec<M>(P, nb, w);
 		w[E] = P.t[nb];
@@ -888,7 +891,7 @@ __device__ __forceinline__ void d_slope(const Grid &g, const Pool &P, const Cons
 		if (active && sub < NF) {
 			const int f = sub, dir = f & 1;
 			double dist;
-			const int32_t code = neighbour_value<M>(P, C, &cnt->status, i, f, epoch, pv, tv, dist);
+			const int32_t code = neighbour_value<M, Grid::DEEP>(P, C, &cnt->status, i, f, epoch, pv, tv, dist);
 			if (!(code & NB_PRESENT)) {
 				const int b = P.bc[(size_t) f * cap + i];
 				if (b < 0) {
@@ -1029,7 +1032,7 @@ __device__ __forceinline__ void d_estimate(const Grid &g, const Pool &P, const C
 		if (active && sub < NF) {
 			const int f = sub, dim = f >> 1, dir = f & 1;
 			double tv, dist;
-			code = neighbour_value<M>(P, C, &cnt->status, i, f, epoch, v, tv, dist);
+			code = neighbour_value<M, Grid::DEEP>(P, C, &cnt->status, i, f, epoch, v, tv, dist);
 			if ((code & NB_PRESENT) && (code & NB_LEAF) && nb_level(code) < li) {
 				// a coarser leaf: its state extrapolated to the same-level position
 				const int nb   = P.nbr[(size_t) f * cap + i];
@@ -1235,7 +1238,7 @@ __device__ __forceinline__ void d_split(const Grid &g, const Pool &P, const Cons
 		__syncwarp();
 		if (active && !fail && c == 0) {
 			P.flags[par] &= ~(F_LEAF | F_SHOULD_SPLIT);
-			mark_up(P, par, epoch);
+			mark_up(P, par, epoch, __ldcg(&cnt->coarsest));
 		}
 	}
 }
@@ -1300,7 +1303,8 @@ __device__ __forceinline__ void unsplit_cell(const Pool &P, const Consts &C, int
 	P.acti[par]  = (int8_t) L;
 	P.clu[par]   = (int8_t) L;
 	append(fresh, &cnt->n_new, par, cap, &cnt->status);
-	mark_up(P, P.parent[par], epoch);
+	if (P.level[par] < __ldcg(&cnt->coarsest)) atomicMin(&cnt->coarsest, (int) P.level[par]);
+	mark_up(P, P.parent[par], epoch, __ldcg(&cnt->coarsest));
 }
 template<class M, class Grid>
 __device__ __forceinline__ void d_unsplit(const Grid &g, const Pool &P, const Consts &C, const int *n_ptr, const int32_t *unsplit_list, int L, int32_t *fresh, int epoch, Counters *cnt) {

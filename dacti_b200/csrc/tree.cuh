@@ -105,8 +105,84 @@ __device__ __forceinline__ bool memo_ok(const Pool &P, int n, int epoch) {
 	return c > __ldcg(P.mod + n) && c < epoch;
 }
 
-// Mean primitive state and time of node n ({p[E], t} in out); `epoch` is the calling kernel's.
+// The mean of a non-leaf node with leaves only below it, memoised; false (nothing done) where it has others.
+// Links, flags and records of the children are read side by side (slot 0, an inactive leaf, stands in for a
+// missing child) and added in slot order.
 template<class M>
+__device__ __forceinline__ bool mean_flat(const Pool &P, int n, int epoch, double *out) {
+	constexpr int E = M::E, NC = 1 << M::D;
+	int ch[NC];
+	uint32_t fl[NC];
+	bool flat = true;
+#pragma unroll
+	for (int k = 0; k < NC; ++k) ch[k] = P.child[(size_t) k * P.cap + n];
+#pragma unroll
+	for (int k = 0; k < NC; ++k) fl[k] = P.flags[ch[k]];
+#pragma unroll
+	for (int k = 0; k < NC; ++k) flat = flat && (fl[k] & (F_ACTIVE | F_LEAF)) != F_ACTIVE;
+	if (!flat) return false;
+	int cnt = 0;
+	double f[E + 1];
+#pragma unroll
+	for (int q = 0; q <= E; ++q) f[q] = 0.0;
+#pragma unroll
+	for (int k = 0; k < NC; ++k) {
+		double pc[E];
+		load_p_rec<M>(P, ch[k], pc);
+		const double tc = P.t[ch[k]];
+		const bool act  = fl[k] & F_ACTIVE;
+		cnt += act;
+#pragma unroll
+		for (int q = 0; q < E; ++q) f[q] = act ? f[q] + pc[q] : f[q];
+		f[E] = act ? f[E] + tc : f[E];
+	}
+	double *memo = P.avg + (size_t) n * Avg<M>::W;
+#pragma unroll
+	for (int q = 0; q <= E; ++q) memo[q] = out[q] = f[q] / (double) cnt;
+	P.cst[n] = epoch;
+	return true;
+}
+
+// The same for a node whose children are leaves, memoised, or have leaves only below them: with neighbours at
+// most one level finer that is nearly every node asked for. The general walk keeps a stack in local memory.
+template<class M>
+__device__ __noinline__ bool mean_two_levels(const Pool &P, int n, int epoch, double *out) {
+	constexpr int E = M::E, NC = 1 << M::D, AW = Avg<M>::W;
+	if (mean_flat<M>(P, n, epoch, out)) return true;
+	int cnt = 0;
+	double f[E + 1];
+#pragma unroll
+	for (int q = 0; q <= E; ++q) f[q] = 0.0;
+#pragma unroll 1
+	for (int k = 0; k < NC; ++k) {
+		const int c       = P.child[(size_t) k * P.cap + n];
+		const uint32_t fl = P.flags[c];
+		if (!(fl & F_ACTIVE)) continue;
+		double v[E + 1];
+		if (fl & F_LEAF) {
+			load_p_rec<M>(P, c, v);
+			v[E] = P.t[c];
+		} else if (memo_ok(P, c, epoch)) {
+#pragma unroll
+			for (int q = 0; q <= E; ++q) v[q] = __ldcg(P.avg + (size_t) c * AW + q);
+		} else if (!mean_flat<M>(P, c, epoch, v)) {
+			return false;
+		}
+#pragma unroll
+		for (int q = 0; q <= E; ++q) f[q] = f[q] + v[q];
+		cnt++;
+	}
+	double *memo = P.avg + (size_t) n * AW;
+#pragma unroll
+	for (int q = 0; q <= E; ++q) memo[q] = out[q] = f[q] / (double) cnt;
+	P.cst[n] = epoch;
+	return true;
+}
+
+// Mean primitive state and time of node n ({p[E], t} in out); `epoch` is the calling kernel's.
+// `DEEP` tries the two-level form before the general walk: shorter for the slowest lane of a run's stage, but the
+// call costs the stage launches occupancy (the indicator of drop3d_large 104 ms a step with it, 54 without).
+template<class M, bool DEEP>
 __device__ void interp_pt(const Pool &P, uint32_t *status, int n, int epoch, double *out) {
 	constexpr int E = M::E, NC = 1 << M::D, AW = Avg<M>::W;
 	if (P.flags[n] & F_LEAF) {
@@ -118,38 +194,10 @@ __device__ void interp_pt(const Pool &P, uint32_t *status, int n, int epoch, dou
 		for (int q = 0; q <= E; ++q) out[q] = __ldcg(P.avg + (size_t) n * AW + q);
 		return;
 	}
-	// Nearly every node asked for has leaves only below it: their links, flags and records are read side by
-	// side (slot 0, an inactive leaf, stands in for a missing child) and added in slot order.
-	int ch[NC];
-	uint32_t fl[NC];
-	bool flat = true;
-#pragma unroll
-	for (int k = 0; k < NC; ++k) ch[k] = P.child[(size_t) k * P.cap + n];
-#pragma unroll
-	for (int k = 0; k < NC; ++k) fl[k] = P.flags[ch[k]];
-#pragma unroll
-	for (int k = 0; k < NC; ++k) flat = flat && (fl[k] & (F_ACTIVE | F_LEAF)) != F_ACTIVE;
-	if (flat) {
-		int cnt = 0;
-		double f[E + 1];
-#pragma unroll
-		for (int q = 0; q <= E; ++q) f[q] = 0.0;
-#pragma unroll
-		for (int k = 0; k < NC; ++k) {
-			double pc[E];
-			load_p_rec<M>(P, ch[k], pc);
-			const double tc = P.t[ch[k]];
-			const bool act  = fl[k] & F_ACTIVE;
-			cnt += act;
-#pragma unroll
-			for (int q = 0; q < E; ++q) f[q] = act ? f[q] + pc[q] : f[q];
-			f[E] = act ? f[E] + tc : f[E];
-		}
-		double *memo = P.avg + (size_t) n * AW;
-#pragma unroll
-		for (int q = 0; q <= E; ++q) memo[q] = out[q] = f[q] / (double) cnt;
-		P.cst[n] = epoch;
-		return;
+	if constexpr (DEEP) {
+		if (mean_two_levels<M>(P, n, epoch, out)) return;
+	} else {
+		if (mean_flat<M>(P, n, epoch, out)) return;
 	}
 	struct Frame {
 		int node, next, cnt;
@@ -206,11 +254,14 @@ __device__ void interp_pt(const Pool &P, uint32_t *status, int n, int epoch, dou
 
 // Stamps a changed subtree: `first` (the parent of a changed leaf, or a cell that has just been
 // split) and its ancestors get mod = epoch; a walk stops at the first ancestor already stamped in this
-// epoch (that walk continues to the root).
-__device__ __forceinline__ void mark_up(const Pool &P, int first, int epoch) {
-	for (int a = first, guard = 0; a != 0 && guard < MAX_TREE; a = P.parent[a], ++guard) {
-		if (__ldcg(P.mod + a) == epoch) break;
+// epoch (that walk continues upwards). Only a node at the level of some leaf is ever asked for its mean, so
+// the walk ends at the coarsest level that any leaf has had (`coarsest`): a node above it holds no memo yet.
+__device__ __forceinline__ void mark_up(const Pool &P, int first, int epoch, int coarsest) {
+	for (int a = first, guard = 0; a != 0 && guard < MAX_TREE; ++guard) {
+		const int up = P.parent[a], l = P.level[a];
+		if (l < coarsest || __ldcg(P.mod + a) == epoch) break;
 		P.mod[a] = epoch;
+		a        = up;
 	}
 }
 
@@ -218,16 +269,19 @@ __device__ __forceinline__ void mark_up(const Pool &P, int first, int epoch) {
 // by many cells of the warp (their parent, grandparent, ...) is read and written once per warp instead
 // of once per cell, and the cells of the first wave no longer all store to the same ancestors. The
 // stamped set is mark_up's. Every lane of the warp calls it (first = 0 for a lane with nothing to stamp).
-__device__ __forceinline__ void mark_up_warp(const Pool &P, int first, int epoch) {
+__device__ __forceinline__ void mark_up_warp(const Pool &P, int first, int epoch, int coarsest) {
 	const int lane = threadIdx.x & 31;
 	int a          = first;
 	for (int guard = 0; guard < MAX_TREE; ++guard) {
 		if (!__any_sync(0xffffffffu, a != 0)) break;
 		const unsigned same = __match_any_sync(0xffffffffu, a);
 		int next            = 0;
-		if (a != 0 && __ffs(same) - 1 == lane && __ldcg(P.mod + a) != epoch) {
-			P.mod[a] = epoch;
-			next     = P.parent[a];
+		if (a != 0 && __ffs(same) - 1 == lane) {
+			const int up = P.parent[a], l = P.level[a];
+			if (l >= coarsest && __ldcg(P.mod + a) != epoch) {
+				P.mod[a] = epoch;
+				next     = up;
+			}
 		}
 		a = next;
 	}
