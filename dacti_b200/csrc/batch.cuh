@@ -33,6 +33,8 @@
 #pragma once
 
 #include <algorithm>
+#include <climits>
+#include <deque>
 
 #include "solver.cuh"
 
@@ -380,6 +382,7 @@ class Batch : public BatchBase {
 
 	std::vector<Solver<M> *> s_;
 	cudaStream_t st_  = nullptr;
+	std::vector<cudaStream_t> side_;  // streams of the trees' own runs
 	Counters *d_cnt_  = nullptr;  // all trees' counters
 	Counters *h_cnt_  = nullptr;  // pinned
 	std::vector<Counters *> own_d_, own_h_;
@@ -467,6 +470,7 @@ public:
 
 	~Batch() override {
 		cudaStreamSynchronize(st_);
+		for (auto s: side_) cudaStreamDestroy(s);
 		// counters and streams go back to the solvers
 		for (size_t t = 0; t < s_.size(); ++t) {
 			Solver<M> *s = s_[t];
@@ -856,9 +860,102 @@ private:
 		sync();
 	}
 
+	// ---- a global step as one device-resident run per tree -----------------------------------------
+	//
+	// Each tree's whole global step is one thread-block cluster (run.cuh), the trees side by side on streams of
+	// their own: no merged schedule, and a tree's substeps wait for no other tree's. The GPU holds nine such
+	// clusters, so this is for batches of nine trees on (24 trees of 2 to 11 thousand cells: three steps in 24 ms,
+	// in lockstep 55; 64 of up to 25 thousand: a step in 45 ms, in lockstep 190 to 390), and for fewer trees where
+	// one cluster is the shape of their runs anyway. A cluster above SIDE_CELLS is the host's, stage by stage: of 64
+	// trees with up to 256^2 base cells and 4 levels a first step took 750 ms with this limit at 2^17.
+	static constexpr int SIDE_STREAMS = 32;
+	static constexpr int SIDE_CELLS   = Solver<M>::RUN_CELLS;
+
+	bool side_by_side() const {
+		if (prof_) return false;
+		for (auto *s: s_)
+			if (s->opts_ != DG_OPT_DEFAULT) return false;
+		if ((int) s_.size() >= Solver<M>::RUN_PEERS) return true;
+		for (auto *s: s_)
+			if (s->most_cells(INT_MAX) > Solver<M>::RUN_CLUSTER_CELLS) return false;
+		return true;
+	}
+
+	void step_side_by_side(int signal, int *force_break, double *global_dt) {
+		const int N = (int) s_.size();
+		while ((int) side_.size() < std::min(N, SIDE_STREAMS)) {
+			cudaStream_t x = nullptr;
+			DG_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+			side_.push_back(x);
+		}
+		DG_CUDA(cudaStreamSynchronize(st_));
+		std::vector<int> order(N);
+		for (int t = 0; t < N; ++t) order[t] = t;
+		std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return s_[a]->cell_count() > s_[b]->cell_count(); });
+		std::vector<typename Solver<M>::Step> p(N);
+		std::vector<Base> before(N);
+		// whatever happens, the trees are back on the batch's stream with their work done
+		struct Back {
+			Batch *b;
+			~Back() {
+				for (auto x: b->side_) cudaStreamSynchronize(x);
+				for (auto *s: b->s_) s->st_ = b->st_;
+			}
+		} back{this};
+		std::deque<int> running;
+		auto close = [&](int t) {
+			if (p[t].broke) {
+				force_break[t] = 1;
+				++stops_;
+			} else {
+				s_[t]->finish_step();
+			}
+			runs_ += p[t].runs;
+			stops_ += p[t].stops;
+			completed_ += p[t].by_host;
+		};
+		for (int k = 0; k < N; ++k) {
+			const int t    = order[k];
+			Solver<M> *s   = s_[t];
+			s->st_         = side_[k % side_.size()];
+			before[t]      = {s->n_split_total_, s->n_unsplit_total_, s->updates_, s->n_substeps_};
+			force_break[t] = 0;
+			global_dt[t]   = s->global_dt_;
+			s->begin_step(signal);
+			// a fifth of the tree free as a step starts, else room for half the tree again, so that few runs stop
+			// for a pool without room
+			const long long top = s->h_cnt_->top;
+			if (pregrow_ && top + top / 5 + 16 * NC > s->P_.cap) {
+				const long long want = s->growth_target(s->P_.cap, std::max(top + top / 2 + 16 * NC, s->grown(top)));
+				if (want > s->P_.cap) s->grow_pool((int) std::min<long long>(want, 2000000000LL));
+			}
+			if (s->advance(p[t], SIDE_CELLS, true)) running.push_back(t);
+			else close(t);
+		}
+		while (!running.empty()) {
+			const int t = running.front();
+			running.pop_front();
+			s_[t]->settle(p[t]);
+			if (s_[t]->advance(p[t], SIDE_CELLS, true)) running.push_back(t);
+			else close(t);
+		}
+		for (int t = 0; t < N; ++t) {
+			Solver<M> *s = s_[t];
+			planned_ += s->n_substeps_ - before[t].substeps;
+			base_[t].split += s->n_split_total_ - before[t].split;
+			base_[t].unsplit += s->n_unsplit_total_ - before[t].unsplit;
+			base_[t].updates += s->updates_ - before[t].updates;
+			base_[t].substeps += s->n_substeps_ - before[t].substeps;
+		}
+	}
+
 public:
 	// Integrator::integrate of every tree (impl/integrate.hpp:12-87), merged.
 	void step(int signal, int *force_break, double *global_dt) override {
+		if (side_by_side()) {
+			step_side_by_side(signal, force_break, global_dt);
+			return;
+		}
 		const int N = (int) s_.size();
 		for (int t = 0; t < N; ++t) {
 			Solver<M> *s  = s_[t];
@@ -964,6 +1061,7 @@ public:
 			if (s->resort_) s->resort();
 			global_dt[t] = s->global_dt_;
 		}
+		DG_CUDA(cudaStreamSynchronize(st_));
 	}
 };
 

@@ -51,7 +51,6 @@ enum : uint32_t {
 	ST_CAPACITY     = 1u << 2,  // node pool or list capacity exceeded
 	ST_SPLIT_UNSPLIT = 1u << 3, // a cell was both split-ready and a coarsening candidate
 	ST_MISSING_BC   = 1u << 4,  // face with neither neighbour nor boundary
-	ST_BARRIER      = 1u << 5,  // a grid barrier of a device-resident run gave up waiting
 };
 
 struct ModelConsts {

@@ -50,7 +50,9 @@ struct RunArgs {
 	BcTable B;
 	Lists Ls;
 	Counters *cnt;
-	RunState *state;  // in and out
+	RunState in;
+	RunState *out;      // host memory: the state as the run left it, written last
+	Counters *out_cnt;  // host memory: the counters
 	unsigned *bar;    // grid barrier: arrivals since the launch
 	double global_dt;
 	int limiter, sigma;
@@ -77,7 +79,8 @@ struct DealtGrid {
 	__device__ __forceinline__ int step() const { return blocks * (RUN_THREADS / 32); }
 };
 
-// A wait longer than this many polls (seconds) gives up, marks the status and ends the run.
+// A wait longer than this many polls (seconds) gives up: the launch ends without leaving a state, which the host
+// takes for the error it is.
 constexpr int BARRIER_POLLS = 1 << 23;
 
 // Every thread of the launch arrives and leaves; writes before it are visible after it. False when the
@@ -100,7 +103,6 @@ __device__ __forceinline__ bool run_barrier(const RunArgs &a, unsigned &arrivals
 			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
 		asm volatile("fence.acq_rel.gpu;" ::: "memory");
 		*s_ok = (int) (seen - arrivals) >= 0;
-		if (!*s_ok) set_status(&a.cnt->status, ST_BARRIER);
 	}
 	__syncthreads();
 	return *s_ok;
@@ -164,16 +166,20 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 	const DealtGrid g{(int) blockIdx.x, (int) gridDim.x, false}, r{(int) blockIdx.x, (int) gridDim.x, true};
 
 	if (lead) {
-		s     = a.state->sch;
-		s_seq = a.state->seq;
-		s_l   = a.state->l;
+		s     = a.in.sch;
+		s_seq = a.in.seq;
+		s_l   = a.in.l;
 		s_ls  = a.Ls;
 		s_top = cnt->top;
 		for (int l = 0; l < MAX_ACTI; ++l) s_clu[l] = cnt->clu[l];
 		s_tot[0] = s_tot[1] = s_tot[2] = s_tot[3] = 0;
 		s_stop = -1;
 	}
-	// every block reads the state before block 0 can write it back
+	if (lead && blockIdx.x == 0) {
+		cnt->n_recv = cnt->n_defer = cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_upd = cnt->n_tmp = 0;
+		cnt->status = 0;
+	}
+	// every block has read the counters before any changes them
 	if (!run_barrier(a, arrivals, &s_ok)) return;
 	while (true) {
 		// the next substep, on every block alike (impl/integrate.hpp:25-39)
@@ -315,19 +321,26 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 		}
 		__syncthreads();
 	}
-	if (lead && blockIdx.x == 0) {
-		RunState &o = *a.state;
-		o.sch       = s;
-		o.seq       = s_seq;
-		o.l         = s_l;
-		o.stop      = s_stop;
-		o.L         = s_L;
-		o.splits    = s_tot[0];
-		o.unsplits  = s_tot[1];
-		o.updates   = s_tot[2];
-		o.substeps  = s_tot[3];
-		for (int l = 0; l < MAX_ACTI; ++l) o.clu[l] = s_ls.clu[l];
-		o.tmp = s_ls.tmp;
+	// the host reads both once the launch is over: no copies to queue behind it
+	if (blockIdx.x == 0 && threadIdx.x < 32) {
+		const int *src = reinterpret_cast<const int *>(cnt);
+		int *dst       = reinterpret_cast<int *>(a.out_cnt);
+		for (int w = threadIdx.x; w < (int) (sizeof(Counters) / 4); w += 32) dst[w] = __ldcg(src + w);
+		__syncwarp();
+		if (lead) {
+			RunState &o = *a.out;
+			o.sch       = s;
+			o.seq       = s_seq;
+			o.l         = s_l;
+			o.L         = s_L;
+			o.splits    = s_tot[0];
+			o.unsplits  = s_tot[1];
+			o.updates   = s_tot[2];
+			o.substeps  = s_tot[3];
+			for (int l = 0; l < MAX_ACTI; ++l) o.clu[l] = s_ls.clu[l];
+			o.tmp  = s_ls.tmp;
+			o.stop = s_stop;
+		}
 	}
 }
 

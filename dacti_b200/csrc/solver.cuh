@@ -84,8 +84,8 @@ class Solver : public SolverBase {
 	Lists Ls_{};
 	Counters *d_cnt_ = nullptr;
 	Counters *h_cnt_ = nullptr;  // pinned, behind h_run_ unless a batch holds the counters
-	RunState *d_run_ = nullptr;  // schedule state of device-resident runs, then the grid barrier's counter
-	RunState *h_run_ = nullptr;  // pinned
+	unsigned *d_bar_ = nullptr;  // the grid barrier of device-resident runs
+	RunState *h_run_ = nullptr;  // pinned: where a run leaves its schedule state
 	int run_cluster_ = 0;        // blocks of a clustered run on this device (0: not asked yet)
 	void *pool_mem_  = nullptr;
 	void *spare_mem_  = nullptr;  // one field's worth of slots: target of the re-sort and gc permutations
@@ -196,9 +196,9 @@ public:
 		DG_CUDA(mem_alloc((void **) &d_cnt_, sizeof(Counters), st_));
 		static_assert(sizeof(RunState) + 16 + sizeof(Counters) <= PINNED_BYTES, "run state and counters share a pinned block");
 		DG_CUDA(pinned_alloc((void **) &h_run_));
-		h_cnt_ = (Counters *) ((char *) h_run_ + (sizeof(RunState) + sizeof(unsigned) + 7) / 8 * 8);
+		h_cnt_ = (Counters *) (h_run_ + 1);
 		DG_CUDA(cudaMemset(d_cnt_, 0, sizeof(Counters)));
-		DG_CUDA(mem_alloc((void **) &d_run_, sizeof(RunState) + sizeof(unsigned), st_));
+		DG_CUDA(mem_alloc((void **) &d_bar_, sizeof(unsigned), st_));
 		upload_tree(c);
 		construct();
 	}
@@ -215,7 +215,7 @@ public:
 		mem_free_idle(sel_mem_);
 		mem_free_idle(pos_mem_);
 		mem_free_idle(d_cnt_);
-		mem_free_idle(d_run_);
+		mem_free_idle(d_bar_);
 		pinned_release(h_run_);
 		mem_free_idle(d_leaves_);
 		mem_free_idle(d_read_);
@@ -740,7 +740,6 @@ private:
 
 	void check_status() {
 		uint32_t s = h_cnt_->status & ~ST_NAN;
-		if (s & ST_BARRIER) throw dg_error(DG_ERR_CUDA, "a grid barrier of a device-resident run gave up waiting");
 		if (s & ST_CAPACITY) throw dg_error(DG_ERR_CAPACITY, "device list or pool capacity exceeded");
 		if (s & ST_DEPTH) throw dg_error(DG_ERR_DEPTH, "tree level jump deeper than supported");
 		if (s & ST_MISSING_BC) throw dg_error(DG_ERR_MISSING_BC, "face without neighbour or boundary condition");
@@ -953,30 +952,41 @@ private:
 		n_launches_++;
 	}
 
-	// Runs substeps from (seq, l) on the device until the global step is done or the host is needed;
-	// `most` is the largest cluster as the run starts. The host's schedule state, lists and counters are
-	// current afterwards. Returns why the run ended (RunStop); `L` is the level of an unfinished substep.
-	int run(int &seq, int &l, int &L, long long most, int peers) {
-		ensure_scratch(std::min<long long>(std::max<long long>(most + most / 2, 4096), RUN_CELLS));
-		RunState &h    = *h_run_;
-		h.sch.max_acti = max_acti_;
-		h.sch.stamp    = stamp_;
-		h.sch.epoch    = epoch_;
-		h.sch.pad      = 0;
-		std::copy(acti_counter_, acti_counter_ + MAX_ACTI, h.sch.counter);
-		std::copy(acti_time_, acti_time_ + MAX_ACTI, h.sch.time);
-		h.seq = seq;
-		h.l   = l;
-		*(unsigned *) (h_run_ + 1) = 0;
-		DG_CUDA(cudaMemcpyAsync(d_run_, h_run_, sizeof(RunState) + sizeof(unsigned), cudaMemcpyHostToDevice, st_));
-		DG_CUDA(cudaMemsetAsync(&d_cnt_->n_recv, 0, (char *) (&d_cnt_->status + 1) - (char *) &d_cnt_->n_recv, st_));
-		const bool clustered = peers >= RUN_PEERS || most <= RUN_CLUSTER_CELLS;
-		// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU
-		static std::mutex whole_gpu;
-		std::unique_lock<std::mutex> hold(whole_gpu, std::defer_lock);
-		if (!clustered) hold.lock();
-		RunArgs a{P_, C_, B_, Ls_, d_cnt_, d_run_, (unsigned *) (d_run_ + 1), global_dt_, limiter_, sigma_ ? 1 : 0,
-		          (int) std::min<long long>(scratch_cap_, RUN_CELLS), clustered ? 1 : 0};
+	// The largest cluster of up to `limit` cells.
+	long long most_cells(int limit) const {
+		long long most = 0;
+		for (int l = 0; l < MAX_ACTI; ++l)
+			if (h_cnt_->clu[l] <= limit) most = std::max<long long>(most, h_cnt_->clu[l]);
+		return most;
+	}
+
+	// Starts a run of the substeps from (seq, l) on, which lasts until the global step is done or the host is
+	// needed; clusters above `limit` cells are left to the host.
+	void run_begin(int seq, int l, int limit, bool clustered) {
+		static_assert(sizeof(RunArgs) <= 4096 && sizeof(Counters) % 4 == 0, "a run's arguments are kernel parameters");
+		const long long most = most_cells(limit);
+		ensure_scratch(std::min<long long>(std::max<long long>(most + most / 2, 4096), limit));
+		RunArgs a{};
+		a.P            = P_;
+		a.C            = C_;
+		a.B            = B_;
+		a.Ls           = Ls_;
+		a.cnt          = d_cnt_;
+		a.in.sch       = {max_acti_, stamp_, epoch_, 0, {}, {}};
+		a.in.seq       = seq;
+		a.in.l         = l;
+		std::copy(acti_counter_, acti_counter_ + MAX_ACTI, a.in.sch.counter);
+		std::copy(acti_time_, acti_time_ + MAX_ACTI, a.in.sch.time);
+		a.out       = h_run_;
+		a.out_cnt   = h_cnt_;
+		a.bar       = d_bar_;
+		a.global_dt = global_dt_;
+		a.limiter   = limiter_;
+		a.sigma     = sigma_ ? 1 : 0;
+		a.rows      = (int) std::min<long long>(scratch_cap_, limit);
+		a.clustered = clustered ? 1 : 0;
+		h_run_->stop = -1;
+		if (!clustered) DG_CUDA(cudaMemsetAsync(d_bar_, 0, sizeof(unsigned), st_));
 		if constexpr (!M::VISC) {
 			if (mixed_) launch_run<false, float>(a, clustered);
 			else launch_run<false, double>(a, clustered);
@@ -989,9 +999,14 @@ private:
 			else if (mixed_) launch_run<false, float>(a, clustered);
 			else launch_run<false, double>(a, clustered);
 		}
-		DG_CUDA(cudaMemcpyAsync(h_run_, d_run_, sizeof(RunState), cudaMemcpyDeviceToHost, st_));
-		sync_counters();
-		if (h_cnt_->status & ST_BARRIER) check_status();  // the run's state is not complete
+	}
+
+	// Waits for the run. The host's schedule state, lists and counters are current afterwards. Returns why the
+	// run ended (RunStop); `L` is the level of an unfinished substep.
+	int run_end(int &seq, int &l, int &L) {
+		DG_CUDA(cudaStreamSynchronize(st_));
+		const RunState &h = *h_run_;
+		if (h.stop < 0) throw dg_error(DG_ERR_CUDA, "a grid barrier of a device-resident run gave up waiting");
 		max_acti_ = h.sch.max_acti;
 		stamp_    = h.sch.stamp;
 		epoch_    = h.sch.epoch;
@@ -1009,61 +1024,104 @@ private:
 		return h.stop;
 	}
 
-public:
-	// Integrator::integrate (impl/integrate.hpp:12-87)
-	void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user, int peers = 1) override {
-		C_.signal   = signal;
-		C_.coarsen  = (n_global_ % coarsen_every_) == 0;
-		*force_break = 0;
-		// Runs on the device serve the default stage choices; the host issues a substep's stages one by one
-		// where a callback or the timing of every stage asks for it, and for clusters that fill the GPU.
-		const bool resident = !fn && !prof_ && opts_ == DG_OPT_DEFAULT;
+	// A global step of this solver in the making: runs on the device, and what a run leaves to the host.
+	struct Step {
 		int seq = 0, l = MAX_ACTI;
-		while (true) {
-			int s = seq, k = l;
+		bool broke = false, done = false;
+		long long runs = 0, stops = 0, by_host = 0;
+	};
+	void begin_step(int signal) {
+		C_.signal  = signal;
+		C_.coarsen = (n_global_ % coarsen_every_) == 0;
+	}
+	// Up to the next run: substeps of clusters above `limit` are the host's. False when the step is over.
+	bool advance(Step &p, int limit, bool clustered) {
+		while (!p.broke && !p.done) {
+			int s = p.seq, k = p.l;
 			const int next = next_substep(s, k);
-			if (next < 0) break;
-			bool broke = false;
-			if (resident && h_cnt_->clu[next] <= RUN_CELLS) {
-				long long most = 0;
-				for (int c = 0; c < MAX_ACTI; ++c)
-					if (h_cnt_->clu[c] <= RUN_CELLS) most = std::max<long long>(most, h_cnt_->clu[c]);
-				int L          = 0;
-				const int stop = run(seq, l, L, most, peers);
-				if (stop == RUN_DONE) break;
-				if (stop == RUN_LARGE) continue;
-				if (stop == RUN_STATUS) {
-					check_status();
-					broke = h_cnt_->status & ST_NAN;
-				} else {
-					// the run closed before the regrid of substep L
-					check_status();
-					const int n = h_cnt_->clu[L];
-					epoch_ += EPOCH_EST<M>;
-					grow_for_splits();
-					substep_tail(L, n);
-					broke = substep_end(L);
-				}
+			if (next < 0) {
+				p.done = true;
+			} else if (h_cnt_->clu[next] <= limit) {
+				run_begin(p.seq, p.l, limit, clustered);
+				++p.runs;
+				return true;
 			} else {
-				seq         = s;
-				l           = k;
-				const int n = h_cnt_->clu[next];
-				substep_head(next);
-				substep_tail(next, n);
-				broke = substep_end(next);
-				if (!broke && fn)
-					fn(user, next, acti_time_[next], (int) n_substeps_, global_dt_ / (double) (1 << next), h_cnt_->clu[next]);
-			}
-			if (broke) {
-				*force_break = 1;
-				*global_dt   = global_dt_;
-				return;
+				p.seq = s;
+				p.l   = k;
+				host_substep(next);
+				p.broke = substep_end(next);
+				++p.by_host;
 			}
 		}
+		return false;
+	}
+	// The end of a run, and of the substep that it left to the host.
+	void settle(Step &p) {
+		int L          = 0;
+		const int stop = run_end(p.seq, p.l, L);
+		p.done         = stop == RUN_DONE;
+		if (stop == RUN_STATUS) {
+			check_status();
+			p.broke = h_cnt_->status & ST_NAN;
+		} else if (stop == RUN_CAPACITY) {
+			// the run closed before the regrid of substep L
+			check_status();
+			const int n = h_cnt_->clu[L];
+			epoch_ += EPOCH_EST<M>;
+			grow_for_splits();
+			substep_tail(L, n);
+			p.broke = substep_end(L);
+			++p.stops;
+			++p.by_host;
+		} else if (stop == RUN_LARGE) {
+			++p.stops;
+		}
+	}
+	void host_substep(int L) {
+		const int n = h_cnt_->clu[L];
+		substep_head(L);
+		substep_tail(L, n);
+	}
+	// Garbage collection and the re-sort after a complete global step; the stream may still be at work.
+	void finish_step() {
 		n_global_++;
 		if (gc_due()) gc();
 		if (resort_) resort();
-		*global_dt = global_dt_;
+	}
+
+public:
+	// Integrator::integrate (impl/integrate.hpp:12-87)
+	void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user, int peers = 1) override {
+		begin_step(signal);
+		*force_break = 0;
+		*global_dt   = global_dt_;
+		Step p;
+		// Runs on the device serve the default stage choices; the host issues a substep's stages one by one
+		// where a callback or the timing of every stage asks for it, and for clusters that fill the GPU.
+		if (!fn && !prof_ && opts_ == DG_OPT_DEFAULT) {
+			// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU
+			static std::mutex whole_gpu;
+			while (!p.done && !p.broke) {
+				const bool clustered = peers >= RUN_PEERS || most_cells(RUN_CELLS) <= RUN_CLUSTER_CELLS;
+				std::unique_lock<std::mutex> hold(whole_gpu, std::defer_lock);
+				if (!clustered) hold.lock();
+				if (advance(p, RUN_CELLS, clustered)) settle(p);
+			}
+		} else {
+			for (int L; !p.broke && (L = next_substep(p.seq, p.l)) >= 0;) {
+				host_substep(L);
+				p.broke = substep_end(L);
+				if (!p.broke && fn)
+					fn(user, L, acti_time_[L], (int) n_substeps_, global_dt_ / (double) (1 << L), h_cnt_->clu[L]);
+			}
+		}
+		if (p.broke) {
+			*force_break = 1;
+			return;
+		}
+		finish_step();
+		DG_CUDA(cudaStreamSynchronize(st_));
+		drain_events();
 	}
 
 	void set_resort(bool on) { resort_ = on; }
@@ -1162,7 +1220,6 @@ public:
 		}
 		run_k(DG_K_OTHER, 0, [&] { k_fill_ranges<<<dim3(grid_for(most), MAX_ACTI), BLOCK, 0, st_>>>(r); });
 		DG_CUDA(cudaGetLastError());
-		sync_counters();
 	}
 
 private:
