@@ -183,7 +183,7 @@ static __global__ void __launch_bounds__(256) kb_begin(TreeArgs *A, int n_trees,
 				s.stamp    = ++z.stamp;
 				s.epoch0   = z.epoch;
 				z.epoch += a.epochs;
-				c->n_recv = c->n_defer = c->n_split = c->n_unsplit = c->n_new = c->n_upd = c->n_tmp = 0;
+				c->n_recv = c->n_defer = c->n_split = c->n_unsplit = c->n_new = c->n_tmp = 0;
 				c->status                                                        = 0;
 			}
 		}
@@ -272,8 +272,7 @@ __global__ void kb_regrid(DG_BATCH_PARAMS, int k) {
 		case 0: d_unsplit_select<M>(g, a.P, a.Ls.clu[L], s.n, L, a.Ls.unsplit, a.cnt); break;
 		case 1: d_split<M>(g, a.P, cst, &a.cnt->n_split, a.Ls.split, L, a.Ls.fresh, s.epoch0 + EX + 1, a.cnt); break;
 		case 2: d_unsplit<M>(g, a.P, cst, &a.cnt->n_unsplit, a.Ls.unsplit, L, a.Ls.fresh, s.epoch0 + EX + 2, a.cnt); break;
-		case 3: d_nbr_fresh<M>(g, a.P, cst, &a.cnt->n_new, a.Ls.fresh, a.Ls.upd, a.cnt); break;
-		case 4: d_nbr_list<M>(g, a.P, cst, &a.cnt->n_upd, a.Ls.upd, a.cnt); break;
+		case 3: d_nbr_fresh<M>(g, a.P, cst, &a.cnt->n_new, a.Ls.fresh, a.cnt); break;
 		case 5: d_reassign<M>(g, a.P, cst, a.Ls.clu[L], nullptr, s.n, L, s.dtL, s.counterL, a.Ls, a.cnt); break;
 		default: d_reassign<M>(g, a.P, cst, a.Ls.fresh, &a.cnt->n_new, 0, L, s.dtL, s.counterL, a.Ls, a.cnt); break;
 	}
@@ -815,8 +814,7 @@ private:
 			regrid(T_RG_CELL, 0);   // unsplit selection
 			regrid(T_RG_FRESH, 1);  // split
 			regrid(T_RG_CELL, 2);   // unsplit
-			regrid(T_RG_FRESH, 3);  // neighbour repair, first pass
-			regrid(T_NBR, 4);       // neighbour repair, second pass
+			regrid(T_NBR, 3);       // neighbour repair
 			regrid(T_RG_CELL, 5);   // reassignment of the cluster
 			regrid(T_RG_FRESH, 6);  // reassignment of new cells
 			kb_swap<<<(nt + 127) / 128, 128, 0, st_>>>(d_trees_, S, nt, ont);

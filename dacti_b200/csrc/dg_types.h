@@ -114,7 +114,6 @@ struct Pool {
 	double *flux;     // [F][cap]
 	double *err, *maxdt, *cfl;
 	int32_t *stamp;   // per-node dedup stamp for list building
-	uint32_t *fmask;  // faces (bit 2 dim + dir) whose neighbour changed in the running regrid; 0 otherwise
 	uint8_t *op;      // refinement op code
 	double *tmp, *tmp2;  // per-node scratch scalars (Jacobi smoothing sweeps, alternately)
 	// Per-substep scratch outside the permuted fields:
@@ -134,9 +133,9 @@ struct Counters {
 	int n_split;
 	int n_unsplit;
 	int n_new;        // new cluster members (children + coarsened parents)
-	int n_upd;        // neighbour-update list
 	int n_tmp;        // rebuilt cluster list
 	uint32_t status;
+	int blocks_done;  // blocks of the running launch that have finished (0 between launches)
 	int coarsest;     // the lowest tree level any active leaf has had
 	// running totals that the batched step keeps on the device (splits, coarsenings, cluster cells after
 	// each substep's flush, substeps)
@@ -151,9 +150,8 @@ struct Lists {
 	int32_t *tmp;      // rebuilt cluster list
 	int32_t *recv;     // receivers of cross-level fluxes
 	int32_t *split;    // split-ready cells
-	int32_t *unsplit;  // parents to coarsen
+	int32_t *unsplit;  // parents to coarsen (batched step)
 	int32_t *fresh;    // new children and coarsened parents
-	int32_t *upd;      // neighbour-update list
 };
 
 }  // namespace dg

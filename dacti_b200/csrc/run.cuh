@@ -5,7 +5,7 @@
 // What bounds a substep of a small cluster is not its cells but its chain of launches: a substep is about
 // twenty stage kernels and one host synchronisation, 100 to 200 us on this GPU whatever the cluster's
 // size, while the stages' own work on a few thousand cells is a microsecond or two each. Here a barrier
-// takes the place of a launch, stages that do not read one another's results share one (seven to nine
+// takes the place of a launch, stages that do not read one another's results share one (six to nine
 // barriers a substep), and the host is not asked until the global step ends or something needs it.
 #pragma once
 
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 		s_stop = -1;
 	}
 	if (lead && blockIdx.x == 0) {
-		cnt->n_recv = cnt->n_defer = cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_upd = cnt->n_tmp = 0;
+		cnt->n_recv = cnt->n_defer = cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_tmp = 0;
 		cnt->status = 0;
 	}
 	// every block has read the counters before any changes them
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 		if (__ldcg(&cnt->n_recv) > 0) d_flux_receive<M, S>(r, P, s_ls.recv, &cnt->n_recv, L, cnt);
 		if (deferred && !run_barrier(a, arrivals, &s_ok)) return;
 		d_update<M, V>(g, P, C, list, n, dtL, e_upd, cnt);
-		if (lead && blockIdx.x == 0) cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_upd = cnt->n_tmp = 0;
+		if (lead && blockIdx.x == 0) cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_tmp = 0;
 		if (!run_barrier(a, arrivals, &s_ok)) return;
 		if (lead && blockIdx.x == 0) cnt->n_recv = cnt->n_defer = 0;
 		d_slope<M, V>(g, P, C, a.B, list, n, a.limiter, epoch0 + 2, cnt);
@@ -283,15 +283,11 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 		}
 		// the neighbour repair reads no time level and the reassignment no neighbour
 		const int n_new = __ldcg(&cnt->n_new);
-		d_nbr_fresh<M>(r, P, C, &cnt->n_new, s_ls.fresh, s_ls.upd, cnt);
+		if (n_new > 0) d_nbr_fresh<M>(r, P, C, &cnt->n_new, s_ls.fresh, cnt);
 		run_reassign<M>(g, P, C, list, n, L, dtL, counter_L, s_ls, cnt, s_warp);
 		d_reassign<M>(g, P, C, s_ls.fresh, &cnt->n_new, 0, L, dtL, counter_L, s_ls, cnt);
 		d_flush(r, P, s_ls.buf[L], &cnt->buf[L], s_ls.tmp, &cnt->n_tmp, L, cnt);
 		if (!run_barrier(a, arrivals, &s_ok)) return;
-		if (n_new > 0) {
-			d_nbr_list<M>(g, P, C, &cnt->n_upd, s_ls.upd, cnt);
-			if (!run_barrier(a, arrivals, &s_ok)) return;
-		}
 		// the substep's end (impl/integrate.hpp:56-67)
 		if (lead) {
 			int v[MAX_ACTI];

@@ -349,7 +349,7 @@ public:
 		    {(void **) &P.k, 8, M::P}, {(void **) &P.tslope, 8, visc_ ? M::G : -1},
 		    {(void **) &P.grad, 8, visc_ ? D * M::G : -1},
 		    {(void **) &P.flux, 8, M::F}, {(void **) &P.err, 8, 1}, {(void **) &P.maxdt, 8, 1},
-		    {(void **) &P.cfl, 8, 1}, {(void **) &P.stamp, 4, 1, 0, 1}, {(void **) &P.fmask, 4, 1, 0, 1}, {(void **) &P.op, 1, 1},
+		    {(void **) &P.cfl, 8, 1}, {(void **) &P.stamp, 4, 1, 0, 1}, {(void **) &P.op, 1, 1},
 		    {(void **) &P.tmp, 8, 1, 0, 1}, {(void **) &P.tmp2, 8, 1, 0, 1},
 		};
 	}
@@ -458,7 +458,7 @@ public:
 		size_t free_b = 0, total_b = 0;
 		DG_CUDA(cudaMemGetInfo(&free_b, &total_b));
 		const size_t released = sizeof(double) * M::F * (NF + 1) * (size_t) scratch_cap_ + spare_bytes_ + sort_bytes_;
-		size_t per_slot = sizeof(int32_t) * (2 * MAX_ACTI + 6);
+		size_t per_slot = sizeof(int32_t) * (2 * MAX_ACTI + 5);
 		for (auto &f: fields(P_))
 			if (f.comps >= 0) per_slot += f.elem * (size_t) (f.comps > 0 ? f.comps : 1);
 		const long long avail = (long long) (free_b + mem_unused() + released) - (1LL << 30);
@@ -533,7 +533,7 @@ public:
 
 	int list_cap_ = 0;
 	void alloc_lists(int cap) {
-		const int nlists = 2 * MAX_ACTI + 6;
+		const int nlists = 2 * MAX_ACTI + 5;
 		size_t one       = align_up(sizeof(int32_t) * (size_t) cap);
 		DG_CUDA(mem_alloc((void **) &list_mem_, one * nlists, st_));
 		char *b = (char *) list_mem_;
@@ -552,8 +552,6 @@ public:
 		Ls_.unsplit = (int32_t *) b;
 		b += one;
 		Ls_.fresh   = (int32_t *) b;
-		b += one;
-		Ls_.upd     = (int32_t *) b;
 		list_cap_   = cap;
 	}
 
@@ -808,26 +806,15 @@ private:
 		const double dtL   = global_dt_ / (double) (1 << L);
 		int32_t *list      = Ls_.clu[L];
 		const int counterL = acti_counter_[L];
-		const int g        = grid_for(n);
 		const int gf       = grid_for((long long) n * (NC + 1));
 		ensure_scratch(n);  // a growth of the pool releases the list scratch; the reassignment uses its marks
-		run_k(DG_K_REGRID, n, [&] { k_unsplit_select<M><<<g, BLOCK, 0, st_>>>(P_, list, n, L, Ls_.unsplit, d_cnt_); });
-		run_k(DG_K_REGRID, 0, [&] {
-			k_split<M><<<gf, BLOCK, 0, st_>>>(P_, C_, &d_cnt_->n_split, Ls_.split, L, Ls_.fresh, ++epoch_, d_cnt_);
-		});
-		run_k(DG_K_REGRID, 0, [&] {
-			k_unsplit<M><<<g, BLOCK, 0, st_>>>(P_, C_, &d_cnt_->n_unsplit, Ls_.unsplit, L, Ls_.fresh, ++epoch_, d_cnt_);
-		});
-		run_k(DG_K_REGRID, 0, [&] {
-			k_nbr_fresh<M><<<gf, BLOCK, 0, st_>>>(P_, C_, &d_cnt_->n_new, Ls_.fresh, Ls_.upd, d_cnt_);
-		});
-		run_k(DG_K_REGRID, 0, [&] {
-			k_nbr_list<M><<<grid_for((long long) n * (NC + 1) * NF), BLOCK, 0, st_>>>(P_, C_, &d_cnt_->n_upd, Ls_.upd, d_cnt_);
+		epoch_ += 2;
+		run_k(DG_K_REGRID, n, [&] {
+			k_regrid<M><<<gf, BLOCK, 0, st_>>>(P_, C_, Ls_.split, list, n, L, counterL, Ls_.fresh, epoch_ - 1, d_cnt_);
 		});
 		const bool ordered = opts_ & DG_OPT_ORDERED_LISTS;
 		run_k(DG_K_REASSIGN, n, [&] {
-			k_reassign<M><<<g, BLOCK, 0, st_>>>(P_, C_, list, nullptr, n, L, dtL, counterL, Ls_, d_cnt_,
-			                                    ordered ? stay_marks() : nullptr);
+			k_repair<M><<<gf, BLOCK, 0, st_>>>(P_, C_, Ls_.fresh, list, n, L, dtL, counterL, Ls_, d_cnt_, ordered ? stay_marks() : nullptr);
 			// the cells that stay at level L, in their list order (the count goes to n_tmp, which the
 			// reassignment of the new cells then appends to)
 			if (ordered) {
@@ -836,12 +823,8 @@ private:
 				                                   Ls_.tmp, &d_cnt_->n_tmp, n, st_));
 			}
 		});
-		run_k(DG_K_REASSIGN, 0, [&] {
-			k_reassign<M><<<gf, BLOCK, 0, st_>>>(P_, C_, Ls_.fresh, &d_cnt_->n_new, 0, L, dtL, counterL, Ls_, d_cnt_,
-			                                     nullptr);
-		});
+		run_k(DG_K_REASSIGN, 0, [&] { k_reassign_fresh<M><<<grid_for(n), BLOCK, 0, st_>>>(P_, C_, L, dtL, counterL, Ls_, d_cnt_); });
 		std::swap(Ls_.clu[L], Ls_.tmp);
-		run_k(DG_K_OTHER, 0, [&] { k_set_count<<<1, 1, 0, st_>>>(&d_cnt_->clu[L], &d_cnt_->n_tmp); });
 		DG_CUDA(cudaGetLastError());
 	}
 

@@ -1139,11 +1139,6 @@ __device__ __forceinline__ void d_unsplit_select(const Grid &g, const Pool &P, c
 		if (unsplit_selected<M>(P, list[tid], L, par, cnt)) append(unsplit_list, &cnt->n_unsplit, par, P.cap, &cnt->status);
 	}
 }
-template<class M>
-__global__ void k_unsplit_select(Pool P, const int32_t *list, int n, int L, int32_t *unsplit_list, Counters *cnt) {
-	d_unsplit_select<M>(PlainGrid{}, P, list, n, L, unsplit_list, cnt);
-}
-
 // Domain::split (integrator/domain.hpp:192-247) plus the child set-up of
 // impl/adaptive_refinement.hpp:167-195. Children take the parent's primitive state extrapolated
 // with its slope, reuse the parent's old child slots when it has any, start with a zero Hancock
@@ -1242,12 +1237,6 @@ __device__ __forceinline__ void d_split(const Grid &g, const Pool &P, const Cons
 		}
 	}
 }
-template<class M>
-__global__ void k_split(Pool P, Consts C, const int *n_ptr, const int32_t *split_list, int L, int32_t *fresh,
-                        int epoch, Counters *cnt) {
-	d_split<M>(PlainGrid{}, P, C, n_ptr, split_list, L, fresh, epoch, cnt);
-}
-
 // Domain::unsplit with interpolated_cell (integrator/domain.hpp:150-180, 296-325): the parent takes
 // the children's mean t, u, k, t_slope and gradient (the gradient sum starts from the parent's own
 // stale gradient, as interpolated_cell does not reset it) and keeps its old slope and rhs.
@@ -1329,10 +1318,12 @@ __device__ __forceinline__ void d_coarsen(const Grid &g, const Pool &P, const Co
 		}
 	}
 }
+// The regrid of a substep in one launch: a split cell and the family of a coarsened one have no cell in common.
 template<class M>
-__global__ void k_unsplit(Pool P, Consts C, const int *n_ptr, const int32_t *unsplit_list, int L, int32_t *fresh,
-                          int epoch, Counters *cnt) {
-	d_unsplit<M>(PlainGrid{}, P, C, n_ptr, unsplit_list, L, fresh, epoch, cnt);
+__global__ void k_regrid(Pool P, Consts C, const int32_t *split_list, const int32_t *list, int n, int L, int counter_L,
+                         int32_t *fresh, int epoch, Counters *cnt) {
+	d_split<M>(PlainGrid{}, P, C, &cnt->n_split, split_list, L, fresh, epoch, cnt);
+	if (counter_L == 1 && C.coarsen) d_coarsen<M>(PlainGrid{}, P, C, list, n, L, fresh, epoch + 1, cnt);
 }
 
 // Domain::update_neighbors for one active leaf (integrator/domain.hpp:249-293): faces without a
@@ -1411,70 +1402,39 @@ __device__ void update_neighbors_subtree(const Pool &P, const Consts &C, uint32_
 	}
 }
 
-// Neighbour repair, first pass (impl/adaptive_refinement.hpp:236-249): new children and coarsened
-// parents, then queue their neighbours for the second pass.
-// Each neighbour is queued once with the mask of its faces towards new cells. A group of lanes serves one
-// new cell (4 in 2D, 8 in 3D with 6 busy), lane f repairing face f and queueing the neighbour across it,
-// so the tree walks of a cell's faces run side by side instead of one after another in one thread. New
-// cells are leaves; a non-leaf (which the stages do not produce) is repaired whole by its group's first
-// lane, as Domain::update_neighbors repairs a subtree.
+// Neighbour repair (impl/adaptive_refinement.hpp:236-249): the faces of new children and coarsened parents, and
+// of the cells behind them the faces towards the new cell. A group of lanes serves one new cell (4 in 2D, 8 in 3D
+// with 6 busy), lane f repairing face f and then what lies behind it, so the tree walks of a cell's faces run side
+// by side. A walk reads the tree only, which no lane changes here, so lanes that meet at one neighbour (the
+// children behind a coarser cell) write the same link, and no list of neighbours with a second pass over it is
+// needed. New cells are leaves; a non-leaf (which the stages do not produce) is repaired whole by its group's
+// first lane, as Domain::update_neighbors repairs a subtree.
 template<class M, class Grid>
-__device__ __forceinline__ void d_nbr_fresh(const Grid &g, const Pool &P, const Consts &C, const int *n_ptr, const int32_t *fresh, int32_t *upd, Counters *cnt) {
+__device__ __forceinline__ void d_nbr_fresh(const Grid &g, const Pool &P, const Consts &C, const int *n_ptr, const int32_t *fresh, Counters *cnt) {
 	constexpr int NF = 2 * M::D, G = NF <= 4 ? 4 : 8, GW = 32 / G;
 	const int n      = *n_ptr;
 	const int cap    = P.cap;
 	const int lane   = threadIdx.x & 31;
 	const int sub    = lane & (G - 1);
 	const int items  = warp_items(n, GW);
-	auto queue = [&](int i, int f) {
+	auto behind = [&](int i, int f) {
 		const int nb = P.nbr[(size_t) f * cap + i];
-		if (nb != 0 && ((P.flags[nb] & F_ACTIVE) || !(P.flags[nb] & F_LEAF))) {
-			if (atomicOr(&P.fmask[nb], 1u << (f ^ 1)) == 0) append(upd, &cnt->n_upd, nb, cap, &cnt->status);
-		}
+		if (nb != 0 && ((P.flags[nb] & F_ACTIVE) || !(P.flags[nb] & F_LEAF)))
+			update_face_subtree<M>(P, C, &cnt->status, nb, f >> 1, 1 - (f & 1));
 	};
 	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
-		const int wbase = it * GW;
-		const int slot = wbase + lane / G;
+		const int slot = it * GW + lane / G;
 		if (slot >= n || sub >= NF) continue;
 		const int i       = fresh[slot];
 		const uint32_t fl = P.flags[i];
 		if (fl & F_LEAF) {
 			if (fl & F_ACTIVE) update_neighbor_face<M>(P, C, i, sub >> 1, sub & 1);
-			queue(i, sub);
+			behind(i, sub);
 		} else if (sub == 0) {
 			update_neighbors_subtree<M>(P, C, &cnt->status, i);
-			for (int f = 0; f < NF; ++f) queue(i, f);
+			for (int f = 0; f < NF; ++f) behind(i, f);
 		}
 	}
-}
-template<class M>
-__global__ void k_nbr_fresh(Pool P, Consts C, const int *n_ptr, const int32_t *fresh, int32_t *upd, Counters *cnt) {
-	d_nbr_fresh<M>(PlainGrid{}, P, C, n_ptr, fresh, upd, cnt);
-}
-
-// Neighbour repair, second pass: the queued neighbours' faces towards new cells, one lane per face (the
-// lane groups of the first pass). The group reads the face mask before its first lane clears it.
-template<class M, class Grid>
-__device__ __forceinline__ void d_nbr_list(const Grid &g, const Pool &P, const Consts &C, const int *n_ptr, const int32_t *list, Counters *cnt) {
-	constexpr int NF = 2 * M::D, G = NF <= 4 ? 4 : 8, GW = 32 / G;
-	const int n      = *n_ptr;
-	const int lane   = threadIdx.x & 31;
-	const int sub    = lane & (G - 1);
-	const int items  = warp_items(n, GW);
-	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
-		const int wbase = it * GW;
-		const int slot = wbase + lane / G;
-		const bool act = slot < n && sub < NF;
-		const int x      = act ? list[slot] : 0;
-		const uint32_t m = act ? P.fmask[x] : 0u;
-		__syncwarp();
-		if (act && (m & (1u << sub))) update_face_subtree<M>(P, C, &cnt->status, x, sub >> 1, sub & 1);
-		if (act && sub == 0) P.fmask[x] = 0;
-	}
-}
-template<class M>
-__global__ void k_nbr_list(Pool P, Consts C, const int *n_ptr, const int32_t *list, Counters *cnt) {
-	d_nbr_list<M>(PlainGrid{}, P, C, n_ptr, list, cnt);
 }
 
 // ACTI reassignment (impl/adaptive_refinement.hpp:264-322): per-cell CFL decides whether a cell
@@ -1532,10 +1492,28 @@ __device__ __forceinline__ void d_reassign(const Grid &g, const Pool &P, const C
 		else if (stays) append(Ls.tmp, &cnt->n_tmp, i, P.cap, &cnt->status);
 	}
 }
+// After the regrid, in one launch: the neighbour repair reads no time level and the reassignment of the old list
+// no neighbour.
 template<class M>
-__global__ void k_reassign(Pool P, Consts C, const int32_t *list, const int *n_ptr, int n_host, int L, double dtL,
-                           int counter_L, Lists Ls, Counters *cnt, uint8_t *stay) {
-	d_reassign<M>(PlainGrid{}, P, C, list, n_ptr, n_host, L, dtL, counter_L, Ls, cnt, stay);
+__global__ void k_repair(Pool P, Consts C, const int32_t *fresh, const int32_t *list, int n, int L, double dtL, int counter_L, Lists Ls,
+                         Counters *cnt, uint8_t *stay) {
+	d_reassign<M>(PlainGrid{}, P, C, list, nullptr, n, L, dtL, counter_L, Ls, cnt, stay);
+	d_nbr_fresh<M>(PlainGrid{}, P, C, &cnt->n_new, fresh, cnt);
+}
+// The new cells' reassignment, the last stage that adds to the rebuilt list; the last block to finish sets the
+// cluster's length.
+template<class M>
+__global__ void k_reassign_fresh(Pool P, Consts C, int L, double dtL, int counter_L, Lists Ls, Counters *cnt) {
+	d_reassign<M>(PlainGrid{}, P, C, Ls.fresh, &cnt->n_new, 0, L, dtL, counter_L, Ls, cnt);
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		__threadfence();
+		if (atomicAdd(&cnt->blocks_done, 1) == (int) gridDim.x - 1) {
+			__threadfence();
+			cnt->clu[L]      = __ldcg(&cnt->n_tmp);
+			cnt->blocks_done = 0;
+		}
+	}
 }
 
 // flush_acti_buffer (impl/acti_utils.hpp:365-372)
@@ -1556,8 +1534,6 @@ static __global__ void k_flush(Pool P, const int32_t *buf, const int *n_ptr, int
                         Counters *cnt) {
 	d_flush(PlainGrid{}, P, buf, n_ptr, clu_list, clu_count, L, cnt);
 }
-
-static __global__ void k_set_count(int *dst, const int *src) { *dst = *src; }
 
 // --------------------------------------------------------------------------------------------
 // Initialisation (integrator/integrator.hpp:100-160)
