@@ -226,7 +226,8 @@ __global__ void __launch_bounds__(BLOCK) kb_flux_receive(DG_BATCH_PARAMS) {
 template<class M, bool V>
 __global__ void __launch_bounds__(BLOCK, 3) kb_update(DG_BATCH_PARAMS) {
 	DG_BATCH_PROLOGUE
-	d_update<M, V>(g, a.P, cst, a.Ls.clu[s.L], s.n, s.dtL, s.epoch0 + 1, a.cnt);
+	d_update<M, V>(g, a.P, cst, a.Ls.clu[s.L], s.n, s.dtL, a.cnt);
+	d_stamp(g, a.P, a.Ls.clu[s.L], s.n, s.epoch0 + 1, a.cnt);
 }
 
 template<class M, bool V>

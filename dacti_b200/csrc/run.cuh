@@ -68,7 +68,7 @@ constexpr int RUN_THREADS = 512;
 // the items to the blocks' warps from the last one on, for the second of two stages that share a barrier: with
 // few items the two then run on different warps instead of one after the other.
 struct DealtGrid {
-	static constexpr bool DEEP = true;
+	static constexpr bool DEEP = true, EARLY = true;
 	int block, blocks;
 	bool rev;
 	__device__ __forceinline__ int begin(int) const {
@@ -95,13 +95,11 @@ __device__ __forceinline__ bool run_barrier(const RunArgs &a, unsigned &arrivals
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		unsigned seen;
-		asm volatile("fence.acq_rel.gpu;" ::: "memory");
-		asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(a.bar) : "memory");
+		asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(a.bar) : "memory");
 		int polls = 0;
 		++seen;
 		while ((int) (seen - arrivals) < 0 && ++polls < BARRIER_POLLS)
 			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
-		asm volatile("fence.acq_rel.gpu;" ::: "memory");
 		*s_ok = (int) (seen - arrivals) >= 0;
 	}
 	__syncthreads();
@@ -231,13 +229,14 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 
 		// the list of new cells, not in use before the regrid, holds the deferred cells' positions
 		d_face_sum<M, V, S>(g, P, C, a.B, list, n, L, dtL, stamp, s_ls.recv, s_ls.fresh, cnt);
+		d_stamp(r, P, list, n, e_upd, cnt);
 		if (!run_barrier(a, arrivals, &s_ok)) return;
 		// the receivers are cells of slower clusters, the updated cells those of this one
 		const bool deferred = __ldcg(&cnt->n_defer) > 0;
 		if (deferred) d_deferred<M, S>(g, P, list, s_ls.fresh, &cnt->n_defer, L, cnt);
 		if (__ldcg(&cnt->n_recv) > 0) d_flux_receive<M, S>(r, P, s_ls.recv, &cnt->n_recv, L, cnt);
 		if (deferred && !run_barrier(a, arrivals, &s_ok)) return;
-		d_update<M, V>(g, P, C, list, n, dtL, e_upd, cnt);
+		d_update<M, V>(g, P, C, list, n, dtL, cnt);
 		if (lead && blockIdx.x == 0) cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_tmp = 0;
 		if (!run_barrier(a, arrivals, &s_ok)) return;
 		if (lead && blockIdx.x == 0) cnt->n_recv = cnt->n_defer = 0;

@@ -764,13 +764,14 @@ private:
 		int e_upd = 0;                       // epoch of this substep's cell update
 		run_k(DG_K_FLUX, n, [&] { launch_face_sum(list, n, L, dtL, stamp_recv); });
 		run_k(DG_K_RECV, 0, [&] {
-			if (mixed_) k_flux_receive<M, float><<<grid_for((long long) n * LPC), BLOCK, 0, st_>>>(P_, Ls_.recv, list, Ls_.fresh, L, d_cnt_);
-			else k_flux_receive<M, double><<<grid_for((long long) n * LPC), BLOCK, 0, st_>>>(P_, Ls_.recv, list, Ls_.fresh, L, d_cnt_);
+			e_upd       = ++epoch_;
+			const int gr = grid_for((long long) n * LPC);
+			if (mixed_) k_flux_receive<M, float><<<gr, BLOCK, 0, st_>>>(P_, Ls_.recv, list, Ls_.fresh, n, L, e_upd, d_cnt_);
+			else k_flux_receive<M, double><<<gr, BLOCK, 0, st_>>>(P_, Ls_.recv, list, Ls_.fresh, n, L, e_upd, d_cnt_);
 		});
 		run_k(DG_K_UPDATE, n, [&] {
-			e_upd = ++epoch_;
-			if (visc_) k_update<M, true><<<g, BLOCK, 0, st_>>>(P_, C_, list, n, dtL, e_upd, d_cnt_);
-			else k_update<M, false><<<g, BLOCK, 0, st_>>>(P_, C_, list, n, dtL, e_upd, d_cnt_);
+			if (visc_) k_update<M, true><<<g, BLOCK, 0, st_>>>(P_, C_, list, n, dtL, d_cnt_);
+			else k_update<M, false><<<g, BLOCK, 0, st_>>>(P_, C_, list, n, dtL, d_cnt_);
 		});
 		run_k(DG_K_SLOPE, n, [&] { launch_slope(list, n); });
 		if constexpr (M::MULTI) multiphase_aux(list, n, L, e_upd);

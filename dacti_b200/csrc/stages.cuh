@@ -25,13 +25,14 @@ __device__ __forceinline__ int gstride() { return gridDim.x * blockDim.x; }
 // Which warp-sized work items a warp of a stage takes: items [begin, end) in steps of step(). A launch of
 // its own walks the whole grid; a batched launch gives each tree a range of blocks.
 struct PlainGrid {
-	static constexpr bool DEEP = false;  // interp_pt's
+	static constexpr bool DEEP = false;   // interp_pt's
+	static constexpr bool EARLY = false;  // d_face_sum asks for records before it knows that it needs them
 	__device__ __forceinline__ int begin(int) const { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
 	__device__ __forceinline__ int end(int items) const { return items; }
 	__device__ __forceinline__ int step() const { return (gridDim.x * blockDim.x) >> 5; }
 };
 struct BlockRange {
-	static constexpr bool DEEP = false;
+	static constexpr bool DEEP = false, EARLY = false;
 	int first, count;  // blocks [first, first + count) of the launch
 	__device__ __forceinline__ int begin(int) const { return (((int) blockIdx.x - first) * blockDim.x + threadIdx.x) >> 5; }
 	__device__ __forceinline__ int end(int items) const { return items; }
@@ -131,20 +132,48 @@ __device__ __forceinline__ S pick_row_dt(const S *du, int dim) {
 // the right state and the face keeps the owner's centre (the reference relabels face.dir = 1).
 // Across a periodic wrap the non-owner's centre moves by the active size.
 // --------------------------------------------------------------------------------------------
-template<class M, bool V, class S>
-__device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, int owner, int other, int dim, int dir_o,
-                                              double dtL, double *Fout) {
+// The reconstruction state of a face's two cells. KEEP holds their centres (along the face's dimension) and times
+// too, for a face whose states are asked for ahead; without it they are read where they are used, which spares the
+// registers of the launches.
+template<class M, class S, bool KEEP>
+struct FaceState {
+	S pl[M::E], hl[M::E], sl[M::E], pr[M::E], hr[M::E], sr[M::E], kl = 0, kr = 0, nl = 0, nr = 0;
+	double geo[KEEP ? 4 : 1];
+	__device__ __forceinline__ void load(const Pool &P, int iL, int iR, int dim) {
+		if constexpr (KEEP) {
+			geo[0] = at(P.center, P.cap, dim, iL), geo[1] = at(P.center, P.cap, dim, iR);
+			geo[2] = P.t[iL], geo[3] = P.t[iR];
+		}
+		load_face_rec<M, S>(P, iL, dim, pl, hl, sl, kl, nl);
+		load_face_rec<M, S>(P, iR, dim, pr, hr, sr, kr, nr);
+	}
+	// k: 0 left cell, 1 right cell
+	__device__ __forceinline__ double center(const Pool &P, int i, int dim, int k) const {
+		if constexpr (KEEP) return k == 0 ? geo[0] : geo[1];
+		else return at(P.center, P.cap, dim, i);
+	}
+	__device__ __forceinline__ double time(const Pool &P, int i, int k) const {
+		if constexpr (KEEP) return k == 0 ? geo[2] : geo[3];
+		else return P.t[i];
+	}
+};
+
+// The flux from the two cells' states (loaded already with KEEP); iL and iR are the left and right cells, one of them
+// the owner, at tree level lo.
+template<class M, bool V, class S, bool KEEP>
+__device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, FaceState<M, S, KEEP> &s, int iL, int iR, int lo, int dim,
+                                              int dir_o, double dtL, double *Fout) {
 	constexpr int E = M::E, D = M::D;
 	const int cap   = P.cap;
-	const int lo    = P.level[owner];
 	const double so = C.size[lo];
-	const double co = at(P.center, cap, dim, owner);
+	const int owner = dir_o == 1 ? iL : iR, other = dir_o == 1 ? iR : iL;
+	const double co = s.center(P, owner, dim, 1 - dir_o);
 	const double fc = co + so * (dir_o - 0.5);
-	const double t0 = P.t[owner];
+	const double t0 = s.time(P, owner, 1 - dir_o);
 	const double t1 = t0 + dtL;
 	const double area = C.area[lo];
 
-	double cx = at(P.center, cap, dim, other);
+	double cx = s.center(P, other, dim, dir_o);
 	if (C.periodic[dim]) {
 		if (dir_o == 1) {
 			if (co + so > 0.5 * C.active[dim]) cx += C.active[dim];
@@ -152,17 +181,14 @@ __device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, in
 			if (co - so < -0.5 * C.active[dim]) cx -= C.active[dim];
 		}
 	}
-	const int iL = dir_o == 1 ? owner : other;
-	const int iR = dir_o == 1 ? other : owner;
 	const double cL = dir_o == 1 ? co : cx;
 	const double cR = dir_o == 1 ? cx : co;
-
-	S pl[E], hl[E], sl[E], pr[E], hr[E], sr[E], kl = 0, kr = 0, nl = 0, nr = 0;
-	load_face_rec<M, S>(P, iL, dim, pl, hl, sl, kl, nl);
-	load_face_rec<M, S>(P, iR, dim, pr, hr, sr, kr, nr);
+	if constexpr (!KEEP) s.load(P, iL, iR, dim);
+	const S(&pl)[E] = s.pl, (&hl)[E] = s.hl, (&sl)[E] = s.sl, (&pr)[E] = s.pr, (&hr)[E] = s.hr, (&sr)[E] = s.sr;
+	const S kl = s.kl, kr = s.kr, nl = s.nl, nr = s.nr;
 	const double tm   = 0.5 * (t1 + t0);
-	const double dt_n = tm - P.t[iL];
-	const double dt_p = tm - P.t[iR];
+	const double dt_n = tm - s.time(P, iL, 0);
+	const double dt_p = tm - s.time(P, iR, 1);
 	// Hancock predictor at the face (reconstruction); geometry and time offsets stay FP64
 	const S xl = (S) (fc - cL), xr = (S) (fc - cR), tl = (S) dt_n, tr = (S) dt_p;
 	S pn[E], pp[E];
@@ -223,6 +249,14 @@ __device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, in
 	} else {
 		for (int q = 0; q < M::F; ++q) Fout[q] = (double) F[q] * area * dtf;
 	}
+}
+
+template<class M, bool V, class S>
+__device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, int owner, int other, int dim, int dir_o,
+                                              double dtL, double *Fout) {
+	const int iL = dir_o == 1 ? owner : other, iR = dir_o == 1 ? other : owner;
+	FaceState<M, S, false> s;
+	interior_flux<M, V, S, false>(P, C, s, iL, iR, P.level[owner], dim, dir_o, dtL, Fout);
 }
 
 // Boundary::boundary_flux (integrator/boundary.hpp:130-160), from the cell-centre state.
@@ -398,6 +432,7 @@ __device__ __forceinline__ double pair_terms(const double *f) {
 template<class M, bool V, class S = double, class Grid>
 __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, int L, double dtL, int stamp, int32_t *recv, int32_t *defer, Counters *cnt) {
 	constexpr int NF = 2 * M::D, G = NF, GW = 32 / G, F = M::F;
+	constexpr bool EARLY = Grid::EARLY && !M::MULTI;  // the five-equation states do not fit the registers that long
 	const int cap    = P.cap;
 	const int lane   = threadIdx.x & 31;
 	const int grp    = lane / G;  // the lane's cell within the warp; lanes past GW * G idle
@@ -427,11 +462,17 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 					for (int q = 0; q < F; ++q) acc[q] = 0.0 - (double) (S) Fb[q];
 					code = DF_TERM;
 				}
-			} else if (!(P.flags[nb] & F_LEAF)) {
-				code = DF_HANG;
-			} else {
+			} else if (const uint32_t fn = P.flags[nb]; EARLY || (fn & F_LEAF)) {
+				// both cells' states are asked for before their facts say who owns the face
+				const int iL = dir == 1 ? i : nb, iR = dir == 1 ? nb : i;
+				const int back = P.nbr[(size_t) (f ^ 1) * cap + nb];
+				FaceState<M, S, true> st;
+				if constexpr (EARLY) st.load(P, iL, iR, dim);
 				const int li = P.level[i], ai = P.acti[i], ln = P.level[nb], an = P.acti[nb];
 				int own = -1, fo = f;
+				if (!(fn & F_LEAF)) {
+					code = DF_HANG;
+				} else
 				if (an <= ai && (ln < li || (ln == li && (dir == 1 || an < ai)))) {
 					own = i;
 				} else if (ln == li && P.clu[nb] == L && ai <= an && (dir == 0 || ai < an)) {
@@ -439,9 +480,14 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 					fo  = f ^ 1;
 				}
 				if (own >= 0) {
-					const int other = own == i ? nb : P.nbr[(size_t) fo * cap + nb];
+					const int other = own == i ? nb : back;
 					double Fi[F];
-					interior_flux<M, V, S>(P, C, own, other, dim, fo & 1, dtL, Fi);
+					if constexpr (EARLY) {
+						if (other != nb && other != i) st.load(P, (fo & 1) ? own : other, (fo & 1) ? other : own, dim);
+						interior_flux<M, V, S, true>(P, C, st, (fo & 1) ? own : other, (fo & 1) ? other : own, own == i ? li : ln, dim, fo & 1, dtL, Fi);
+					} else {
+						interior_flux<M, V, S>(P, C, own, other, dim, fo & 1, dtL, Fi);
+					}
 					code = DF_TERM;
 					if (own == i && (ln < li || P.clu[nb] != L)) {
 						code   = DF_RAW;
@@ -457,6 +503,8 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 						acc[q] = dir ? 0.0 - v : 0.0 + v;
 					}
 				}
+			} else {
+				code = DF_HANG;
 			}
 		}
 		const unsigned lo = __ballot_sync(0xffffffffu, code & 1), hi = __ballot_sync(0xffffffffu, code & 2);
@@ -557,13 +605,28 @@ __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS) k_face_sum(Pool
 	d_face_sum<M, V, S>(PlainGrid{}, P, C, B, list, n, L, dtL, stamp, recv, defer, cnt);
 }
 
+// Stamps the ancestors of the cells that the substep updates, for the subtree means that the stages after the
+// update form. The walk is a chain of dependent loads and needs nothing of the update, so it runs beside the face
+// sums of a run (or in the receive launch) instead of at the end of every update.
+template<class Grid>
+__device__ __forceinline__ void d_stamp(const Grid &g, const Pool &P, const int32_t *list, int n, int epoch, Counters *cnt) {
+	const int coarsest = __ldcg(&cnt->coarsest);
+	const int items    = warp_items(n, 32);
+	// warp-uniform loop: the whole warp stamps its cells' ancestors together
+	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
+		const int tid = it * 32 + (threadIdx.x & 31);
+		mark_up_warp(P, tid < n ? P.parent[list[tid]] : 0, epoch, coarsest);
+	}
+}
+
 // The receivers' sums and the deferred cells' face sums: both gather face-flux slots of the running cluster
-// and neither reads what the other writes.
+// and neither reads what the other writes. With them the stamps of the update to come.
 template<class M, class T = double>
-__global__ void __launch_bounds__(BLOCK) k_flux_receive(Pool P, const int32_t *recv, const int32_t *list, const int32_t *defer,
-                                                        int L, Counters *cnt) {
+__global__ void __launch_bounds__(BLOCK, 3) k_flux_receive(Pool P, const int32_t *recv, const int32_t *list, const int32_t *defer,
+                                                        int n, int L, int epoch, Counters *cnt) {
 	d_flux_receive<M, T>(PlainGrid{}, P, recv, &cnt->n_recv, L, cnt);
 	d_deferred<M, T>(PlainGrid{}, P, list, defer, &cnt->n_defer, L, cnt);
+	d_stamp(PlainGrid{}, P, list, n, epoch, cnt);
 }
 
 // The same face sums over tiles of TC consecutive list positions, one 128-thread block per tile. After
@@ -736,16 +799,13 @@ k_face_tile(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L, doub
 // only when the receive stage has marked the cell. Without viscous terms (V = false) the gradient
 // inputs are never read, so t_slope is not maintained.
 template<class M, bool V, class Grid>
-__device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Consts &C, const int32_t *list, int n, double dtL, int epoch, Counters *cnt) {
+__device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Consts &C, const int32_t *list, int n, double dtL, Counters *cnt) {
 	constexpr int E = M::E;
 	const int cap  = P.cap;
 	const int lane = threadIdx.x & 31;
-	const int coarsest = __ldcg(&cnt->coarsest);
-	// warp-uniform loop: the whole warp stamps the updated cells' ancestors together
 	const int items = warp_items(n, 32);
 	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
 		const int tid = it * 32 + lane;
-		int up        = 0;
 		if (tid < n) {
 			const int i  = list[tid];
 			const int li = P.level[i];
@@ -807,15 +867,12 @@ __device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Con
 				P.flags[i] = fl0 & ~F_RECV;
 			}
 			P.t[i] = P.t[i] + dtL;
-			up     = P.parent[i];
 		}
-		mark_up_warp(P, up, epoch, coarsest);
 	}
 }
 template<class M, bool V>
-__global__ void __launch_bounds__(BLOCK, 3) k_update(Pool P, Consts C, const int32_t *list, int n, double dtL, int epoch,
-                                                     Counters *cnt) {
-	d_update<M, V>(PlainGrid{}, P, C, list, n, dtL, epoch, cnt);
+__global__ void __launch_bounds__(BLOCK, 3) k_update(Pool P, Consts C, const int32_t *list, int n, double dtL, Counters *cnt) {
+	d_update<M, V>(PlainGrid{}, P, C, list, n, dtL, cnt);
 }
 
 
@@ -837,15 +894,13 @@ __device__ __forceinline__ int32_t neighbour_value(const Pool &P, const Consts &
 	constexpr int E = M::E;
 	const int nb = P.nbr[(size_t) f * P.cap + i];
 	if (nb == 0) return 0;
+	// the neighbour's own state is asked for before the flags say whether it is a leaf: one load less in the chain
 	const uint32_t fl = P.flags[nb];
 	const int ln      = P.level[nb];
 	double w[E + 1];
-	if (!(fl & F_LEAF)) {
-		interp_pt<M, DEEP>(P, status, nb, epoch, w);
-	} else {
-		load_p_rec<M>(P, nb, w);
-		w[E] = P.t[nb];
-	}
+	load_p_rec<M>(P, nb, w);
+	w[E] = P.t[nb];
+	if (!(fl & F_LEAF)) interp_pt<M, DEEP>(P, status, nb, epoch, w);
 #pragma unroll
 	for (int q = 0; q < E; ++q) v[q] = w[q];
 	tv   = w[E];
