@@ -16,7 +16,7 @@ namespace dg {
 
 struct DeviceMemory {
 	static constexpr size_t KEEP      = size_t(4) << 30;
-	static constexpr size_t KEEP_IDLE = size_t(1) << 30;
+	static constexpr size_t KEEP_IDLE = size_t(4) << 30;
 
 	cudaMemPool_t pool  = nullptr;
 	cudaStream_t stream = nullptr;  // of frees whose last use the host has waited for

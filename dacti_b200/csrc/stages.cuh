@@ -1384,12 +1384,18 @@ __global__ void k_regrid(Pool P, Consts C, const int32_t *split_list, const int3
 // Domain::update_neighbors for one active leaf (integrator/domain.hpp:249-293): faces without a
 // boundary get the node found at the same level (or the coarser leaf); a neighbour more than one
 // level coarser is flagged should_split.
+// `near`: what is known of the other side during a regrid's repair: NEAR_NONE, NEAR_NEW (i is a cell that the regrid
+// made), or a cell that lies against the face.
+constexpr int NEAR_NONE = -1, NEAR_NEW = -2;
 template<class M>
-__device__ void update_neighbor_face(const Pool &P, const Consts &C, int i, int dim, int dir) {
-	const int cap = P.cap;
-	const int f   = 2 * dim + dir;
+__device__ __forceinline__ void update_neighbor_face(const Pool &P, const Consts &C, int i, int dim, int dir, int near = NEAR_NONE) {
+	constexpr int D = M::D;
+	const int cap   = P.cap;
+	const int f     = 2 * dim + dir;
 	if (P.bc[(size_t) f * cap + i] >= 0) return;
-	const int nb = find_neighbor<M::D>(P, C, i, dim, dir);
+	const int nb = near == NEAR_NONE  ? find_neighbor<D>(P, C, i, dim, dir)
+	               : near == NEAR_NEW ? find_neighbor_new<D>(P, C, i, dim, dir)
+	                                  : find_neighbor_at<D>(P, C, i, dim, dir, near);
 	if (nb == 0 || !(P.flags[nb] & F_ACTIVE)) return;
 	P.nbr[(size_t) f * cap + i] = nb;
 	if (P.level[nb] < P.level[i] - 1) atomicOr(&P.flags[nb], (uint32_t) F_SHOULD_SPLIT);
@@ -1406,7 +1412,7 @@ __device__ void update_neighbors_leaf(const Pool &P, const Consts &C, int i) {
 // neighbour's subtree that does not touch the face towards the new cell finds the same neighbours as
 // before, so the reference's full subtree update leaves it unchanged.
 template<class M>
-__device__ void update_face_subtree(const Pool &P, const Consts &C, uint32_t *status, int root, int dim, int dir) {
+__device__ void update_face_subtree(const Pool &P, const Consts &C, uint32_t *status, int root, int dim, int dir, int near) {
 	constexpr int NC = 1 << M::D, NH = NC / 2;
 	constexpr int CAP = NH * MAX_TREE;
 	int stack[CAP];
@@ -1417,7 +1423,7 @@ __device__ void update_face_subtree(const Pool &P, const Consts &C, uint32_t *st
 		if (x == 0) continue;  // a subtree without active leaves that the host left out
 		const uint32_t fl = P.flags[x];
 		if (fl & F_LEAF) {
-			if (fl & F_ACTIVE) update_neighbor_face<M>(P, C, x, dim, dir);
+			if (fl & F_ACTIVE) update_neighbor_face<M>(P, C, x, dim, dir, near);
 			continue;
 		}
 		for (int c = NC - 1; c >= 0; --c) {
@@ -1433,7 +1439,7 @@ __device__ void update_face_subtree(const Pool &P, const Consts &C, uint32_t *st
 
 // update_neighbors applied to a node: leaves directly, non-leaves through all their descendants.
 template<class M>
-__device__ void update_neighbors_subtree(const Pool &P, const Consts &C, uint32_t *status, int root) {
+__device__ __noinline__ void update_neighbors_subtree(const Pool &P, const Consts &C, uint32_t *status, int root) {
 	constexpr int NC = 1 << M::D;
 	constexpr int CAP = 8 * MAX_TREE;
 	int stack[CAP];
@@ -1472,22 +1478,22 @@ __device__ __forceinline__ void d_nbr_fresh(const Grid &g, const Pool &P, const 
 	const int lane   = threadIdx.x & 31;
 	const int sub    = lane & (G - 1);
 	const int items  = warp_items(n, GW);
-	auto behind = [&](int i, int f) {
-		const int nb = P.nbr[(size_t) f * cap + i];
-		if (nb != 0 && ((P.flags[nb] & F_ACTIVE) || !(P.flags[nb] & F_LEAF)))
-			update_face_subtree<M>(P, C, &cnt->status, nb, f >> 1, 1 - (f & 1));
-	};
 	for (int it = g.begin(items), last = g.end(items); it < last; it += g.step()) {
 		const int slot = it * GW + lane / G;
 		if (slot >= n || sub >= NF) continue;
 		const int i       = fresh[slot];
 		const uint32_t fl = P.flags[i];
-		if (fl & F_LEAF) {
-			if (fl & F_ACTIVE) update_neighbor_face<M>(P, C, i, sub >> 1, sub & 1);
-			behind(i, sub);
-		} else if (sub == 0) {
-			update_neighbors_subtree<M>(P, C, &cnt->status, i);
-			for (int f = 0; f < NF; ++f) behind(i, f);
+		int f0 = sub, f1 = sub + 1;
+		if (!(fl & F_LEAF)) {
+			f0 = 0, f1 = sub == 0 ? NF : 0;
+			if (sub == 0) update_neighbors_subtree<M>(P, C, &cnt->status, i);
+		} else if (fl & F_ACTIVE) {
+			update_neighbor_face<M>(P, C, i, sub >> 1, sub & 1, NEAR_NEW);
+		}
+		for (int f = f0; f < f1; ++f) {
+			const int nb = P.nbr[(size_t) f * cap + i];
+			if (nb != 0 && ((P.flags[nb] & F_ACTIVE) || !(P.flags[nb] & F_LEAF)))
+				update_face_subtree<M>(P, C, &cnt->status, nb, f >> 1, 1 - (f & 1), i);
 		}
 	}
 }
@@ -1547,10 +1553,12 @@ __device__ __forceinline__ void d_reassign(const Grid &g, const Pool &P, const C
 		else if (stays) append(Ls.tmp, &cnt->n_tmp, i, P.cap, &cnt->status);
 	}
 }
+// The walks that are rarely needed are calls, which take the pool and the constants by reference: as grid constants
+// they are not copied to every thread's stack for that (2.5 KB; the copies took five times the stage's time).
 // After the regrid, in one launch: the neighbour repair reads no time level and the reassignment of the old list
 // no neighbour.
 template<class M>
-__global__ void k_repair(Pool P, Consts C, const int32_t *fresh, const int32_t *list, int n, int L, double dtL, int counter_L, Lists Ls,
+__global__ void k_repair(const __grid_constant__ Pool P, const __grid_constant__ Consts C, const int32_t *fresh, const int32_t *list, int n, int L, double dtL, int counter_L, Lists Ls,
                          Counters *cnt, uint8_t *stay) {
 	d_reassign<M>(PlainGrid{}, P, C, list, nullptr, n, L, dtL, counter_L, Ls, cnt, stay);
 	d_nbr_fresh<M>(PlainGrid{}, P, C, &cnt->n_new, fresh, cnt);
@@ -1627,7 +1635,7 @@ __global__ void k_init_cells(Pool P, Consts C, const int32_t *list, int n, Count
 }
 
 template<class M>
-__global__ void k_nbr_init(Pool P, Consts C, const int32_t *list, int n) {
+__global__ void k_nbr_init(const __grid_constant__ Pool P, const __grid_constant__ Consts C, const int32_t *list, int n) {
 	for (int tid = gtid(); tid < n; tid += gstride()) update_neighbors_leaf<M>(P, C, list[tid]);
 }
 

@@ -53,38 +53,98 @@ __device__ __forceinline__ void store_p_rec(const Pool &P, int i, const double *
 
 __device__ __forceinline__ void set_status(uint32_t *status, uint32_t bit) { atomicOr(status, bit); }
 
+// The centre of the same-level neighbour of node i across face (dim, dir) in integer coordinates of its level
+// (integrator/domain.hpp:65-82, 249-293); false when it lies outside the active box of a non-periodic dimension.
+template<int D>
+__device__ __forceinline__ bool neighbor_target(const Pool &P, const Consts &C, int i, int l, int dim, int dir, int *tc, int &own) {
+	for (int d = 0; d < D; ++d) tc[d] = P.coord[(size_t) d * P.cap + i];
+	own = 0;
+	for (int d = 0; d < D; ++d)
+		if (d == dim) own = tc[d], tc[d] += 2 * dir - 1;
+	int t = 0;
+	for (int d = 0; d < D; ++d)
+		if (d == dim) t = tc[d];
+	const int lo = C.a0[l][dim], hi = C.a0[l][dim] + C.na[l][dim];
+	if (t < lo || t >= hi) {
+		if (!C.periodic[dim]) return false;
+		t += (t < lo) ? C.na[l][dim] : -C.na[l][dim];
+	}
+	for (int d = 0; d < D; ++d)
+		if (d == dim) tc[d] = t;
+	return true;
+}
+
+// From node a at level m, which contains the cell tc of level l, down to it: the leaf on the way or the cell.
+template<int D>
+__device__ __forceinline__ int descend(const Pool &P, int a, int m, const int *tc, int l) {
+	for (int guard = 0; guard < MAX_TREE && !(P.flags[a] & F_LEAF) && m < l; ++guard) {
+		int ci = 0;
+		for (int d = 0; d < D; ++d) ci |= ((tc[d] >> (l - m - 1)) & 1) << d;
+		a = P.child[(size_t) ci * P.cap + a];
+		++m;
+	}
+	return a;
+}
+
 // Domain::find(location, node.tree_level) for the face (dim, dir) of node i, as used by
 // update_neighbors (integrator/domain.hpp:65-82, 249-293, 407-417). The location is the centre of
 // the same-level neighbour; in integer cell coordinates the root-down descent becomes: step up to
 // the common ancestor, then down towards the target until a leaf or the node's level. Returns 0 when
 // the location lies outside the active box of a non-periodic dimension.
 template<int D>
-__device__ int find_neighbor(const Pool &P, const Consts &C, int i, int dim, int dir) {
-	const int cap = P.cap;
-	const int l   = P.level[i];
-	int tc[3];
-	for (int d = 0; d < D; ++d) tc[d] = P.coord[(size_t) d * cap + i];
-	tc[dim] += 2 * dir - 1;
-	const int lo = C.a0[l][dim], hi = C.a0[l][dim] + C.na[l][dim];
-	if (tc[dim] < lo || tc[dim] >= hi) {
-		if (!C.periodic[dim]) return 0;
-		tc[dim] += (tc[dim] < lo) ? C.na[l][dim] : -C.na[l][dim];
-	}
-	const int own = P.coord[(size_t) dim * cap + i];
+__device__ __noinline__ int find_neighbor(const Pool &P, const Consts &C, int i, int dim, int dir) {
+	const int l = P.level[i];
+	int tc[3], own;
+	if (!neighbor_target<D>(P, C, i, l, dim, dir, tc, own)) return 0;
+	int t = 0;
+	for (int d = 0; d < D; ++d)
+		if (d == dim) t = tc[d];
 	int a = i, m = l;
 	// ascend while the ancestor at level m does not contain the target along `dim`
-	for (int guard = 0; guard < MAX_TREE && m > 0 && ((tc[dim] >> (l - m)) != (own >> (l - m))); ++guard) {
+	for (int guard = 0; guard < MAX_TREE && m > 0 && ((t >> (l - m)) != (own >> (l - m))); ++guard) {
 		a = P.parent[a];
 		--m;
 	}
-	// descend towards the target
-	for (int guard = 0; guard < MAX_TREE && !(P.flags[a] & F_LEAF) && m < l; ++guard) {
-		int ci = 0;
-		for (int d = 0; d < D; ++d) ci |= ((tc[d] >> (l - m - 1)) & 1) << d;
-		a = P.child[(size_t) ci * cap + a];
-		++m;
-	}
-	return a;
+	return descend<D>(P, a, m, tc, l);
+}
+
+// find_neighbor during the regrid's repair, from a node that should hold the target or lie below a node that does.
+// The walk up to the common ancestor is long where that is far (to the root across the middle of the domain), and
+// the slowest lane ends the stage. A hint that this regrid removed has its parent in the tree; whether the node
+// contains the target is checked by its coordinates, and find_neighbor takes over where it does not. Any node of the
+// tree that contains the target leads down to the same leaf or cell as the root.
+template<int D>
+__device__ __forceinline__ int find_neighbor_from(const Pool &P, const Consts &C, int i, int l, const int *tc, int dim, int dir, int a) {
+	if (a != 0 && (P.flags[a] & F_GARBAGE)) a = P.parent[a];
+	int m = P.level[a];
+	for (; a != 0 && m > l; --m) a = P.parent[a];
+	bool holds = a != 0 && m >= 0 && !(P.flags[a] & F_GARBAGE);
+	for (int d = 0; d < D; ++d) holds = holds && P.coord[(size_t) d * P.cap + a] == tc[d] >> max(l - m, 0);
+	return holds ? descend<D>(P, a, m, tc, l) : find_neighbor<D>(P, C, i, dim, dir);
+}
+
+// find_neighbor for a cell that the running regrid made: from its parent for a sibling, else from a link that was
+// right before the regrid, what the parent of a new child had behind the face, or a child of a coarsened parent.
+template<int D>
+__device__ __forceinline__ int find_neighbor_new(const Pool &P, const Consts &C, int i, int dim, int dir) {
+	const int cap = P.cap, l = P.level[i], par = P.parent[i], f = 2 * dim + dir;
+	int tc[3], own;
+	if (!neighbor_target<D>(P, C, i, l, dim, dir, tc, own)) return 0;
+	int t = 0;
+	for (int d = 0; d < D; ++d)
+		if (d == dim) t = tc[d];
+	if (l > 0 && (t >> 1) == (own >> 1)) return descend<D>(P, par, l - 1, tc, l);
+	const int kid = P.child[(size_t) (dir << dim) * cap + i];  // a child on the face, if i has or had children
+	return find_neighbor_from<D>(P, C, i, l, tc, dim, dir, P.nbr[(size_t) f * cap + (kid != 0 ? kid : par)]);
+}
+
+// find_neighbor for a cell whose face (dim, dir) lies against the cell `near`.
+template<int D>
+__device__ __forceinline__ int find_neighbor_at(const Pool &P, const Consts &C, int i, int dim, int dir, int near) {
+	const int l = P.level[i];
+	int tc[3], own;
+	if (!neighbor_target<D>(P, C, i, l, dim, dir, tc, own)) return 0;
+	return find_neighbor_from<D>(P, C, i, l, tc, dim, dir, near);
 }
 
 // Subtree means of non-leaf nodes. Domain::interpolate_p / interpolate_t (integrator/domain.hpp:
