@@ -138,6 +138,16 @@ int dg_read_cells(dg_solver *s, int *levels, double *data, long long max_cells, 
 	});
 }
 
+int dg_read_fields(dg_solver *s, const dg_cell_fields *f, long long max_cells, long long *n_out) {
+	if (!s || !f || !f->level || !f->acti || !f->center || !f->t || !f->u || !f->p || !f->error || !f->max_dt || !f->cfl)
+		return DG_ERR_ARG;
+	if (s->impl->model_id() == DG_MULTI && !f->k) return DG_ERR_ARG;
+	return guarded(s, [&] {
+		long long n = s->impl->read_fields(*f, max_cells);
+		if (n_out) *n_out = n;
+	});
+}
+
 int dg_read_slopes(dg_solver *s, double *slopes, long long max_cells, long long *n_out) {
 	if (!s || !slopes) return DG_ERR_ARG;
 	return guarded(s, [&] {

@@ -38,6 +38,7 @@ public:
 	virtual void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user, int peers = 1) = 0;
 	virtual long long cell_count() = 0;
 	virtual long long read_cells(int *levels, double *data, long long max_cells) = 0;
+	virtual long long read_fields(const dg_cell_fields &f, long long max_cells) = 0;
 	virtual long long read_cells_via(int *levels, double *data, long long max_cells, void *scratch, size_t bytes) = 0;
 	virtual long long read_slopes(double *data, long long max_cells) = 0;
 	virtual long long read_gradients(double *data, long long max_cells) = 0;
@@ -556,13 +557,13 @@ public:
 	}
 
 	// ---------------------------------------------------------------------------------------
-	template<typename T>
-	void upload_soa(T *dst, const T *src_rowmajor, int n, int comps) {
-		std::vector<T> tmp((size_t) n * comps);
-		for (int i = 0; i < n; ++i)
-			for (int c = 0; c < comps; ++c) tmp[(size_t) c * n + i] = src_rowmajor[(size_t) i * comps + c];
-		for (int c = 0; c < comps; ++c)
-			DG_CUDA(cudaMemcpy(dst + (size_t) c * P_.cap, tmp.data() + (size_t) c * n, sizeof(T) * n, cudaMemcpyHostToDevice));
+	// Rows of `comps` values per node into the pool, through a device buffer that holds the largest field.
+	template<class To, class From>
+	void upload_rows(To *dst, const From *src, int n, int comps, void *buf) {
+		if (n <= 0 || comps <= 0) return;
+		DG_CUDA(cudaMemcpyAsync(buf, src, sizeof(From) * (size_t) n * comps, cudaMemcpyHostToDevice, st_));
+		k_take_rows<From, To><<<grid_for((long long) n * comps), BLOCK, 0, st_>>>((const From *) buf, dst, n, comps, P_.cap);
+		DG_CUDA(cudaGetLastError());
 	}
 
 	std::vector<int32_t> active_leaves_;
@@ -570,46 +571,29 @@ public:
 	void upload_tree(const dg_case &c) {
 		const int n = c.n_nodes;
 		DG_CUDA(cudaStreamSynchronize(st_));
-		std::vector<int8_t> lv(n), ac(n, -1), cl(n, CLU_NONE);
-		std::vector<int32_t> coord((size_t) n * D, 0);
-		std::vector<int16_t> bc((size_t) n * NF);
 		max_tree_level_ = C_.max_refinement_level;
 		for (int z = 0; z < C_.n_zones; ++z) max_tree_level_ = std::max(max_tree_level_, C_.zlevel[z]);
-		for (int i = 0; i < n; ++i) {
-			lv[i] = (int8_t) c.level[i];
-			max_tree_level_ = std::max(max_tree_level_, (int) c.level[i]);
-			for (int f = 0; f < NF; ++f) bc[(size_t) i * NF + f] = (int16_t) c.bc[(size_t) i * NF + f];
-		}
+		int deepest = 0;
+		for (int i = 0; i < n; ++i) deepest = std::max(deepest, (int) c.level[i]);
+		max_tree_level_ = std::max(max_tree_level_, deepest);
+		void *buf = nullptr;
+		DG_CUDA(mem_alloc(&buf, 8 * (size_t) std::max({NC, NF, D, E}) * (size_t) std::max(n, 1), st_));
+		upload_rows(P_.parent, c.parent, n, 1, buf);
+		upload_rows(P_.child, c.children, n, NC, buf);
+		upload_rows(P_.level, c.level, n, 1, buf);
+		upload_rows(P_.flags, (const uint32_t *) c.flags, n, 1, buf);
+		upload_rows(P_.bc, c.bc, n, NF, buf);
+		upload_rows(P_.center, c.center, n, D, buf);
+		upload_rows(P_.p, c.p, n, E, buf);
+		mem_free(buf, st_);
+		DG_CUDA(cudaMemsetAsync(P_.acti, 0xff, n, st_));  // -1
+		DG_CUDA(cudaMemsetAsync(P_.clu, 0xff, n, st_));   // CLU_NONE
 		// integer coordinates, parents before children
-		std::vector<int> order;
-		order.reserve(n);
-		if (n > 1) order.push_back(1);
-		for (size_t h = 0; h < order.size(); ++h) {
-			int x = order[h];
-			if (c.flags[x] & DG_F_LEAF) continue;
-			for (int k = 0; k < NC; ++k) {
-				int ch = c.children[(size_t) x * NC + k];
-				if (ch <= 0) continue;
-				for (int d = 0; d < D; ++d) coord[(size_t) ch * D + d] = 2 * coord[(size_t) x * D + d] + ((k >> d) & 1);
-				order.push_back(ch);
-			}
-		}
-		upload_soa(P_.parent, c.parent, n, 1);
-		upload_soa(P_.child, c.children, n, NC);
-		upload_soa(P_.level, lv.data(), n, 1);
-		upload_soa(P_.acti, ac.data(), n, 1);
-		upload_soa(P_.clu, cl.data(), n, 1);
-		upload_soa(P_.flags, (const uint32_t *) c.flags, n, 1);
-		upload_soa(P_.coord, coord.data(), n, D);
-		upload_soa(P_.bc, bc.data(), n, NF);
-		upload_soa(P_.center, c.center, n, D);
-		upload_soa(P_.p, c.p, n, E);
+		for (int l = 1; l <= deepest; ++l) k_coords<D><<<grid_for(n), BLOCK, 0, st_>>>(P_, n, l);
 		// Node::error as the scene leaves it: -1 on every split child (integrator/domain.hpp:215), kept by
 		// leaves that never get an estimate (inactive ones) and summed by unsplit (domain.hpp:306-309)
-		{
-			std::vector<double> err((size_t) n, -1.0);
-			upload_soa(P_.err, err.data(), n, 1);
-		}
+		k_fill_f64<<<grid_for(n), BLOCK, 0, st_>>>(P_.err, -1.0, n);
+		DG_CUDA(cudaGetLastError());
 		active_leaves_.clear();
 		for (int i = 1; i < n; ++i)
 			if ((c.flags[i] & DG_F_LEAF) && (c.flags[i] & DG_F_ACTIVE)) active_leaves_.push_back(i);
@@ -1271,6 +1255,43 @@ public:
 	long long cell_count() override {
 		long long n = 0;
 		for (int l = 0; l < MAX_ACTI; ++l) n += h_cnt_->clu[l] + h_cnt_->buf[l];
+		return n;
+	}
+
+	long long read_fields(const dg_cell_fields &f, long long max_cells) override {
+		const long long n = cell_count();
+		if (n > max_cells) throw dg_error(DG_ERR_ARG, "read buffer too small");
+		if (n == 0) return 0;
+		// one buffer, the arrays one after another
+		struct Part {
+			void *host;
+			size_t bytes;
+		};
+		const size_t d = sizeof(double) * (size_t) n, w = sizeof(int32_t) * (size_t) n;
+		const Part part[10] = {{f.center, d * D}, {f.t, d}, {f.u, d * E}, {f.p, d * E}, {f.error, d}, {f.max_dt, d}, {f.cfl, d},
+		                       {f.k, d * M::P}, {f.level, w}, {f.acti, w}};
+		size_t at[10], total = 0;
+		for (int k = 0; k < 10; ++k) at[k] = total, total += align_up(part[k].bytes);
+		char *buf = nullptr;
+		DG_CUDA(mem_alloc((void **) &buf, total, st_));
+		const FieldArrays o{(int32_t *) (buf + at[8]), (int32_t *) (buf + at[9]), (double *) (buf + at[0]), (double *) (buf + at[1]),
+		                    (double *) (buf + at[2]), (double *) (buf + at[3]), (double *) (buf + at[4]), (double *) (buf + at[5]),
+		                    (double *) (buf + at[6]), (double *) (buf + at[7])};
+		long long base = 0;
+		for (int pass = 0; pass < 2; ++pass) {
+			for (int l = 0; l < MAX_ACTI; ++l) {
+				const int cnt = pass == 0 ? h_cnt_->clu[l] : h_cnt_->buf[l];
+				if (cnt == 0) continue;
+				k_gather_fields<M><<<grid_for(cnt), BLOCK, 0, st_>>>(P_, pass == 0 ? Ls_.clu[l] : Ls_.buf[l], cnt, (int) base, o);
+				base += cnt;
+			}
+		}
+		cudaError_t e = cudaGetLastError();
+		for (int k = 0; k < 10 && e == cudaSuccess; ++k)
+			if (part[k].bytes > 0) e = cudaMemcpyAsync(part[k].host, buf + at[k], part[k].bytes, cudaMemcpyDeviceToHost, st_);
+		if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+		mem_free(buf, st_);
+		if (e != cudaSuccess) throw dg_error(DG_ERR_CUDA, std::string("read_fields: ") + cudaGetErrorString(e));
 		return n;
 	}
 

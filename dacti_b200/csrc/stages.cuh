@@ -1758,6 +1758,59 @@ __global__ void k_set_hold(Pool P, const int32_t *list, int n, int base, const u
 	}
 }
 
+// The arrays of a field-wise read-back on the device, one row per cell in each.
+struct FieldArrays {
+	int32_t *level, *acti;
+	double *center, *t, *u, *p, *err, *maxdt, *cfl, *k;
+};
+
+// Gather of the active cells field by field: each array goes to the host as it is, where records would be taken
+// apart there, at the price of a second pass over them in fresh memory.
+template<class M>
+__global__ void k_gather_fields(Pool P, const int32_t *list, int n, int base, FieldArrays o) {
+	constexpr int E = M::E, D = M::D;
+	const int cap = P.cap;
+	for (int tid = gtid(); tid < n; tid += gstride()) {
+		const int i    = list[tid];
+		const size_t r = (size_t) base + tid;
+		o.level[r]     = P.level[i];
+		o.acti[r]      = P.acti[i];
+		for (int d = 0; d < D; ++d) o.center[r * D + d] = at(P.center, cap, d, i);
+		o.t[r] = P.t[i];
+		for (int q = 0; q < E; ++q) o.u[r * E + q] = at(P.u, cap, q, i);
+		for (int q = 0; q < E; ++q) o.p[r * E + q] = at(P.p, cap, q, i);
+		o.err[r]   = P.err[i];
+		o.maxdt[r] = P.maxdt[i];
+		o.cfl[r]   = P.cfl[i];
+		for (int q = 0; q < M::P; ++q) o.k[r * M::P + q] = at(P.k, cap, q, i);
+	}
+}
+
+// The uploaded tree's rows (node by node, as the host keeps them) into the pool's arrays (component by component):
+// on the host the transposition was most of a large tree's construction.
+template<class From, class To>
+__global__ void k_take_rows(const From *__restrict__ src, To *__restrict__ dst, int n, int comps, int cap) {
+	for (long long t = gtid(); t < (long long) n * comps; t += gstride()) {
+		const int i = (int) (t / comps), c = (int) (t - (long long) i * comps);
+		dst[(size_t) c * cap + i] = (To) src[t];
+	}
+}
+static __global__ void k_fill_f64(double *a, double v, int n) {
+	for (int j = gtid(); j < n; j += gstride()) a[j] = v;
+}
+// Integer coordinates of the nodes at level l from their parents'.
+template<int D>
+__global__ void k_coords(Pool P, int n, int l) {
+	for (int i = gtid(); i < n; i += gstride()) {
+		if (i < 2 || P.level[i] != l) continue;
+		const int par = P.parent[i];
+		if (P.flags[par] & F_LEAF) continue;
+		for (int k = 0; k < (1 << D); ++k)
+			if (P.child[(size_t) k * P.cap + par] == i)
+				for (int d = 0; d < D; ++d) P.coord[(size_t) d * P.cap + i] = 2 * P.coord[(size_t) d * P.cap + par] + ((k >> d) & 1);
+	}
+}
+
 // Gather of active-cell records for the read-back API.
 template<class M>
 __global__ void k_gather_cells(Pool P, const int32_t *list, int n, int base, double *out, int32_t *lv) {

@@ -56,6 +56,11 @@ class DgStats(ctypes.Structure):
     ]
 
 
+class DgCellFields(ctypes.Structure):
+    _fields_ = [("level", ctypes.POINTER(ctypes.c_int)), ("acti", ctypes.POINTER(ctypes.c_int))] + \
+        [(f, ctypes.POINTER(ctypes.c_double)) for f in ("center", "t", "u", "p", "error", "max_dt", "cfl", "k")]
+
+
 KERNEL_KINDS = ("flux", "recv", "update", "slope", "aux", "estimate", "regrid", "reassign", "flush", "init", "gc",
                 "other")
 
@@ -87,6 +92,8 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
                                   ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]
     lib.dg_read_cells_noalloc.argtypes = [vp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_double),
                                           ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]
+    lib.dg_read_fields.argtypes = [vp, ctypes.POINTER(DgCellFields), ctypes.c_longlong,
+                                   ctypes.POINTER(ctypes.c_longlong)]
     lib.dg_read_slopes.argtypes = [vp, ctypes.POINTER(ctypes.c_double), ctypes.c_longlong,
                                    ctypes.POINTER(ctypes.c_longlong)]
     lib.dg_read_gradients.argtypes = lib.dg_read_slopes.argtypes
@@ -133,7 +140,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
 
 
 EXPORTED_SYMBOLS = ("dg_set_device", "dg_create", "dg_set_stream", "dg_step", "dg_step_many", "dg_cell_count",
-                    "dg_read_cells", "dg_read_slopes", "dg_read_gradients", "dg_forecast_features", "dg_set_hold", "dg_set_coarsen_interval",
+                    "dg_read_cells", "dg_read_fields", "dg_read_slopes", "dg_read_gradients", "dg_forecast_features", "dg_set_hold", "dg_set_coarsen_interval",
                     "dg_tree_size", "dg_read_tree",
                     "dg_mlp_last_error", "dg_mlp_create", "dg_mlp_param_count", "dg_mlp_set_params",
                     "dg_mlp_get_params", "dg_mlp_predict", "dg_mlp_loss_grad", "dg_mlp_train", "dg_mlp_destroy",
@@ -227,7 +234,20 @@ class Solver:
         return int(n.value)
 
     def active_cells(self) -> Snapshot:
-        return self._read(self._lib.dg_read_cells)
+        sh = self.shape
+        D, E = sh.dims, sh.E
+        n = self.n_active_cells()
+        lv, acti = np.empty(n, np.int32), np.empty(n, np.int32)
+        center, u, p = np.empty((n, D)), np.empty((n, E)), np.empty((n, E))
+        t, error, max_dt, cfl = (np.empty(n) for _ in range(4))
+        k = np.empty((n, sh.P)) if sh.P > 0 else None
+        it, dbl = ctypes.c_int, ctypes.c_double
+        f = DgCellFields(_ptr(lv, it), _ptr(acti, it), *(_ptr(a, dbl) for a in (center, t, u, p, error, max_dt, cfl)),
+                         _ptr(k, dbl) if k is not None else None)
+        self._check(self._lib.dg_read_fields(self._h, ctypes.byref(f), n, None))
+        st = self.stats()
+        return Snapshot(D, E, int(st.n_global_steps), int(st.n_substeps), int(st.tree_size), int(sum(st.n_clusters)),
+                        self.time, st.global_dt, float(st.cell_updates), lv, acti, center, t, u, p, error, max_dt, cfl, k)
 
     def _read(self, fn) -> Snapshot:
         sh = self.shape

@@ -189,6 +189,14 @@ int dg_cell_count(dg_solver *s, long long *n);
  * multiphase model: mu, unused, interface normal[D], curvature, smoothed volume fraction; 0 otherwise). */
 int dg_read_cells(dg_solver *s, int *levels, double *data, long long max_cells, long long *n_out);
 
+/* The same values in the same order, one array per field (max_cells rows each): what a host that keeps fields
+ * apart reads without taking records apart. k ([n][P], multiphase only) may be null for the other models. */
+typedef struct dg_cell_fields {
+	int *level, *acti;
+	double *center, *t, *u, *p, *error, *max_dt, *cfl, *k;
+} dg_cell_fields;
+int dg_read_fields(dg_solver *s, const dg_cell_fields *fields, long long max_cells, long long *n_out);
+
 /* The limited slopes (Cell::slope, integrator/cell.hpp:19) of the active cells, slopes[n][D][E], in the
  * order of dg_read_cells: what a writer needs to evaluate Cell::get_p(x, t) (cell.hpp:23-31) at points
  * of the cell, as DACTI's VTU writer does at the cell vertices (driver/io/vtu_writer.hpp:40-62). */

@@ -109,3 +109,18 @@ def test_runs_side_by_side():
         want = _run(c, 3)
         o = np.argsort(_keys(got, 1.0))
         assert got.u[o].tobytes() == want[3][4].tobytes() and st.cell_updates == want[2][0]
+
+
+@pytest.mark.parametrize("name", ["tiny", "walls3", "drop2", "drop3_mixed"])
+def test_fields_equal_records(name):
+    """active_cells (field arrays) and the record read-back give the same values, before and after steps."""
+    make, _, form = CASES[name]
+    s = Solver(make())
+    s.set_form(form)
+    for _ in range(2):
+        a, b = s.active_cells(), s.active_cells_noalloc()
+        for f in ("tree_level", "acti_level", "center", "t", "u", "p", "error", "max_dt", "cfl", "k"):
+            x, y = getattr(a, f), getattr(b, f)
+            assert (x is None and y is None) or (x.dtype == y.dtype and x.shape == y.shape and x.tobytes() == y.tobytes())
+        s.integrate()
+    s.close()
