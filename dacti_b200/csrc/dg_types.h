@@ -56,6 +56,9 @@ enum : uint32_t {
 struct ModelConsts {
 	double ns_mu, ns_lambda;
 	double gamma1, gamma2, P1, P2, cp1, cp2, cv1, cv2, mu1, mu2, lambda1, lambda2, sigma;
+	// 1 / (gamma1 - 1) - 1 / (gamma2 - 1), gamma1 P1 / (gamma1 - 1), gamma2 P2 / (gamma2 - 1)
+	double eos[3];
+	float eos_f[4];
 };
 
 struct Consts {

@@ -85,6 +85,26 @@ __device__ __forceinline__ S mix_p0(const ModelConsts &m, S a) {
 	else if (a > 1 - (S) MULTI_EPS) return P1;
 	else return (a * g1 * P1 / (g1 - 1) + (1 - a) * g2 * P2 / (g2 - 1)) / (1 + a / (g1 - 1) + (1 - a) / (g2 - 1));
 }
+// Both closures of one volume fraction, with the divisions they share formed once. A face's star state has the
+// volume fraction of one of its two sides, and a cell's is the same before and after the EOS recovery, so a flux
+// needs two of these and an update one, where each use used to form its own (up to six divisions each inside a
+// smeared interface).
+template<class S>
+struct Mix {
+	S g, p0;
+};
+template<class M, class S = double>
+__device__ __forceinline__ Mix<S> mix_of(const ModelConsts &m, S a) {
+	if constexpr (!M::MULTI) {
+		return {(S) 0, (S) 0};
+	} else {
+		const S g1 = (S) m.gamma1, g2 = (S) m.gamma2, P1 = (S) m.P1, P2 = (S) m.P2;
+		if (a < (S) MULTI_EPS) return {g2, P2};
+		if (a > 1 - (S) MULTI_EPS) return {g1, P1};
+		const S x = a / (g1 - 1), y = (1 - a) / (g2 - 1);
+		return {1 + 1 / (x + y), (a * g1 * P1 / (g1 - 1) + (1 - a) * g2 * P2 / (g2 - 1)) / (1 + x + y)};
+	}
+}
 __device__ __forceinline__ double mix_temperature(const ModelConsts &m, double r0, double r1, double p, double a) {
 	if (a < MULTI_EPS) return (p + m.P2) / ((m.gamma2 - 1) * r1 * m.cv2);
 	else if (a > 1 - MULTI_EPS) return (p + m.P1) / ((m.gamma1 - 1) * r0 * m.cv1);
@@ -97,8 +117,8 @@ __device__ __forceinline__ double mix_temperature(const ModelConsts &m, double r
 // Sound speed, pressure and variable conversions
 // --------------------------------------------------------------------------------------------
 template<class M, class S = double>
-__device__ __forceinline__ S sound_speed_rp(const ModelConsts &m, S r0, S r1, S p, S a) {
-	if constexpr (M::MULTI) return sqrt(mix_gamma<S>(m, a) * (p + mix_p0<S>(m, a)) / (r0 + r1));
+__device__ __forceinline__ S sound_speed_rp(const Mix<S> &x, S r0, S r1, S p) {
+	if constexpr (M::MULTI) return sqrt(x.g * (p + x.p0) / (r0 + r1));
 	else return sqrt((S) EULER_GAMMA * p / r0);
 }
 template<class M>
@@ -124,12 +144,11 @@ __device__ __forceinline__ bool supersonic(const ModelConsts &m, const S *p) {
 }
 
 template<class M>
-__device__ __forceinline__ double pressure(const ModelConsts &m, const double *u) {
+__device__ __forceinline__ double pressure(const Mix<double> &x, const double *u) {
 	double ke = 0;
 	for (int i = 0; i < M::D; ++i) ke += 0.5 * u[M::IU + i] * u[M::IU + i];
 	if constexpr (M::MULTI) {
-		double g = mix_gamma(m, u[M::IA]);
-		return (g - 1) * (u[M::IP] - ke / (u[0] + u[1])) - mix_gamma(m, u[M::IA]) * mix_p0(m, u[M::IA]);
+		return (x.g - 1) * (u[M::IP] - ke / (u[0] + u[1])) - x.g * x.p0;
 	} else {
 		return (EULER_GAMMA - 1) * (u[M::IP] - ke / u[0]);
 	}
@@ -137,23 +156,27 @@ __device__ __forceinline__ double pressure(const ModelConsts &m, const double *u
 
 // primitive_variables (model/euler.hpp:266-274, model/multi.hpp:448-458)
 template<class M>
-__device__ __forceinline__ void prim_from_cons(const ModelConsts &m, const double *u, double *p) {
+__device__ __forceinline__ void prim_from_cons(const Mix<double> &x, const double *u, double *p) {
 	if constexpr (M::MULTI) {
 		p[0] = u[0];
 		p[1] = u[1];
 		for (int i = 0; i < M::D; ++i) p[M::IU + i] = u[M::IU + i] / (u[0] + u[1]);
-		p[M::IP] = pressure<M>(m, u);
+		p[M::IP] = pressure<M>(x, u);
 		p[M::IA] = u[M::IA];
 	} else {
 		p[0] = u[0];
 		for (int i = 0; i < M::D; ++i) p[M::IU + i] = u[M::IU + i] / u[0];
-		p[M::IP] = pressure<M>(m, u);
+		p[M::IP] = pressure<M>(x, u);
 	}
+}
+template<class M>
+__device__ __forceinline__ void prim_from_cons(const ModelConsts &m, const double *u, double *p) {
+	prim_from_cons<M>(mix_of<M>(m, M::MULTI ? u[M::E - 1] : 0.0), u, p);
 }
 
 // conserved_variables (model/euler.hpp:276-286, model/multi.hpp:460-472)
 template<class M>
-__device__ __forceinline__ void cons_from_prim(const ModelConsts &m, const double *p, double *u) {
+__device__ __forceinline__ void cons_from_prim(const Mix<double> &x, const double *p, double *u) {
 	double ke = 0;
 	if constexpr (M::MULTI) {
 		u[0] = p[0];
@@ -162,8 +185,7 @@ __device__ __forceinline__ void cons_from_prim(const ModelConsts &m, const doubl
 			u[M::IU + i] = (p[0] + p[1]) * p[M::IU + i];
 			ke += 0.5 * p[M::IU + i] * p[M::IU + i];
 		}
-		double a = p[M::IA];
-		u[M::IP] = (p[M::IP] + mix_gamma(m, a) * mix_p0(m, a)) / (mix_gamma(m, a) - 1) + (p[0] + p[1]) * ke;
+		u[M::IP] = (p[M::IP] + x.g * x.p0) / (x.g - 1) + (p[0] + p[1]) * ke;
 		u[M::IA] = p[M::IA];
 	} else {
 		u[0] = p[0];
@@ -173,6 +195,11 @@ __device__ __forceinline__ void cons_from_prim(const ModelConsts &m, const doubl
 		}
 		u[M::IP] = p[M::IP] / (EULER_GAMMA - 1) + p[0] * ke;
 	}
+}
+
+template<class M>
+__device__ __forceinline__ void cons_from_prim(const ModelConsts &m, const double *p, double *u) {
+	cons_from_prim<M>(mix_of<M>(m, M::MULTI ? p[M::E - 1] : 0.0), p, u);
 }
 
 // get_grad_input (model/navier_stokes.hpp:377-385, model/multi.hpp:148-156)
@@ -231,7 +258,7 @@ __device__ __forceinline__ double max_delta_time(const ModelConsts &m, const dou
 // semantics: every component not written here is 0.
 // --------------------------------------------------------------------------------------------
 template<class M, class S = double>
-__device__ __forceinline__ void phys_flux(const ModelConsts &m, const S *p, S un, int dim, bool projected, S *F) {
+__device__ __forceinline__ void phys_flux(const Mix<S> &x, const S *p, S un, int dim, bool projected, S *F) {
 	constexpr int D = M::D;
 	S vn         = projected ? un : pick<M::IU, D>(p, dim);
 	S ke         = 0;
@@ -244,8 +271,7 @@ __device__ __forceinline__ void phys_flux(const ModelConsts &m, const S *p, S un
 		F[0] = vn * p[0];
 		F[1] = vn * p[1];
 		put_add<M::IU, D>(F, dim, p[M::IP]);
-		S a      = p[M::IA];
-		F[M::IP] = vn * (mix_gamma<S>(m, a) / (mix_gamma<S>(m, a) - 1) * (p[M::IP] + mix_p0<S>(m, a)) + ke * (p[0] + p[1]));
+		F[M::IP] = vn * (x.g / (x.g - 1) * (p[M::IP] + x.p0) + ke * (p[0] + p[1]));
 		F[M::IA] = vn * p[M::IA];
 		F[M::IA + 1] = vn;
 		put<M::IA + 2, D>(F, dim, p[M::IA]);
@@ -261,16 +287,20 @@ __device__ __forceinline__ void phys_flux(const ModelConsts &m, const S *p, S un
 }
 
 // middle_state (model/euler.hpp:118-153, model/multi.hpp:205-246): the HLLC-type star state in
-// primitive variables; `ka` enters only the multiphase contact speed.
+// primitive variables; `ka` enters only the multiphase contact speed. `xm` is the star state's closure.
 template<class M, class S = double>
-__device__ __forceinline__ void middle_state(const ModelConsts &m, const S *pn, const S *pp, S ka, int dim, S *pm) {
+__device__ __forceinline__ void middle_state(const ModelConsts &m, const S *pn, const S *pp, S ka, int dim, S *pm, Mix<S> &xm) {
 	constexpr int D = M::D;
 	const int ip = M::IP;
 	const S un = pick<M::IU, D>(pn, dim), up = pick<M::IU, D>(pp, dim);
 	S c_n, c_p, rn, rp;
+	Mix<S> xn_{};
 	if constexpr (M::MULTI) {
-		c_n = sound_speed_rp<M, S>(m, pn[0], pn[1], pn[ip], pn[M::IA]);
-		c_p = sound_speed_rp<M, S>(m, pp[0], pp[1], pp[ip], pp[M::IA]);
+		const Mix<S> xn = mix_of<M, S>(m, pn[M::IA]);
+		xm              = mix_of<M, S>(m, pp[M::IA]);
+		c_n = sound_speed_rp<M, S>(xn, pn[0], pn[1], pn[ip]);
+		c_p = sound_speed_rp<M, S>(xm, pp[0], pp[1], pp[ip]);
+		xn_ = xn;
 		rn  = pn[0] + pn[1];
 		rp  = pp[0] + pp[1];
 	} else {
@@ -294,6 +324,7 @@ __device__ __forceinline__ void middle_state(const ModelConsts &m, const S *pn, 
 	for (int q = 0; q < M::E; ++q) pm[q] = 0;
 	if (Sn > 0) {
 		for (int q = 0; q < M::E; ++q) pm[q] = pn[q];
+		xm = xn_;
 	} else if (Sp < 0) {
 		for (int q = 0; q < M::E; ++q) pm[q] = pp[q];
 	} else if (Sm > 0 && Sn < 0) {
@@ -302,6 +333,7 @@ __device__ __forceinline__ void middle_state(const ModelConsts &m, const S *pn, 
 			pm[1]      = pn[1] * (Sn - un) / (Sn - Sm);
 			pm[ip]     = pn[ip] + (pn[0] + pn[1]) * (Sn - un) * (Sm - un);
 			pm[M::IA]  = pn[M::IA];
+			xm         = xn_;
 		} else {
 			pm[0]  = pn[0] * (Sn - un) / (Sn - Sm);
 			pm[ip] = pn[ip] + pn[0] * (Sn - un) * (Sm - un);

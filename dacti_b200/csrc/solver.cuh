@@ -269,6 +269,12 @@ public:
 		m.lambda1 = pr[DG_P_LAMBDA1];
 		m.lambda2 = pr[DG_P_LAMBDA2];
 		m.sigma = pr[DG_P_SIGMA];
+		{
+			const double g1 = m.gamma1, g2 = m.gamma2;
+			m.eos[0] = 1 / (g1 - 1) - 1 / (g2 - 1), m.eos[1] = g1 * m.P1 / (g1 - 1), m.eos[2] = g2 * m.P2 / (g2 - 1);
+			const float f1 = (float) g1, f2 = (float) g2;
+			m.eos_f[0] = 1 / (f1 - 1) - 1 / (f2 - 1), m.eos_f[1] = f1 * (float) m.P1 / (f1 - 1), m.eos_f[2] = f2 * (float) m.P2 / (f2 - 1);
+		}
 		if constexpr (M::MULTI) visc_ = m.mu1 != 0.0 || m.mu2 != 0.0 || m.lambda1 != 0.0 || m.lambda2 != 0.0;
 		else visc_ = M::VISC;
 		sigma_ = m.sigma != 0.0;
@@ -869,10 +875,10 @@ private:
 	// ---- device-resident runs (run.cuh) ---------------------------------------------------------
 
 	// Largest cluster a run takes. Above it a substep's launches fill the GPU, and each of them has the
-	// registers and block size of its own stage, where a run has one for all: drop3d_large of perf/cases.py
-	// steps in 707 to 711 ms with this limit at 4096 to 32768 cells, 721 at 65536 and 925 at 131072, and
-	// drop3d (17 thousand cells a substep) in 243 ms at 4096, 198 at 32768, 289 without runs.
-	static constexpr int RUN_CELLS = 1 << 15;
+	// registers and block size of its own stage, where a run has one for all. Between 32768 and 98304 cells the
+	// two are even (drop3d of perf/cases.py, clusters of 17 thousand cells on average, steps in 137 to 133 ms, the
+	// larger drop3d_large in 664 to 675); at 16384 the runs lose (the cylinder 109 ms against 80).
+	static constexpr int RUN_CELLS = 1 << 16;
 	// Largest cluster for which a run is one thread-block cluster (its barrier is 0.35 us, the grid's 1.3):
 	// up to about here the run of sixteen SMs is as fast as the one of all (drop2d 107 ms against 118,
 	// lax_tiny 23 against 27).

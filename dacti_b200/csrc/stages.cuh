@@ -125,6 +125,13 @@ __device__ __forceinline__ S pick_row_dt(const S *du, int dim) {
 	return r;
 }
 
+// The constants of the interface compression's energy term, in the form's own precision.
+template<class S>
+__device__ __forceinline__ const S *compression_consts(const ModelConsts &m) {
+	if constexpr (sizeof(S) == 8) return m.eos;
+	else return m.eos_f;
+}
+
 // --------------------------------------------------------------------------------------------
 // Interior face flux: Model::flux(left, right, face) with the face of the owning cell
 // (impl/flux.hpp:32-39, 80-91; model/euler.hpp:156-200, navier_stokes.hpp:387-408,
@@ -201,8 +208,9 @@ __device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, Fa
 	S ka = 0;
 	if constexpr (M::MULTI) ka = (S) 0.5 * (kl + kr);
 	S pm[E], F[M::F];
-	middle_state<M, S>(C.m, pn, pp, ka, dim, pm);
-	phys_flux<M, S>(C.m, pm, (S) 0, dim, false, F);
+	Mix<S> xm{};
+	middle_state<M, S>(C.m, pn, pp, ka, dim, pm, xm);
+	phys_flux<M, S>(xm, pm, (S) 0, dim, false, F);
 	const double dtf = t1 - t0;
 
 	if constexpr (M::MULTI) {
@@ -218,10 +226,8 @@ __device__ __forceinline__ void interior_flux(const Pool &P, const Consts &C, Fa
 			}
 			F[0] += uc * (1 - a) * pm[0];
 			F[1] += uc * (-a) * pm[1];
-			const ModelConsts &m = C.m;
-			const S g1 = (S) m.gamma1, g2 = (S) m.gamma2, P1 = (S) m.P1, P2 = (S) m.P2;
-			F[IP] += uc * ((1 - a) * pm[0] - a * pm[1]) * ke +
-			         uc * (1 - a) * a * (pm[IP] * (1 / (g1 - 1) - 1 / (g2 - 1)) + g1 * P1 / (g1 - 1) - g2 * P2 / (g2 - 1));
+			const S *eos = compression_consts<S>(C.m);
+			F[IP] += uc * ((1 - a) * pm[0] - a * pm[1]) * ke + uc * (1 - a) * a * (pm[IP] * eos[0] + eos[1] - eos[2]);
 			F[IA] += uc * (1 - a) * a;
 		}
 	}
@@ -277,14 +283,15 @@ __device__ __forceinline__ void boundary_flux(const Pool &P, const Consts &C, co
 	}
 	const int type = B.type[b];
 	if (type == BC_FREESLIP) {
-		phys_flux<M, S>(C.m, pc, pick<M::IU, D>(pb, dim), dim, true, F);
+		phys_flux<M, S>(mix_of<M, S>(C.m, pc[M::E - 1]), pc, pick<M::IU, D>(pb, dim), dim, true, F);
 	} else if (type == BC_NOSLIP) {
 		for (int q = 0; q < M::F; ++q) F[q] = 0;
 		put<M::IU, D>(F, dim, pb[M::IP]);
 	} else {
 		S pm[E];
-		middle_state<M, S>(C.m, pb, pc, (S) 0, dim, pm);
-		phys_flux<M, S>(C.m, pm, (S) 0, dim, false, F);
+		Mix<S> xm{};
+		middle_state<M, S>(C.m, pb, pc, (S) 0, dim, pm, xm);
+		phys_flux<M, S>(xm, pm, (S) 0, dim, false, F);
 	}
 	if constexpr (M::VISC && V) {
 		constexpr int G = M::G;
@@ -838,7 +845,8 @@ __device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Con
 				s[M::IA] = -pold[M::IA] * du[M::IA + 1];
 				for (int q = 0; q < E; ++q) u[q] = u[q] + s[q];
 			}
-			prim_from_cons<M>(C.m, u, p);
+			const Mix<double> x = mix_of<M>(C.m, M::MULTI ? u[M::E - 1] : 0.0);
+			prim_from_cons<M>(x, u, p);
 			if (isnan(p[M::IP]) || isnan(p[0])) set_status(&cnt->status, ST_NAN);
 			if constexpr (M::MULTI) {
 				p[0] = smax(p[0], 1e-3);
@@ -847,7 +855,7 @@ __device__ __forceinline__ void d_update(const Grid &g, const Pool &P, const Con
 				p[0] = smax(p[0], 1e-3);
 			}
 			p[M::IP] = smax(p[M::IP], 1e-3);
-			cons_from_prim<M>(C.m, p, u);
+			cons_from_prim<M>(x, p, u);
 			if constexpr (M::G > 0 && V) {
 				double gnew[M::G];
 				grad_input<M>(C.m, p, gnew);
