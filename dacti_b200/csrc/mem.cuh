@@ -108,6 +108,14 @@ public:
 	}
 };
 
+// Held by the one launch that takes every SM of the current device and whose blocks wait for one another.
+inline std::mutex &whole_gpu() {
+	static std::mutex m[64];
+	int dev = 0;
+	cudaGetDevice(&dev);
+	return m[dev >= 0 && dev < 64 ? dev : 0];
+}
+
 // A pinned host block of PINNED_BYTES; up to PINNED_KEEP of them wait for the next solver, since pinning a page
 // costs as much as building a small one.
 constexpr size_t PINNED_BYTES = 2048;

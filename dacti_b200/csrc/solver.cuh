@@ -1073,11 +1073,10 @@ public:
 		// Runs on the device serve the default stage choices; the host issues a substep's stages one by one
 		// where a callback or the timing of every stage asks for it, and for clusters that fill the GPU.
 		if (!fn && !prof_ && opts_ == DG_OPT_DEFAULT) {
-			// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU
-			static std::mutex whole_gpu;
 			while (!p.done && !p.broke) {
 				const bool clustered = peers >= RUN_PEERS || most_cells(RUN_CELLS) <= RUN_CLUSTER_CELLS;
-				std::unique_lock<std::mutex> hold(whole_gpu, std::defer_lock);
+				// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU
+				std::unique_lock<std::mutex> hold(whole_gpu(), std::defer_lock);
 				if (!clustered) hold.lock();
 				if (advance(p, RUN_CELLS, clustered)) settle(p);
 			}

@@ -3,7 +3,7 @@
 A substep callback makes the host issue every stage of every substep itself; without one the same step
 runs on the device. Both use the same arithmetic, so cells, time levels, state and counters are equal bit
 for bit. The cases cover a cluster of a few cells, the edges of the sizes that choose a run's shape (one
-thread-block cluster up to 2048 cells, the whole GPU above, the launches above 32768), clusters that
+thread-block cluster up to 2048 cells, the whole GPU above, the launches above 65536), clusters that
 outgrow the scratch, runs that stop for a pool without room, surface tension, both forms, and a NaN.
 """
 import dataclasses
@@ -31,7 +31,7 @@ CASES = {
     "drop2": (lambda: cases.shock_drop(2, 4, 3), 2, "fp64"),
     "drop2_terms": (lambda: cases.shock_drop(2, 4, 2, mu=(1e-3, 1.8e-5), conductivity=(0.6, 0.026)), 2, "mixed"),
     "drop3_mixed": (lambda: cases.shock_drop(3, 4, 2), 2, "mixed"),
-    "above_runs": (lambda: cases.shock_drop(3, 5, 3), 1, "fp64"),  # clusters on both sides of 32768 cells
+    "above_runs": (lambda: cases.shock_drop(3, 5, 3), 3, "fp64"),  # clusters of up to 127 thousand cells
 }
 
 
