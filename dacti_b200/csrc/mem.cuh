@@ -16,7 +16,7 @@ namespace dg {
 
 struct DeviceMemory {
 	static constexpr size_t KEEP      = size_t(4) << 30;
-	static constexpr size_t KEEP_IDLE = size_t(4) << 30;
+	static constexpr size_t KEEP_IDLE = size_t(512) << 20;
 
 	cudaMemPool_t pool  = nullptr;
 	cudaStream_t stream = nullptr;  // of frees whose last use the host has waited for
@@ -65,7 +65,14 @@ struct DeviceMemory {
 inline cudaError_t mem_alloc(void **p, size_t bytes, cudaStream_t st) {
 	cudaError_t e;
 	DeviceMemory *d = DeviceMemory::of_device(e);
-	return d ? cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st) : e;
+	if (!d) return e;
+	e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st);
+	if (e != cudaErrorMemoryAllocation) return e;
+	// blocks freed before, of other sizes, may hold the room: give them back and ask once more
+	cudaGetLastError();
+	if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+	cudaMemPoolTrimTo(d->pool, 0);
+	return cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st);
 }
 // Gives memory back once the work queued on `st` so far is done with it.
 inline void mem_free(void *p, cudaStream_t st) {
