@@ -83,21 +83,25 @@ __global__ void k_predict(const __nv_bfloat16 *wb, Layout L, const float *x, lon
 // A block of 256 threads takes 32 samples through the network and back with all operands in shared memory:
 // in the forward pass and in the backward pass through the layers a lane is a sample and a warp has eight
 // of the 64 units; the weight gradients are 32-term products of activations and deltas, 4 x 4 of the second
-// layer's per thread, summed per tile and then over tiles in registers. What bounds it is the latency of
-// that chain, about 4 us a tile; the form before this (a sample per thread, one warp reduction and one
-// shared-memory atomic for each of 5185 weights per warp) took 730 us a tile of 128 samples.
+// layer's per thread. What bounds it is the latency of that chain.
+//
+// Every value is rounded as one thread per sample and one warp reduction per weight would round it: products
+// before they are added (a unit within rounding of zero is on or off by that), units in ascending order, the 32
+// samples of a tile in the pairs of a butterfly, four tiles to a block sum. A gradient's sign decides a
+// step of Adam, so another rounding is another network.
 
 constexpr int GT   = 256;  // threads
 constexpr int TS   = 32;   // samples of a tile
+constexpr int TB   = 4;    // tiles of a block sum
 constexpr int ROW  = 68;   // row stride of [sample][unit] arrays: 16-byte rows that start in different banks
 constexpr int XMAX = TS * MAX_IN / GT;  // inputs of a tile per thread
-static_assert(H == 64 && GT == 256 && TS == 32, "the thread mapping below is for these sizes");
+static_assert(H == 64 && GT == 256 && TS == 32 && TB * TS == TPB, "the thread mapping below is for these sizes");
 
 struct TileMem {
-	float *W, *G, *X, *A1, *A2, *D1, *D2, *A1T, *D2T, *part, *dz, *y;
+	float *W, *G, *X, *A1, *A2, *D1, *D2, *A1T, *D2T, *dz, *y;
 	static __host__ __device__ int pad(long long n) { return (int) ((n + 3) / 4 * 4); }
 	static __host__ __device__ size_t floats(const Layout &L) {
-		return 2 * (size_t) pad(L.n) + 2 * pad((long long) TS * L.nin) + 4 * TS * ROW + 2 * H * TS + 8 * TS + TS + 2 * TS;
+		return 3 * (size_t) pad(L.n) + 2 * pad((long long) TS * L.nin) + 4 * TS * ROW + 2 * H * TS + TS + 2 * TS;
 	}
 	__device__ TileMem(float *m, const Layout &L) {
 		auto take = [&](size_t n) {
@@ -105,9 +109,9 @@ struct TileMem {
 			m += n;
 			return r;
 		};
-		W = take(pad(L.n)), G = take(pad(L.n)), X = take(2 * pad((long long) TS * L.nin));
+		W = take(pad(L.n)), G = take(2 * pad(L.n)), X = take(2 * pad((long long) TS * L.nin));
 		A1 = take(TS * ROW), A2 = take(TS * ROW), D1 = take(TS * ROW), D2 = take(TS * ROW);
-		A1T = take(H * TS), D2T = take(H * TS), part = take(8 * TS), dz = take(TS), y = take(2 * TS);
+		A1T = take(H * TS), D2T = take(H * TS), dz = take(TS), y = take(2 * TS);
 	}
 };
 
@@ -167,10 +171,25 @@ __device__ __forceinline__ void store_tile(const Layout &L, float *X, float *y, 
 	if (threadIdx.x < TS) y[threadIdx.x] = yr;
 }
 
-// Adds a tile's gradient to `g` and its loss to `loss` (the lanes of the first warp). X and y of the tile are
-// in shared memory (stored before a barrier); `live` samples count.
+// The sums over a tile's samples of N values each, v(sample, out): node HALF of the butterfly that pairs the samples
+// 16 apart, then 8, 4, 2 and 1.
+template<int N, int HALF, class V>
+__device__ __forceinline__ void sum_samples(int q, const V &v, float (&out)[N]) {
+	if constexpr (HALF == TS) {
+		v(q, out);
+	} else {
+		float b[N];
+		sum_samples<N, 2 * HALF>(q, v, out);
+		sum_samples<N, 2 * HALF>(q + HALF, v, b);
+#pragma unroll
+		for (int k = 0; k < N; ++k) out[k] += b[k];
+	}
+}
+
+// Adds a tile's gradient to `g` and its loss to `loss_sum`. X and y of the tile are in shared memory (stored before a
+// barrier); `live` samples count.
 __device__ __forceinline__ void tile_grad(const TileMem &m, const Layout &L, const float *X, const float *y, int live, float pw,
-                                          GradShare &g, double &loss) {
+                                          GradShare &g, double *loss_sum) {
 	const int t = threadIdx.x, lane = t & 31, u0 = 8 * (t >> 5);
 	float a1[8], a2[8];
 #pragma unroll
@@ -178,7 +197,7 @@ __device__ __forceinline__ void tile_grad(const TileMem &m, const Layout &L, con
 	for (int i = 0; i < L.nin; ++i) {
 		const float v = X[lane * L.nin + i];
 #pragma unroll
-		for (int c = 0; c < 8; ++c) a1[c] = fmaf(m.W[L.w1 + (u0 + c) * L.nin + i], v, a1[c]);
+		for (int c = 0; c < 8; ++c) a1[c] += m.W[L.w1 + (u0 + c) * L.nin + i] * v;
 	}
 #pragma unroll
 	for (int c = 0; c < 8; ++c) {
@@ -198,28 +217,35 @@ __device__ __forceinline__ void tile_grad(const TileMem &m, const Layout &L, con
 #pragma unroll
 		for (int c = 0; c < 8; ++c) {
 			const float4 w = *(const float4 *) (m.W + L.w2 + (u0 + c) * H + j);
-			a2[c]          = fmaf(w.w, v[3], fmaf(w.z, v[2], fmaf(w.y, v[1], fmaf(w.x, v[0], a2[c]))));
+			a2[c] += w.x * v[0];
+			a2[c] += w.y * v[1];
+			a2[c] += w.z * v[2];
+			a2[c] += w.w * v[3];
 		}
 	}
-	float z = 0.f;
 #pragma unroll
-	for (int c = 0; c < 8; ++c) {
-		a2[c] = fmaxf(a2[c], 0.f);
-		z     = fmaf(m.W[L.w3 + u0 + c], a2[c], z);
-	}
+	for (int c = 0; c < 8; ++c) a2[c] = fmaxf(a2[c], 0.f);
 #pragma unroll
 	for (int c = 0; c < 8; c += 4) *(float4 *) (m.A2 + lane * ROW + u0 + c) = make_float4(a2[c], a2[c + 1], a2[c + 2], a2[c + 3]);
-	m.part[u0 / 8 * TS + lane] = z;
 	__syncthreads();
-	z = m.W[L.b3];
-#pragma unroll
-	for (int w = 0; w < 8; ++w) z += m.part[w * TS + lane];
+	// the logit, on every warp alike: a sum in the units' order
+	float z = m.W[L.b3];
+#pragma unroll 4
+	for (int k = 0; k < H; k += 4) {
+		const float4 a = *(const float4 *) (m.A2 + lane * ROW + k), w = *(const float4 *) (m.W + L.w3 + k);
+		z += w.x * a.x;
+		z += w.y * a.y;
+		z += w.z * a.z;
+		z += w.w * a.w;
+	}
 	const float yt = y[lane];
 	float dz       = sigmoidf(z) * (pw * yt + 1.f - yt) - pw * yt;
 	if (lane >= live) dz = 0.f;
 	if (t < TS) {
-		if (lane < live) loss += (double) (pw * yt * softplus(-z) + (1.f - yt) * softplus(z));
 		m.dz[lane] = dz;
+		double l   = lane < live ? (double) (pw * yt * softplus(-z) + (1.f - yt) * softplus(z)) : 0.0;
+		for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+		if (t == 0) atomicAdd(loss_sum, l);
 	}
 	float d[8];
 #pragma unroll
@@ -236,54 +262,48 @@ __device__ __forceinline__ void tile_grad(const TileMem &m, const Layout &L, con
 	for (int k = 0; k < H; ++k) {
 		const float v   = m.D2T[k * TS + lane];
 		const float4 wa = *(const float4 *) (m.W + L.w2 + k * H + u0), wb = *(const float4 *) (m.W + L.w2 + k * H + u0 + 4);
-		d[0] = fmaf(wa.x, v, d[0]), d[1] = fmaf(wa.y, v, d[1]), d[2] = fmaf(wa.z, v, d[2]), d[3] = fmaf(wa.w, v, d[3]);
-		d[4] = fmaf(wb.x, v, d[4]), d[5] = fmaf(wb.y, v, d[5]), d[6] = fmaf(wb.z, v, d[6]), d[7] = fmaf(wb.w, v, d[7]);
+		d[0] += wa.x * v, d[1] += wa.y * v, d[2] += wa.z * v, d[3] += wa.w * v;
+		d[4] += wb.x * v, d[5] += wb.y * v, d[6] += wb.z * v, d[7] += wb.w * v;
 	}
 #pragma unroll
 	for (int c = 0; c < 8; ++c) d[c] = a1[c] > 0.f ? d[c] : 0.f;
 #pragma unroll
 	for (int c = 0; c < 8; c += 4) *(float4 *) (m.D1 + lane * ROW + u0 + c) = make_float4(d[c], d[c + 1], d[c + 2], d[c + 3]);
-	float s2[16];
-#pragma unroll
-	for (float &v: s2) v = 0.f;
 	const int k0 = 4 * (t >> 4), j0 = 4 * (t & 15);
-#pragma unroll 4
-	for (int q = 0; q < TS; ++q) {
+	float s2[16];
+	sum_samples<16, 1>(0, [&](int q, float (&o)[16]) {
 		const float4 dk = *(const float4 *) (m.D2 + q * ROW + k0), aj = *(const float4 *) (m.A1 + q * ROW + j0);
 		const float dv[4] = {dk.x, dk.y, dk.z, dk.w}, av[4] = {aj.x, aj.y, aj.z, aj.w};
 #pragma unroll
 		for (int a = 0; a < 4; ++a)
 #pragma unroll
-			for (int b = 0; b < 4; ++b) s2[4 * a + b] = fmaf(dv[a], av[b], s2[4 * a + b]);
-	}
+			for (int b = 0; b < 4; ++b) o[4 * a + b] = dv[a] * av[b];
+	}, s2);
 #pragma unroll
 	for (int q = 0; q < 16; ++q) g.w2[q] += s2[q];
-	float one = 0.f;
+	float one[1] = {0.f};
 	if (t < 64) {
-		for (int q = 0; q < TS; ++q) one += m.D2[q * ROW + t];
+		sum_samples<1, 1>(0, [&](int q, float (&o)[1]) { o[0] = m.D2[q * ROW + t]; }, one);
 	} else if (t < 128) {
-		for (int q = 0; q < TS; ++q) one = fmaf(m.dz[q], m.A2[q * ROW + t - 64], one);
+		sum_samples<1, 1>(0, [&](int q, float (&o)[1]) { o[0] = m.dz[q] * m.A2[q * ROW + t - 64]; }, one);
 	} else if (t == 192) {
-		for (int q = 0; q < TS; ++q) one += m.dz[q];
+		sum_samples<1, 1>(0, [&](int q, float (&o)[1]) { o[0] = m.dz[q]; }, one);
 	}
 	__syncthreads();
 	float s1[MAX_IN / 4];
-#pragma unroll
-	for (float &v: s1) v = 0.f;
-	for (int q = 0; q < TS; ++q) {
+	sum_samples<MAX_IN / 4, 1>(0, [&](int q, float (&o)[MAX_IN / 4]) {
 		const float v = m.D1[q * ROW + (t >> 2)];
 #pragma unroll
-		for (int c = 0; c < MAX_IN / 4; ++c)
-			if ((t & 3) + 4 * c < L.nin) s1[c] = fmaf(v, X[q * L.nin + (t & 3) + 4 * c], s1[c]);
-	}
+		for (int c = 0; c < MAX_IN / 4; ++c) o[c] = (t & 3) + 4 * c < L.nin ? v * X[q * L.nin + (t & 3) + 4 * c] : 0.f;
+	}, s1);
 #pragma unroll
 	for (int c = 0; c < MAX_IN / 4; ++c) g.w1[c] += s1[c];
-	if (t >= 128 && t < 192)
-		for (int q = 0; q < TS; ++q) one += m.D1[q * ROW + t - 128];
-	g.one += one;
+	if (t >= 128 && t < 192) sum_samples<1, 1>(0, [&](int q, float (&o)[1]) { o[0] = m.D1[q * ROW + t - 128]; }, one);
+	g.one += one[0];
 }
 
-// Sums of the loss and of its gradient over all n samples into loss_sum / grad.
+// Sums of the loss and of its gradient over all n samples into loss_sum / grad. A block sums the tiles of TPB samples
+// in their order, the blocks add to the gradient as they end.
 __global__ void __launch_bounds__(GT) k_grad(const float *w, Layout L, const float *x, const float *y, long long n, float pw,
                                              float *grad, double *loss_sum) {
 	extern __shared__ __align__(16) float sm[];
@@ -291,34 +311,33 @@ __global__ void __launch_bounds__(GT) k_grad(const float *w, Layout L, const flo
 	for (int p = threadIdx.x; p < L.n; p += GT) m.W[p] = w[p];
 	GradShare g;
 	g.zero();
-	double loss           = 0.0;
-	const long long tiles = (n + TS - 1) / TS;
-	for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-		float xr[XMAX], yr;
-		fetch_tile(L, x, y, nullptr, tile * TS, n, xr, yr);
-		__syncthreads();  // the previous tile's readers are done
-		store_tile(L, m.X, m.y, xr, yr);
-		__syncthreads();
-		tile_grad(m, L, m.X, m.y, (int) min((long long) TS, n - tile * TS), pw, g, loss);
+	for (long long base = (long long) blockIdx.x * TPB; base < n; base += (long long) gridDim.x * TPB) {
+		for (long long first = base; first < min(n, base + TPB); first += TS) {
+			float xr[XMAX], yr;
+			fetch_tile(L, x, y, nullptr, first, n, xr, yr);
+			__syncthreads();  // the previous tile's readers are done
+			store_tile(L, m.X, m.y, xr, yr);
+			__syncthreads();
+			tile_grad(m, L, m.X, m.y, (int) min((long long) TS, n - first), pw, g, loss_sum);
+		}
 	}
 	g.each(L, [&](long long p, float v) { atomicAdd(grad + p, v); });
-	if (threadIdx.x < 32) {
-		for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-		if (threadIdx.x == 0) atomicAdd(loss_sum, loss);
-	}
 }
 
-// One epoch of Adam in one launch of one thread-block cluster. The minibatch's tiles go round the blocks; each
-// block leaves its gradient in its shared memory, sums its share of the parameters over the cluster's blocks in
-// their order, steps those parameters (moments and weights stay in registers for the whole epoch) and writes
-// them into every block's copy of the weights. Two cluster barriers a step take the place of two launches and a
-// pass over the gradient in global memory: 24 steps of 512 samples took 18 ms and take 0.5 ms.
-// bc[step] holds Adam's bias corrections.
+// One epoch of Adam in one launch of one thread-block cluster. A round takes a tile of the minibatch on each block; the
+// blocks leave their gradients in shared memory, and each block sums its share of the parameters over the cluster,
+// four tiles to a block sum. After a minibatch's rounds it steps those parameters (moments and weights
+// stay in registers for the whole epoch) and writes them into every block's copy of the weights. A cluster barrier a round
+// and one a step take the place of two launches and a pass over the gradient in global memory. The gradients have two
+// buffers: a block writes one while others may still read the other. A call of 24 steps of 512 samples takes 0.52 ms
+// (18.0 with two launches a step and a reduction and an atomic per weight and warp). bc[step] holds Adam's bias
+// corrections.
 __global__ void __launch_bounds__(GT) k_epoch(float *w, __nv_bfloat16 *wb, float *mom, float *var, Layout L, const float *x,
                                               const float *y, const int *perm, long long n, long long batch, float pw, float lr,
                                               const float2 *bc, double *loss_sum) {
 	constexpr float B1 = 0.9f, B2 = 0.999f, EPS = 1e-8f;
-	constexpr int MINE = 4;  // parameters of a thread, at least the largest network's over eight blocks
+	constexpr int MINE = 4;         // parameters of a thread, at least the largest network's over eight blocks
+	constexpr int MOST_BLOCKS = 16;
 	extern __shared__ __align__(16) float sm[];
 	const TileMem m(sm, L);
 	cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -335,9 +354,8 @@ __global__ void __launch_bounds__(GT) k_epoch(float *w, __nv_bfloat16 *wb, float
 		pm[c]  = at[c] < 0 ? 0.f : mom[at[c]];
 		pv[c]  = at[c] < 0 ? 0.f : var[at[c]];
 	}
-	double loss  = 0.0;
-	const int xn = TileMem::pad((long long) TS * L.nin);
-	int buf      = 0;
+	const int xn = TileMem::pad((long long) TS * L.nin), gn = TileMem::pad(L.n);
+	int buf = 0, gbuf = 0;
 	float xr[XMAX], yr;
 	// the tile of this block that follows tile `tile` of the minibatch at `first`
 	auto next = [&](long long &first, long long &tile) {
@@ -357,27 +375,44 @@ __global__ void __launch_bounds__(GT) k_epoch(float *w, __nv_bfloat16 *wb, float
 	__syncthreads();
 	int step = 0;
 	for (long long first = 0; first < n; first += batch, ++step) {
-		const long long cnt = min(batch, n - first);
-		GradShare g;
-		g.zero();
-		for (long long tile = rank; tile * TS < cnt; tile += blocks) {
-			more = next(nf, nt);
-			if (more) fetch_tile(L, x, y, perm, nf + nt * TS, nf + min(batch, n - nf), xr, yr);
-			tile_grad(m, L, m.X + buf * xn, m.y + buf * TS, (int) min((long long) TS, cnt - tile * TS), pw, g, loss);
-			buf ^= 1;
-			if (more) store_tile(L, m.X + buf * xn, m.y + buf * TS, xr, yr);
-			__syncthreads();
+		const long long cnt = min(batch, n - first), tiles = (cnt + TS - 1) / TS;
+		float sum[MINE];
+#pragma unroll
+		for (float &v: sum) v = 0.f;
+		for (long long t0 = 0; t0 < tiles; t0 += blocks, gbuf ^= 1) {
+			const long long tile = t0 + rank;
+			float *G             = m.G + gbuf * gn;
+			if (tile < tiles) {
+				GradShare g;
+				g.zero();
+				more = next(nf, nt);
+				if (more) fetch_tile(L, x, y, perm, nf + nt * TS, nf + min(batch, n - nf), xr, yr);
+				tile_grad(m, L, m.X + buf * xn, m.y + buf * TS, (int) min((long long) TS, cnt - tile * TS), pw, g, loss_sum);
+				buf ^= 1;
+				if (more) store_tile(L, m.X + buf * xn, m.y + buf * TS, xr, yr);
+				g.each(L, [&](long long p, float v) { G[p] = v; });
+			}
+			cl.sync();
+			const int live = (int) min((long long) blocks, tiles - t0);
+#pragma unroll
+			for (int c = 0; c < MINE; ++c) {
+				if (at[c] < 0) continue;
+#pragma unroll
+				for (int r0 = 0; r0 < MOST_BLOCKS; r0 += TB) {
+					if (r0 >= live) break;
+					float s = 0.f;
+#pragma unroll
+					for (int r = r0; r < r0 + TB; ++r) s += r < live ? cl.map_shared_rank(G, r)[at[c]] : 0.f;
+					sum[c] += s;
+				}
+			}
 		}
-		g.each(L, [&](long long p, float v) { m.G[p] = v; });
-		cl.sync();
 		const float2 c2   = bc[step];
 		const float scale = 1.f / (float) cnt;
 #pragma unroll
 		for (int c = 0; c < MINE; ++c) {
 			if (at[c] < 0) continue;
-			float s = 0.f;
-			for (int r = 0; r < blocks; ++r) s += cl.map_shared_rank(m.G, r)[at[c]];
-			const float gr = s * scale;
+			const float gr = sum[c] * scale;
 			pm[c]          = B1 * pm[c] + (1.f - B1) * gr;
 			pv[c]          = B2 * pv[c] + (1.f - B2) * gr * gr;
 			pw_[c] -= lr * (pm[c] / c2.x) / (sqrtf(pv[c] / c2.y) + EPS);
@@ -393,10 +428,6 @@ __global__ void __launch_bounds__(GT) k_epoch(float *w, __nv_bfloat16 *wb, float
 			var[at[c]] = pv[c];
 			wb[at[c]]  = __float2bfloat16(pw_[c]);
 		}
-	if (threadIdx.x < 32) {
-		for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-		if (threadIdx.x == 0) atomicAdd(loss_sum, loss);
-	}
 }
 
 __global__ void k_to_bf16(const float *w, __nv_bfloat16 *wb, long long n) {
@@ -578,9 +609,8 @@ int dg_mlp_loss_grad(dg_mlp *h, const float *x, const float *y, long long n, flo
 	MLP_CUDA(cudaMemcpyAsync(dy.p, y, sizeof(float) * n, cudaMemcpyHostToDevice, h->st));
 	MLP_CUDA(cudaMemsetAsync(h->g, 0, sizeof(float) * h->L.n, h->st));
 	MLP_CUDA(cudaMemsetAsync(h->loss, 0, sizeof(double), h->st));
-	const int blocks = (int) std::min<long long>((n + TS - 1) / TS, 148 * 2);
-	k_grad<<<blocks, GT, smem_grad(h->L), h->st>>>(h->w, h->L, (const float *) dx.p, (const float *) dy.p, n, pos_weight, h->g,
-	                                               h->loss);
+	k_grad<<<grid_of(n), GT, smem_grad(h->L), h->st>>>(h->w, h->L, (const float *) dx.p, (const float *) dy.p, n, pos_weight, h->g,
+	                                                   h->loss);
 	MLP_CUDA(cudaGetLastError());
 	MLP_CUDA(cudaMemcpyAsync(grad, h->g, sizeof(float) * h->L.n, cudaMemcpyDeviceToHost, h->st));
 	MLP_CUDA(cudaMemcpyAsync(loss, h->loss, sizeof(double), cudaMemcpyDeviceToHost, h->st));
