@@ -213,7 +213,7 @@ static __global__ void __launch_bounds__(256) kb_split_check(const TreeArgs *A, 
 template<class M, bool V, class R>
 __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS) kb_face_sum(DG_BATCH_PARAMS) {
 	DG_BATCH_PROLOGUE
-	d_face_sum<M, V, R>(g, a.P, cst, a.B, a.Ls.clu[s.L], s.n, s.L, s.dtL, s.stamp, a.Ls.recv, a.Ls.fresh, a.cnt);
+	d_face_sum<M, V, R>(g, a.P, cst, a.B, a.Ls.clu[s.L], s.n, s.L, s.dtL, s.stamp, a.Ls.recv, a.Ls.fresh, a.cnt, &a.cnt->status);
 }
 
 template<class M, class R>

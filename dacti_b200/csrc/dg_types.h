@@ -138,6 +138,7 @@ struct Counters {
 	int n_new;        // new cluster members (children + coarsened parents)
 	int n_tmp;        // rebuilt cluster list
 	uint32_t status;
+	uint32_t face_status;  // a run's face sums set it, for `status` (run.cuh)
 	int blocks_done;  // blocks of the running launch that have finished (0 between launches)
 	int coarsest;     // the lowest tree level any active leaf has had
 	// running totals that the batched step keeps on the device (splits, coarsenings, cluster cells after

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 	}
 	if (lead && blockIdx.x == 0) {
 		cnt->n_recv = cnt->n_defer = cnt->n_split = cnt->n_unsplit = cnt->n_new = cnt->n_tmp = 0;
-		cnt->status = 0;
+		cnt->status = cnt->face_status = 0;
 	}
 	// every block has read the counters before any changes them
 	if (!run_barrier(a, arrivals, &s_ok)) return;
@@ -228,9 +228,12 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) k_run(const __grid_constant__ 
 		const int e_upd     = epoch0 + 1;
 
 		// the list of new cells, not in use before the regrid, holds the deferred cells' positions
-		d_face_sum<M, V, S>(g, P, C, a.B, list, n, L, dtL, stamp, s_ls.recv, s_ls.fresh, cnt);
+		// `status` decides at a substep's end whether the run stops, and a block that is ahead may be here before the
+		// others have read it: the face sums have a word of their own
+		d_face_sum<M, V, S>(g, P, C, a.B, list, n, L, dtL, stamp, s_ls.recv, s_ls.fresh, cnt, &cnt->face_status);
 		d_stamp(r, P, list, n, e_upd, cnt);
 		if (!run_barrier(a, arrivals, &s_ok)) return;
+		if (lead && blockIdx.x == 0) atomicOr(&cnt->status, __ldcg(&cnt->face_status));
 		// the receivers are cells of slower clusters, the updated cells those of this one
 		const bool deferred = __ldcg(&cnt->n_defer) > 0;
 		if (deferred) d_deferred<M, S>(g, P, list, s_ls.fresh, &cnt->n_defer, L, cnt);

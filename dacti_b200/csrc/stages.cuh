@@ -437,7 +437,7 @@ __device__ __forceinline__ double pair_terms(const double *f) {
 // their slots, instead of evaluating up to 2^(D-1) fluxes again in one lane while the warp waits.
 // In the mixed form every flux is rounded to FP32 once, as both sides read it; sums stay FP64.
 template<class M, bool V, class S = double, class Grid>
-__device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, int L, double dtL, int stamp, int32_t *recv, int32_t *defer, Counters *cnt) {
+__device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const Consts &C, const BcTable &B, const int32_t *list, int n, int L, double dtL, int stamp, int32_t *recv, int32_t *defer, Counters *cnt, uint32_t *status) {
 	constexpr int NF = 2 * M::D, G = NF, GW = 32 / G, F = M::F;
 	constexpr bool EARLY = Grid::EARLY && !M::MULTI;  // the five-equation states do not fit the registers that long
 	const int cap    = P.cap;
@@ -461,7 +461,7 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 			if (nb == 0) {
 				const int b = P.bc[(size_t) f * cap + i];
 				if (b < 0) {
-					set_status(&cnt->status, ST_MISSING_BC);
+					set_status(status, ST_MISSING_BC);
 				} else {
 					double Fb[F];
 					boundary_flux<M, V, S>(P, C, B, i, b, dim, dir, dtL, Fb);
@@ -502,7 +502,7 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 #pragma unroll
 						for (int q = 0; q < F; ++q) dst[q] = (S) Fi[q];
 						if (P.clu[nb] != L && atomicExch(&P.stamp[nb], stamp) != stamp)
-							append(recv, &cnt->n_recv, nb, cap, &cnt->status);
+							append(recv, &cnt->n_recv, nb, cap, status);
 					}
 #pragma unroll
 					for (int q = 0; q < F; ++q) {
@@ -525,7 +525,7 @@ __device__ __forceinline__ void d_face_sum(const Grid &g, const Pool &P, const C
 			}
 			if (sub == 0) {
 				P.dmask[slot] = (int) (((lo >> base) & gm) | (((hi >> base) & gm) << 8));
-				append(defer, &cnt->n_defer, slot, cap, &cnt->status);
+				append(defer, &cnt->n_defer, slot, cap, status);
 			}
 		}
 		// the group's face terms in the fixed pairing order, on every lane of the group
@@ -609,7 +609,7 @@ __device__ __forceinline__ void d_deferred(const Grid &g, const Pool &P, const i
 template<class M, bool V, class S = double>
 __global__ void __launch_bounds__(FACE_THREADS, FACE_MIN_BLOCKS) k_face_sum(Pool P, Consts C, BcTable B, const int32_t *list, int n, int L,
                                                     double dtL, int stamp, int32_t *recv, int32_t *defer, Counters *cnt) {
-	d_face_sum<M, V, S>(PlainGrid{}, P, C, B, list, n, L, dtL, stamp, recv, defer, cnt);
+	d_face_sum<M, V, S>(PlainGrid{}, P, C, B, list, n, L, dtL, stamp, recv, defer, cnt, &cnt->status);
 }
 
 // Stamps the ancestors of the cells that the substep updates, for the subtree means that the stages after the
