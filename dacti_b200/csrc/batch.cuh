@@ -35,6 +35,7 @@
 #include <algorithm>
 #include <climits>
 #include <deque>
+#include <exception>
 
 #include "solver.cuh"
 
@@ -913,6 +914,18 @@ private:
 			stops_ += p[t].stops;
 			completed_ += p[t].by_host;
 		};
+		// A tree's error ends that tree's step only: the others' runs are in flight, and a solver's lists and schedule are
+		// current when its run has been settled. The first error is the batch's once every tree is through.
+		std::exception_ptr failed;
+		auto go_on = [&](int t, auto &&up_to) {
+			try {
+				up_to();
+				if (s_[t]->advance(p[t], SIDE_CELLS, true)) running.push_back(t);
+				else close(t);
+			} catch (...) {
+				if (!failed) failed = std::current_exception();
+			}
+		};
 		for (int k = 0; k < N; ++k) {
 			const int t    = order[k];
 			Solver<M> *s   = s_[t];
@@ -920,23 +933,21 @@ private:
 			before[t]      = {s->n_split_total_, s->n_unsplit_total_, s->updates_, s->n_substeps_};
 			force_break[t] = 0;
 			global_dt[t]   = s->global_dt_;
-			s->begin_step(signal);
-			// a fifth of the tree free as a step starts, else room for half the tree again, so that few runs stop
-			// for a pool without room
-			const long long top = s->h_cnt_->top;
-			if (pregrow_ && top + top / 5 + 16 * NC > s->P_.cap) {
-				const long long want = s->growth_target(s->P_.cap, std::max(top + top / 2 + 16 * NC, s->grown(top)));
-				if (want > s->P_.cap) s->grow_pool((int) std::min<long long>(want, 2000000000LL));
-			}
-			if (s->advance(p[t], SIDE_CELLS, true)) running.push_back(t);
-			else close(t);
+			go_on(t, [&] {
+				s->begin_step(signal);
+				// a fifth of the tree free as a step starts, else room for half the tree again, so that few runs stop
+				// for a pool without room
+				const long long top = s->h_cnt_->top;
+				if (pregrow_ && top + top / 5 + 16 * NC > s->P_.cap) {
+					const long long want = s->growth_target(s->P_.cap, std::max(top + top / 2 + 16 * NC, s->grown(top)));
+					if (want > s->P_.cap) s->grow_pool((int) std::min<long long>(want, 2000000000LL));
+				}
+			});
 		}
 		while (!running.empty()) {
 			const int t = running.front();
 			running.pop_front();
-			s_[t]->settle(p[t]);
-			if (s_[t]->advance(p[t], SIDE_CELLS, true)) running.push_back(t);
-			else close(t);
+			go_on(t, [&] { s_[t]->settle(p[t]); });
 		}
 		for (int t = 0; t < N; ++t) {
 			Solver<M> *s = s_[t];
@@ -946,6 +957,7 @@ private:
 			base_[t].updates += s->updates_ - before[t].updates;
 			base_[t].substeps += s->n_substeps_ - before[t].substeps;
 		}
+		if (failed) std::rethrow_exception(failed);
 	}
 
 public:
