@@ -1109,9 +1109,11 @@ public:
 		const int n   = top - 1;
 		if (n <= 0) return;
 		ensure_spare();
-		int bits = D * max_tree_level_;
+		const int top_level = std::min(max_tree_level_, SORT_LEVELS<D>);
+		int bits            = D * top_level;
 		while (bits < 31 && (1 << bits) <= top) ++bits;
 		const int end_bit = bits + SORT_CODE_BITS;
+		static_assert(D * SORT_LEVELS<D> + SORT_CODE_BITS <= 64, "a sort key has 64 bits");
 		size_t temp = 0;
 		DG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp, (uint64_t *) nullptr, (uint64_t *) nullptr,
 		                                        (int32_t *) nullptr, (int32_t *) nullptr, n, 0, end_bit, st_));
@@ -1137,7 +1139,7 @@ public:
 		b += align_up(sizeof(int32_t) * (top + 1));
 		void *tmp = b;
 		const int g = grid_for(n);
-		run_k(DG_K_OTHER, 0, [&] { k_sort_keys<D><<<g, BLOCK, 0, st_>>>(P_, top, max_tree_level_, bits, k_in, v_in); });
+		run_k(DG_K_OTHER, 0, [&] { k_sort_keys<D><<<g, BLOCK, 0, st_>>>(P_, top, top_level, bits, k_in, v_in); });
 		DG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, temp, k_in, k_out, v_in, v_out, n, 0, end_bit, st_));
 		run_k(DG_K_OTHER, 0, [&] { k_sort_inverse<<<g, BLOCK, 0, st_>>>(v_out, n, newidx); });
 		auto rows = [&](const RowTable &t) {

@@ -2156,7 +2156,10 @@ constexpr int SORT_CODE_BITS = 5;      // of the codes 0 .. SORT_OTHERS
 
 // Keys of `bits` low bits under the cluster: the Morton code of the cell's corner at tree level `top_level`
 // (D * top_level <= bits), or, for a slot in no cluster, its number, behind all clusters. A sort over the
-// bits in use takes half the passes of one over 64 (29 bits instead of 64 for 3D trees of 8 levels).
+// bits in use takes half the passes of one over 64 (29 bits instead of 64 for 3D trees of 8 levels). A tree may be
+// allowed deeper than SORT_LEVELS; cells below share the code of their ancestor there, and the key keeps its 64 bits.
+template<int D>
+constexpr int SORT_LEVELS = D == 2 ? 29 : 19;  // what spread2 and spread3 take
 template<int D>
 __global__ void k_sort_keys(Pool P, int top, int top_level, int bits, uint64_t *keys, int32_t *vals) {
 	for (int j = gtid(); j < top - 1; j += gstride()) {
@@ -2165,10 +2168,11 @@ __global__ void k_sort_keys(Pool P, int top, int top_level, int bits, uint64_t *
 		uint64_t code   = cl >= 0 ? (uint64_t) cl : (uint64_t) SORT_OTHERS;
 		uint64_t m      = (uint64_t) i;
 		if (cl >= 0) {
-			const int sh = max(top_level - P.level[i], 0);
+			const int sh = top_level - P.level[i];
 			m            = 0;
 			for (int d = 0; d < D; ++d) {
-				const uint64_t c = (uint64_t) P.coord[(size_t) d * P.cap + i] << sh;
+				uint64_t c = (uint64_t) P.coord[(size_t) d * P.cap + i];
+				c          = sh >= 0 ? c << sh : c >> -sh;
 				m |= (D == 2 ? spread2(c) : spread3(c)) << d;
 			}
 		}
