@@ -477,6 +477,9 @@ int fail(int code, const std::string &msg) {
 
 size_t smem_predict(const Layout &L) { return sizeof(float) * L.n; }
 size_t smem_grad(const Layout &L) { return sizeof(float) * TileMem::floats(L); }
+// The limit of a kernel's shared memory holds for the device, not for a network: it is the widest network's.
+int smem_limit_predict() { return (int) smem_predict(Layout(MAX_IN)); }
+int smem_limit_grad() { return (int) smem_grad(Layout(MAX_IN)); }
 
 // Device copies of host arrays on the network's stream, given back on scope exit.
 struct DevBuf {
@@ -503,8 +506,8 @@ static int mlp_create_steps(dg_mlp *h, int n_in, unsigned long long seed) {
 	MLP_CUDA(cudaMalloc(&h->v, sizeof(float) * n));
 	MLP_CUDA(cudaMalloc(&h->wb, sizeof(__nv_bfloat16) * n));
 	MLP_CUDA(cudaMalloc(&h->loss, sizeof(double)));
-	MLP_CUDA(cudaFuncSetAttribute(k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_grad(h->L)));
-	MLP_CUDA(cudaFuncSetAttribute(k_epoch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_grad(h->L)));
+	MLP_CUDA(cudaFuncSetAttribute(k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit_grad()));
+	MLP_CUDA(cudaFuncSetAttribute(k_epoch, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit_grad()));
 	MLP_CUDA(cudaFuncSetAttribute(k_epoch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 	{
 		// sixteen blocks where the device can place such a cluster, else the portable eight
@@ -525,7 +528,7 @@ static int mlp_create_steps(dg_mlp *h, int n_in, unsigned long long seed) {
 		}
 		h->cluster = fit > 0 ? 16 : 8;
 	}
-	MLP_CUDA(cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_predict(h->L)));
+	MLP_CUDA(cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit_predict()));
 	// He-uniform hidden layers, Glorot-uniform output layer, zero biases
 	std::vector<float> w(n, 0.f);
 	uint64_t s = seed;

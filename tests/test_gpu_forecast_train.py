@@ -64,3 +64,21 @@ def test_gradient_over_many_tiles():
     assert abs(loss - rl) <= 1e-5 * abs(rl)
     assert np.abs(g - rg).max() <= 1e-5 * np.abs(rg).max()
     net.close()
+
+
+@pytest.mark.parametrize("widths", [(20, 15), (32, 1), (15, 32, 20)])
+def test_networks_of_several_widths_at_once(widths):
+    """A network made later, with fewer inputs, takes nothing from those that are there."""
+    rng = np.random.default_rng(5)
+    nets = [Mlp(w, seed=3) for w in widths]
+    for _ in range(2):
+        for net in nets:
+            x = rng.normal(size=(100, net.n_in)).astype(np.float32)
+            y = (rng.random(100) < 0.3).astype(np.float32)
+            loss, g = net.loss_grad(x, y, pos_weight=PW)
+            rl, rg = ref.loss_grad(net.params.astype(np.float64), x, y, PW)
+            assert abs(loss - rl) <= 1e-5 * abs(rl) and np.abs(g - rg).max() <= 1e-5 * np.abs(rg).max()
+            assert np.isfinite(net.train(x, y, epochs=1, batch=64, lr=LR, pos_weight=PW, seed=SEED))
+            assert np.isfinite(net.predict(x)).all()
+    for net in nets:
+        net.close()
