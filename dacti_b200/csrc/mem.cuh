@@ -20,6 +20,7 @@ struct DeviceMemory {
 
 	cudaMemPool_t pool  = nullptr;
 	cudaStream_t stream = nullptr;  // of frees whose last use the host has waited for
+	size_t total        = 0;        // the device's memory
 	int users           = 0;
 
 	static std::mutex &lock() {
@@ -49,6 +50,8 @@ struct DeviceMemory {
 			if ((e = cudaMemPoolCreate(&pool, &p)) != cudaSuccess) return nullptr;
 			unsigned long long keep = KEEP;
 			e                       = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+			size_t free_now = 0, total = 0;
+			if (e == cudaSuccess) e = cudaMemGetInfo(&free_now, &total);
 			if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
 			if (e != cudaSuccess) {
 				cudaMemPoolDestroy(pool);
@@ -56,6 +59,7 @@ struct DeviceMemory {
 			}
 			d.pool   = pool;
 			d.stream = stream;
+			d.total  = total;
 		}
 		return &d;
 	}
@@ -93,6 +97,13 @@ inline size_t mem_unused() {
 	    cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
 		return 0;
 	return reserved > used ? (size_t) (reserved - used) : 0;
+}
+// Whether more than half of the device's memory is in use by solvers.
+inline bool mem_tight() {
+	cudaError_t e;
+	DeviceMemory *d         = DeviceMemory::of_device(e);
+	unsigned long long used = 0;
+	return !d || cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > d->total / 2;
 }
 // A user of the current device's pool, as long as it lives.
 class MemoryUser {

@@ -364,26 +364,39 @@ public:
 	static size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
 	// The spare buffer of the re-sort and gc holds the largest field of the pool (the reconstruction records,
-	// in practice), or a second pool where that is small enough: a re-sort then writes every field once, in
-	// three launches, and the two change places.
-	static constexpr size_t SECOND_POOL_MAX = size_t(4) << 30;
-	bool spare_dirty_ = true;  // the spare buffer holds something else than an earlier state of the pool
+	// in practice), or a second pool where that is small and fits: a re-sort then writes every field once, in
+	// three launches, and the two change places. Launches are what a re-sort of a small pool consists of (some seventy field
+	// by field, 0.2 ms); above SECOND_POOL_MAX the copies are, a thousandth of a step, and the memory is worth more. A solver
+	// gives the second pool up again once more than half of the device's memory is in use.
+	static constexpr size_t SECOND_POOL_MAX = size_t(256) << 20;
+	bool spare_dirty_ = true;   // the spare buffer holds something else than an earlier state of the pool
+	bool spare_small_ = false;  // a second pool of this size did not fit
 	size_t pool_bytes(Pool &P) {
 		size_t total = 0;
 		for (auto &f: fields(P)) total += field_bytes(f, P.cap);
 		return total;
 	}
-	bool second_pool() { return pool_bytes(P_) <= SECOND_POOL_MAX; }
+	bool second_pool() { return spare_bytes_ >= pool_bytes(P_); }
 	void ensure_spare() {
-		size_t need = 0;
-		for (auto &f: fields(P_)) need = std::max(need, field_bytes(f, P_.cap));
-		if (second_pool()) need = pool_bytes(P_);
-		if (spare_mem_ && spare_bytes_ >= need) return;
+		size_t field = 0;
+		for (auto &f: fields(P_)) field = std::max(field, field_bytes(f, P_.cap));
+		const size_t whole = pool_bytes(P_);
+		const bool two     = whole <= SECOND_POOL_MAX && !spare_small_ && !mem_tight();
+		if (spare_mem_ && spare_bytes_ >= (two ? whole : field) && (two || spare_bytes_ < whole)) return;
 		mem_free(spare_mem_, st_);
-		spare_mem_ = nullptr;
-		DG_CUDA(mem_alloc((void **) &spare_mem_, need, st_));
-		spare_bytes_ = need;
-		spare_dirty_ = true;
+		spare_mem_    = nullptr;
+		spare_bytes_  = 0;
+		spare_dirty_  = true;
+		cudaError_t e = mem_alloc((void **) &spare_mem_, two ? whole : field, st_);
+		spare_bytes_  = two ? whole : field;
+		if (two && e == cudaErrorMemoryAllocation) {
+			cudaGetLastError();
+			spare_small_ = true;
+			e            = mem_alloc((void **) &spare_mem_, field, st_);
+			spare_bytes_ = field;
+		}
+		if (e != cudaSuccess) spare_mem_ = nullptr, spare_bytes_ = 0;
+		DG_CUDA(e);
 	}
 
 	// Bytes of one field: comps < 0 marks a field this case does not store (no storage, null pointer);
@@ -490,6 +503,7 @@ public:
 		spare_mem_   = nullptr;
 		spare_bytes_ = 0;
 		spare_dirty_ = true;
+		spare_small_ = false;
 		mem_free(sort_mem_, st_);
 		sort_mem_   = nullptr;
 		sort_bytes_ = 0;
@@ -788,9 +802,10 @@ private:
 	// The capacity wanted when `need` slots must fit: a quarter more, and twice the old one while that is small
 	// (a growth costs about 0.3 ms whatever the size, and a tree that refines from a coarse grid grows ten times
 	// its size within a few steps).
+	static constexpr size_t DOUBLING_MAX = size_t(512) << 20;
 	long long grown(long long need) {
 		const long long cap = P_.cap;
-		return std::max(need + need / 4, pool_bytes(P_) < SECOND_POOL_MAX / 8 ? cap * 2 : cap * 5 / 4);
+		return std::max(need + need / 4, pool_bytes(P_) < DOUBLING_MAX ? cap * 2 : cap * 5 / 4);
 	}
 
 	void substep_tail(int L, int n) {
@@ -1123,8 +1138,17 @@ public:
 			mem_free(sort_mem_, st_);
 			sort_mem_   = nullptr;
 			sort_bytes_ = 0;
-			DG_CUDA(mem_alloc((void **) &sort_mem_, need + need / 2, st_));
-			sort_bytes_ = need + need / 2;
+			// half as much again for a tree that grows, where there is room for it
+			size_t got    = need + need / 2;
+			cudaError_t e = mem_alloc(&sort_mem_, got, st_);
+			if (e == cudaErrorMemoryAllocation) {
+				cudaGetLastError();
+				got = need;
+				e   = mem_alloc(&sort_mem_, got, st_);
+			}
+			if (e != cudaSuccess) sort_mem_ = nullptr;
+			DG_CUDA(e);
+			sort_bytes_ = got;
 		}
 		char *b          = (char *) sort_mem_;
 		uint64_t *k_in   = (uint64_t *) b;

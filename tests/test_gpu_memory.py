@@ -1,0 +1,44 @@
+"""Solver memory where the GPU has little left: what fitted without the re-sort's second pool still runs."""
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+SCRIPT = """
+import dataclasses, sys
+import torch
+from dacti_b200 import cases
+from dacti_b200.solver import Solver
+
+def make():
+    c = cases.lax_liu3(5, 2)
+    return Solver(dataclasses.replace(c, params=dataclasses.replace(c.params, pool_capacity=500000)))
+
+def run(s):
+    for _ in range(4):
+        assert not s.integrate()[1]
+    a = s.active_cells()
+    s.close()
+    return [getattr(a, f).tobytes() for f in ("tree_level", "acti_level", "center", "t", "u", "p", "error")]
+
+first = Solver(cases.lax_liu3(3, 1))  # the kernels' own memory is reserved at their first launch
+first.integrate()
+first.close()
+s = make()
+hold = torch.empty(torch.cuda.mem_get_info()[0] - (150 << 20), dtype=torch.uint8, device="cuda")
+tight = run(s)
+del hold
+torch.cuda.empty_cache()
+assert tight == run(make())
+"""
+
+
+def test_resort_without_room_for_a_second_pool():
+    """A pool of half a million slots (about 200 MB) on a GPU with 150 MB left, in a fresh process so that nothing freed
+    before helps: the re-sort's one-field buffer serves, with the same cells in the same order."""
+    r = subprocess.run([sys.executable, "-c", SCRIPT], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
