@@ -1024,15 +1024,13 @@ private:
 		C_.coarsen = (n_global_ % coarsen_every_) == 0;
 	}
 	// Up to the next run: substeps of clusters above `limit` are the host's. False when the step is over.
-	bool advance(Step &p, int limit, bool clustered) {
+	bool run_due(Step &p, int limit) {
 		while (!p.broke && !p.done) {
 			int s = p.seq, k = p.l;
 			const int next = next_substep(s, k);
 			if (next < 0) {
 				p.done = true;
 			} else if (h_cnt_->clu[next] <= limit) {
-				run_begin(p.seq, p.l, limit, clustered);
-				++p.runs;
 				return true;
 			} else {
 				p.seq = s;
@@ -1044,11 +1042,16 @@ private:
 		}
 		return false;
 	}
-	// The end of a run, and of the substep that it left to the host.
-	void settle(Step &p) {
-		int L          = 0;
-		const int stop = run_end(p.seq, p.l, L);
-		p.done         = stop == RUN_DONE;
+	// The same, and starts the run.
+	bool advance(Step &p, int limit, bool clustered) {
+		if (!run_due(p, limit)) return false;
+		run_begin(p.seq, p.l, limit, clustered);
+		++p.runs;
+		return true;
+	}
+	// The substep that a run which ended for `stop` left to the host; `L` is its level.
+	void after_run(Step &p, int stop, int L) {
+		p.done = stop == RUN_DONE;
 		if (stop == RUN_STATUS) {
 			check_status();
 			p.broke = h_cnt_->status & ST_NAN;
@@ -1065,6 +1068,12 @@ private:
 		} else if (stop == RUN_LARGE) {
 			++p.stops;
 		}
+	}
+	// The end of a run, and of the substep that it left to the host.
+	void settle(Step &p) {
+		int L          = 0;
+		const int stop = run_end(p.seq, p.l, L);
+		after_run(p, stop, L);
 	}
 	void host_substep(int L) {
 		const int n = h_cnt_->clu[L];
@@ -1088,12 +1097,18 @@ public:
 		// Runs on the device serve the default stage choices; the host issues a substep's stages one by one
 		// where a callback or the timing of every stage asks for it, and for clusters that fill the GPU.
 		if (!fn && !prof_ && opts_ == DG_OPT_DEFAULT) {
-			while (!p.done && !p.broke) {
+			while (run_due(p, RUN_CELLS)) {
 				const bool clustered = peers >= RUN_PEERS || most_cells(RUN_CELLS) <= RUN_CLUSTER_CELLS;
-				// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU
-				std::unique_lock<std::mutex> hold(whole_gpu(), std::defer_lock);
-				if (!clustered) hold.lock();
-				if (advance(p, RUN_CELLS, clustered)) settle(p);
+				int stop, L;
+				{
+					// a grid-wide run takes every SM; two of them wait for one another on the host, not on the GPU.
+					// What the host does for a solver goes on beside another's run
+					std::unique_lock<std::mutex> hold(whole_gpu(), std::defer_lock);
+					if (!clustered) hold.lock();
+					advance(p, RUN_CELLS, clustered);
+					stop = run_end(p.seq, p.l, L);
+				}
+				after_run(p, stop, L);
 			}
 		} else {
 			for (int L; !p.broke && (L = next_substep(p.seq, p.l)) >= 0;) {

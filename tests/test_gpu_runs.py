@@ -111,6 +111,21 @@ def test_runs_side_by_side():
         assert got.u[o].tobytes() == want[3][4].tobytes() and st.cell_updates == want[2][0]
 
 
+def test_large_runs_side_by_side():
+    """Fewer solvers than make one-cluster runs: clusters that the host steps (262144 cells), grid-wide runs and a
+    small tree at once, on a thread each."""
+    batch = [cases.lax_liu3(9, 1), cases.lax_liu3(6, 3), cases.lax_liu3(9, 1, max_cfl=0.4), cases.lax_liu3(7, 2), cases.lax_liu3(3, 2)]
+    side = [Solver(c) for c in batch]
+    for _ in range(3):
+        step_many(side, threads=5)
+    for c, s in zip(batch, side):
+        got, st = s.active_cells(), s.stats()
+        s.close()
+        want = _run(c, 3)
+        o = np.argsort(_keys(got, 1.0))
+        assert got.u[o].tobytes() == want[3][4].tobytes() and st.cell_updates == want[2][0]
+
+
 @pytest.mark.parametrize("name", ["tiny", "walls3", "drop2", "drop3_mixed"])
 def test_fields_equal_records(name):
     """active_cells (field arrays) and the record read-back give the same values, before and after steps."""
