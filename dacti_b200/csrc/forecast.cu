@@ -455,6 +455,7 @@ struct dg_mlp {
 	Layout L{1};
 	int device = 0;
 	cudaStream_t st = nullptr;
+	cudaEvent_t copied = nullptr;  // an epoch's order and bias corrections are on the device
 	float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
 	__nv_bfloat16 *wb = nullptr;
 	double *loss = nullptr;
@@ -500,6 +501,7 @@ static int mlp_create_steps(dg_mlp *h, int n_in, unsigned long long seed) {
 	const long long n = h->L.n;
 	MLP_CUDA(cudaGetDevice(&h->device));
 	MLP_CUDA(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
+	MLP_CUDA(cudaEventCreateWithFlags(&h->copied, cudaEventDisableTiming));
 	MLP_CUDA(cudaMalloc(&h->w, sizeof(float) * n));
 	MLP_CUDA(cudaMalloc(&h->g, sizeof(float) * n));
 	MLP_CUDA(cudaMalloc(&h->m, sizeof(float) * n));
@@ -638,6 +640,10 @@ int dg_mlp_train(dg_mlp *h, const float *x, const float *y, long long n, int epo
 	std::vector<int> perm(n);
 	for (long long k = 0; k < n; ++k) perm[k] = (int) k;
 	std::vector<float2> bc(steps);
+	struct Drain {  // the arrays outlive their copies, on an error too
+		cudaStream_t st;
+		~Drain() { cudaStreamSynchronize(st); }
+	} drain{h->st};
 	cudaLaunchConfig_t cfg{};
 	cudaLaunchAttribute at[1];
 	at[0].id               = cudaLaunchAttributeClusterDimension;
@@ -651,8 +657,8 @@ int dg_mlp_train(dg_mlp *h, const float *x, const float *y, long long n, int epo
 	cfg.numAttrs           = 1;
 	uint64_t s = seed;
 	for (int e = 0; e < epochs; ++e) {
-		// the host draws the next epoch's order while the GPU runs this one (pageable copies leave the host's
-		// arrays free when they return)
+		// the host draws the next epoch's order while the GPU runs this one, once this one's has left the host's arrays
+		if (e > 0) MLP_CUDA(cudaEventSynchronize(h->copied));
 		for (long long k = n - 1; k > 0; --k) std::swap(perm[k], perm[(long long) (splitmix(s) % (uint64_t) (k + 1))]);
 		for (long long k = 0; k < steps; ++k) {
 			h->t++;
@@ -660,6 +666,7 @@ int dg_mlp_train(dg_mlp *h, const float *x, const float *y, long long n, int epo
 		}
 		MLP_CUDA(cudaMemcpyAsync(dperm.p, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, h->st));
 		MLP_CUDA(cudaMemcpyAsync(dbc.p, bc.data(), sizeof(float2) * steps, cudaMemcpyHostToDevice, h->st));
+		MLP_CUDA(cudaEventRecord(h->copied, h->st));
 		MLP_CUDA(cudaMemsetAsync(h->loss, 0, sizeof(double), h->st));
 		MLP_CUDA(cudaLaunchKernelEx(&cfg, k_epoch, h->w, h->wb, h->m, h->v, h->L, (const float *) dx.p, (const float *) dy.p,
 		                            (const int *) dperm.p, n, (long long) batch, pos_weight, lr, (const float2 *) dbc.p, h->loss));
@@ -682,6 +689,7 @@ int dg_mlp_destroy(dg_mlp *h) {
 	cudaFree(h->v);
 	cudaFree(h->wb);
 	cudaFree(h->loss);
+	if (h->copied) cudaEventDestroy(h->copied);
 	if (h->st) cudaStreamDestroy(h->st);
 	delete h;
 	return DG_OK;

@@ -82,3 +82,34 @@ def test_networks_of_several_widths_at_once(widths):
             assert np.isfinite(net.predict(x)).all()
     for net in nets:
         net.close()
+
+
+@pytest.mark.parametrize("n,batch,epochs", [(300, 64, 3), (1024, 512, 5)])
+def test_epochs_match_oracle(n, batch, epochs):
+    """Several epochs: each runs in its own order, which the host draws while the GPU runs the one before."""
+    rng = np.random.default_rng(n)
+    net = Mlp(15, seed=2)
+    w = net.params.astype(np.float64)
+    x = rng.normal(size=(n, 15)).astype(np.float32)
+    y = (rng.random(n) < 0.3).astype(np.float32)
+    got = net.train(x, y, epochs=epochs, batch=batch, lr=LR, pos_weight=PW, seed=SEED)
+    perm, state, mask = list(range(n)), SEED, (1 << 64) - 1
+    m, v, t = np.zeros_like(w), np.zeros_like(w), 0
+    for _ in range(epochs):
+        for k in range(n - 1, 0, -1):
+            state = (state + 0x9E3779B97F4A7C15) & mask
+            z = ((state ^ (state >> 30)) * 0xBF58476D1CE4E5B9) & mask
+            z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+            j = (z ^ (z >> 31)) % (k + 1)
+            perm[k], perm[j] = perm[j], perm[k]
+        loss = 0.0
+        for first in range(0, n, batch):
+            idx = perm[first:first + batch]
+            part, g = ref.loss_grad(w, x[idx], y[idx], PW)
+            loss, g, t = loss + part, g / len(idx), t + 1
+            m, v = 0.9 * m + 0.1 * g, 0.999 * v + 0.001 * g * g
+            w = w - LR * (m / (1 - 0.9 ** t)) / (np.sqrt(v / (1 - 0.999 ** t)) + 1e-8)
+    off = net.params - w  # the bounds of test_epoch_matches_oracle
+    assert np.sqrt((off ** 2).mean()) <= 1e-3 * LR * t
+    assert abs(got - loss / n) <= 1e-5 * abs(loss / n) + LR * 1e-3
+    net.close()
