@@ -968,6 +968,7 @@ public:
 			return;
 		}
 		const int N = (int) s_.size();
+		for (auto *s: s_) s->need_state();
 		for (int t = 0; t < N; ++t) {
 			Solver<M> *s  = s_[t];
 			s->C_.signal  = signal;

@@ -14,6 +14,7 @@ thread_local int g_device = 0;
 template<typename Fn>
 int guarded(dg_solver *s, Fn &&fn) {
 	try {
+		if (s) s->impl->need_state();
 		cudaError_t e = cudaSetDevice(s ? s->device : g_device);
 		if (e != cudaSuccess) throw dg::dg_error(DG_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
 		fn();
@@ -223,7 +224,10 @@ int dg_batch_create(dg_solver **s, int n, dg_batch **out) {
 		if (!s[k] || s[k]->device != s[0]->device) return DG_ERR_ARG;
 	return guarded(s[0], [&] {
 		std::vector<dg::SolverBase *> v;
-		for (int k = 0; k < n; ++k) v.push_back(s[k]->impl);
+		for (int k = 0; k < n; ++k) {
+			s[k]->impl->need_state();
+			v.push_back(s[k]->impl);
+		}
 		const int model = v[0]->model_id(), dims = v[0]->dims();
 		for (auto *x: v)
 			if (x->model_id() != model || x->dims() != dims)

@@ -61,6 +61,7 @@ void noalloc_prepare(int device) { (void) scratch_address(device); }
 extern "C" int dg_read_cells_noalloc(dg_solver *s, int *levels, double *data, long long max_cells, long long *n_out) {
 	if (!s || !levels || !data) return DG_ERR_ARG;
 	try {
+		s->impl->need_state();
 		cudaError_t e = cudaSetDevice(s->device);
 		if (e != cudaSuccess) throw dg::dg_error(DG_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
 		void *scratch = scratch_address(s->device);

@@ -79,8 +79,9 @@ struct DealtGrid {
 	__device__ __forceinline__ int step() const { return blocks * (RUN_THREADS / 32); }
 };
 
-// A wait longer than this many polls (seconds) gives up: the launch ends without leaving a state, which the host
-// takes for the error it is.
+// A wait longer than this many polls (seconds of them) gives up: the launch ends without leaving a state, and the host
+// takes the solver for lost. All blocks of a run are on the GPU together, so a wait is as long as the slowest block's
+// stage, microseconds to milliseconds; polls, unlike a clock, stand still where another process has the GPU.
 constexpr int BARRIER_POLLS = 1 << 23;
 
 // Every thread of the launch arrives and leaves; writes before it are visible after it. False when the

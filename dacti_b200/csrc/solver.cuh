@@ -2,9 +2,9 @@
 // level scheduler of Integrator::integrate, issuing the stage kernels of stages.cuh.
 #pragma once
 
-#include "../../include/dacti_gpu.h"
 #include "mem.cuh"
 #include "run.cuh"
+#include "solver_base.h"
 
 #include <cub/cub.cuh>
 
@@ -12,53 +12,9 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <stdexcept>
-#include <string>
 #include <vector>
 
 namespace dg {
-
-struct dg_error : std::runtime_error {
-	int code;
-	dg_error(int c, const std::string &m) :
-	    std::runtime_error(m), code(c) {}
-};
-
-#define DG_CUDA(x)                                                                                     \
-	do {                                                                                               \
-		cudaError_t e_ = (x);                                                                          \
-		if (e_ != cudaSuccess)                                                                         \
-			throw ::dg::dg_error(DG_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));         \
-	} while (0)
-
-class SolverBase {
-public:
-	virtual ~SolverBase() = default;
-	// `peers`: solvers that step at the same time on streams of their own (1: this one has the GPU)
-	virtual void step(int signal, int *force_break, double *global_dt, dg_substep_fn fn, void *user, int peers = 1) = 0;
-	virtual long long cell_count() = 0;
-	virtual long long read_cells(int *levels, double *data, long long max_cells) = 0;
-	virtual long long read_fields(const dg_cell_fields &f, long long max_cells) = 0;
-	virtual long long read_cells_via(int *levels, double *data, long long max_cells, void *scratch, size_t bytes) = 0;
-	virtual long long read_slopes(double *data, long long max_cells) = 0;
-	virtual long long read_gradients(double *data, long long max_cells) = 0;
-	virtual long long forecast_features(double *data, long long max_cells) = 0;
-	virtual long long tree_size() = 0;
-	virtual long long read_tree(int32_t *parent, int32_t *child, int32_t *level, uint32_t *flags, double *p, double *meta,
-	                            long long max_nodes) = 0;
-	virtual int dims() const = 0;
-	virtual void set_hold(const uint8_t *hold, long long n) = 0;
-	virtual void set_coarsen_interval(int k) = 0;
-	virtual void stats(dg_stats *out) = 0;
-	virtual void set_stream(cudaStream_t s) = 0;
-	virtual void own_stream() = 0;  // give the solver a stream of its own if it runs on the legacy default
-	virtual void set_profiling(bool on) = 0;
-	virtual void set_form(int form) = 0;
-	virtual void set_options(int opts) = 0;
-	virtual void prepare_noalloc() = 0;  // loads the read-back gather kernel on the current device
-	virtual int model_id() const = 0;
-	std::string last_error;
-};
 
 inline int grid_for(long long n, int max_blocks = 148 * 16) {
 	long long b = (n + BLOCK - 1) / BLOCK;
@@ -993,9 +949,11 @@ private:
 	// Waits for the run. The host's schedule state, lists and counters are current afterwards. Returns why the
 	// run ended (RunStop); `L` is the level of an unfinished substep.
 	int run_end(int &seq, int &l, int &L) {
+		lost = true;  // the lists are in the run's hands until its state is here
 		DG_CUDA(cudaStreamSynchronize(st_));
 		const RunState &h = *h_run_;
 		if (h.stop < 0) throw dg_error(DG_ERR_CUDA, "a grid barrier of a device-resident run gave up waiting");
+		lost      = false;
 		max_acti_ = h.sch.max_acti;
 		stamp_    = h.sch.stamp;
 		epoch_    = h.sch.epoch;
@@ -1020,6 +978,7 @@ private:
 		long long runs = 0, stops = 0, by_host = 0;
 	};
 	void begin_step(int signal) {
+		need_state();
 		C_.signal  = signal;
 		C_.coarsen = (n_global_ % coarsen_every_) == 0;
 	}
