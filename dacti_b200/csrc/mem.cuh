@@ -4,7 +4,9 @@
 // tree replaces its pool, lists and scratch every few steps, and while many solvers step side by side each
 // such call waits for every other solver's kernels. Allocations from the pool are ordered with the solver's
 // own stream instead. While solvers live the pool keeps up to KEEP bytes that nothing uses; when the last
-// one is gone it gives back all but KEEP_IDLE.
+// one is gone it gives back all but KEEP_IDLE. CUDA's release threshold counts what the pool holds, used or not, so it
+// follows what is in use: a fixed one of KEEP let a synchronisation unmap everything unused, which the next growth
+// mapped again, as soon as solvers used more than that.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -17,10 +19,12 @@ namespace dg {
 struct DeviceMemory {
 	static constexpr size_t KEEP      = size_t(4) << 30;
 	static constexpr size_t KEEP_IDLE = size_t(512) << 20;
+	static constexpr size_t LARGE     = size_t(16) << 20;  // allocations after which the release threshold is looked at
 
 	cudaMemPool_t pool  = nullptr;
 	cudaStream_t stream = nullptr;  // of frees whose last use the host has waited for
 	size_t total        = 0;        // the device's memory
+	size_t threshold    = KEEP;     // the pool's release threshold as last set
 	int users           = 0;
 
 	static std::mutex &lock() {
@@ -63,6 +67,19 @@ struct DeviceMemory {
 		}
 		return &d;
 	}
+
+	size_t in_use() const {
+		unsigned long long used = 0;
+		return cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess ? (size_t) used : 0;
+	}
+	// The release threshold at KEEP above what is in use; set where it is off by an eighth of KEEP.
+	void follow() {
+		const size_t want = in_use() + KEEP;
+		std::lock_guard<std::mutex> l(lock());
+		if (want < threshold + KEEP / 8 && threshold < want + KEEP / 8) return;
+		unsigned long long keep = want;
+		if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) threshold = want;
+	}
 };
 
 // `bytes` of device memory for work on stream `st`, from its order on.
@@ -71,7 +88,10 @@ inline cudaError_t mem_alloc(void **p, size_t bytes, cudaStream_t st) {
 	DeviceMemory *d = DeviceMemory::of_device(e);
 	if (!d) return e;
 	e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st);
-	if (e != cudaErrorMemoryAllocation) return e;
+	if (e != cudaErrorMemoryAllocation) {
+		if (bytes >= DeviceMemory::LARGE) d->follow();
+		return e;
+	}
 	// blocks freed before, of other sizes, may hold the room: give them back and ask once more
 	cudaGetLastError();
 	if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
@@ -101,9 +121,8 @@ inline size_t mem_unused() {
 // Whether more than half of the device's memory is in use by solvers.
 inline bool mem_tight() {
 	cudaError_t e;
-	DeviceMemory *d         = DeviceMemory::of_device(e);
-	unsigned long long used = 0;
-	return !d || cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > d->total / 2;
+	DeviceMemory *d = DeviceMemory::of_device(e);
+	return !d || d->in_use() > d->total / 2;
 }
 // A user of the current device's pool, as long as it lives.
 class MemoryUser {
@@ -119,10 +138,12 @@ public:
 	MemoryUser(const MemoryUser &)            = delete;
 	MemoryUser &operator=(const MemoryUser &) = delete;
 	~MemoryUser() {
-		std::lock_guard<std::mutex> l(DeviceMemory::lock());
-		if (!d_ || --d_->users > 0) return;
+		if (!d_) return;
+		// what the user held has been given back on `stream` (mem_free_idle)
 		cudaStreamSynchronize(d_->stream);
-		cudaMemPoolTrimTo(d_->pool, DeviceMemory::KEEP_IDLE);
+		d_->follow();
+		std::lock_guard<std::mutex> l(DeviceMemory::lock());
+		cudaMemPoolTrimTo(d_->pool, --d_->users > 0 ? d_->threshold : DeviceMemory::KEEP_IDLE);
 	}
 };
 
