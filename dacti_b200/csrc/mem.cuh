@@ -1,31 +1,43 @@
-// Device memory of the solvers: one stream-ordered pool per device, owned by the library.
+// Device memory of the solvers: small blocks from one stream-ordered pool per device, owned by the library, large
+// ones from cudaMalloc.
 //
 // cudaMalloc and cudaFree wait for the whole device. A solver makes about fifteen allocations, a growing
 // tree replaces its pool, lists and scratch every few steps, and while many solvers step side by side each
 // such call waits for every other solver's kernels. Allocations from the pool are ordered with the solver's
-// own stream instead. While solvers live the pool keeps up to KEEP bytes that nothing uses; when the last
-// one is gone it gives back all but KEEP_IDLE. CUDA's release threshold counts what the pool holds, used or not, so it
-// follows what is in use: a fixed one of KEEP let a synchronisation unmap everything unused, which the next growth
-// mapped again, as soon as solvers used more than that.
+// own stream instead. But the pool maps and unmaps memory at 6.5 ms a GiB each way, with stalls of a second and more
+// on a shared host, where cudaMalloc takes 1 to 2 ms and cudaFree 0.5 ms a GiB whatever the size: a tree that grows from 2 to
+// 36 GiB takes 0.15 s with the one and 0.7 to 4.7 s with the other. So blocks of LARGE bytes on do not come from the pool.
+// A large block that is given back waits in a list for the next moment that waits for the device anyway: an allocation that
+// does not fit, the end of a user, or KEEP bytes of them.
+//
+// While solvers live the pool keeps up to KEEP bytes that nothing uses; when the last one is gone it gives
+// back all but KEEP_IDLE. CUDA's release threshold counts what the pool holds, used or not, so it follows what is in
+// use: a fixed one let a synchronisation unmap everything unused, which the next growth mapped again, as soon as solvers
+// used more than that.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 namespace dg {
 
 struct DeviceMemory {
-	static constexpr size_t KEEP      = size_t(4) << 30;
+	static constexpr size_t KEEP      = size_t(2) << 30;
 	static constexpr size_t KEEP_IDLE = size_t(512) << 20;
-	static constexpr size_t LARGE     = size_t(16) << 20;  // allocations after which the release threshold is looked at
+	static constexpr size_t LARGE     = size_t(64) << 20;  // a mapping of this size takes as long as cudaMalloc
+	static constexpr size_t NOTICE    = size_t(4) << 20;   // allocations after which the release threshold is looked at
 
 	cudaMemPool_t pool  = nullptr;
 	cudaStream_t stream = nullptr;  // of frees whose last use the host has waited for
 	size_t total        = 0;        // the device's memory
 	size_t threshold    = KEEP;     // the pool's release threshold as last set
 	int users           = 0;
+	std::unordered_map<void *, size_t> large;  // blocks from cudaMalloc
+	std::vector<void *> retired;               // the same, given back
+	size_t large_bytes = 0, retired_bytes = 0;
 
 	static std::mutex &lock() {
 		static std::mutex m;
@@ -34,7 +46,7 @@ struct DeviceMemory {
 
 	// The current device's memory, made at its first use; null with the error in `e`.
 	static DeviceMemory *of_device(cudaError_t &e) {
-		static DeviceMemory all[64];
+		static DeviceMemory *all = new DeviceMemory[64];  // outlives every user, at the process's end too
 		int dev = 0;
 		if ((e = cudaGetDevice(&dev)) != cudaSuccess) return nullptr;
 		if (dev < 0 || dev >= 64) {
@@ -68,17 +80,57 @@ struct DeviceMemory {
 		return &d;
 	}
 
-	size_t in_use() const {
+	size_t pool_in_use() const {
 		unsigned long long used = 0;
 		return cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess ? (size_t) used : 0;
 	}
 	// The release threshold at KEEP above what is in use; set where it is off by an eighth of KEEP.
 	void follow() {
-		const size_t want = in_use() + KEEP;
+		const size_t want = pool_in_use() + KEEP;
 		std::lock_guard<std::mutex> l(lock());
 		if (want < threshold + KEEP / 8 && threshold < want + KEEP / 8) return;
 		unsigned long long keep = want;
 		if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) threshold = want;
+	}
+	cudaError_t alloc(void **p, size_t bytes, cudaStream_t st) {
+		if (bytes < LARGE) {
+			const cudaError_t e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, st);
+			if (e == cudaSuccess && bytes >= NOTICE) follow();
+			return e;
+		}
+		const cudaError_t e = cudaMalloc(p, bytes);
+		if (e != cudaSuccess) return e;
+		std::lock_guard<std::mutex> l(lock());
+		large[*p] = bytes;
+		large_bytes += bytes;
+		return cudaSuccess;
+	}
+	// Takes back a large block, which work already queued may still use; false for a block of the pool.
+	bool retire(void *p) {
+		{
+			std::lock_guard<std::mutex> l(lock());
+			const auto it = large.find(p);
+			if (it == large.end()) return false;
+			large_bytes -= it->second;
+			retired_bytes += it->second;
+			large.erase(it);
+			retired.push_back(p);
+			if (retired_bytes <= KEEP) return true;
+		}
+		reclaim();
+		return true;
+	}
+	// Frees the retired blocks once nothing uses them.
+	void reclaim() {
+		std::vector<void *> gone;
+		{
+			std::lock_guard<std::mutex> l(lock());
+			gone.swap(retired);
+			retired_bytes = 0;
+		}
+		if (gone.empty()) return;
+		cudaDeviceSynchronize();
+		for (void *p: gone) cudaFree(p);
 	}
 };
 
@@ -87,28 +139,28 @@ inline cudaError_t mem_alloc(void **p, size_t bytes, cudaStream_t st) {
 	cudaError_t e;
 	DeviceMemory *d = DeviceMemory::of_device(e);
 	if (!d) return e;
-	e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st);
-	if (e != cudaErrorMemoryAllocation) {
-		if (bytes >= DeviceMemory::LARGE) d->follow();
-		return e;
-	}
-	// blocks freed before, of other sizes, may hold the room: give them back and ask once more
+	e = d->alloc(p, bytes, st);
+	if (e != cudaErrorMemoryAllocation) return e;
+	// blocks given back before may hold the room: free them and ask once more
 	cudaGetLastError();
 	if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+	d->reclaim();
 	cudaMemPoolTrimTo(d->pool, 0);
-	return cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, d->pool, st);
+	return d->alloc(p, bytes, st);
 }
 // Gives memory back once the work queued on `st` so far is done with it.
 inline void mem_free(void *p, cudaStream_t st) {
-	if (p) cudaFreeAsync(p, st);
+	cudaError_t e;
+	DeviceMemory *d = p ? DeviceMemory::of_device(e) : nullptr;
+	if (d && !d->retire(p)) cudaFreeAsync(p, st);
 }
 // Gives back memory that nothing queued uses any more, whatever became of the stream it was used on.
 inline void mem_free_idle(void *p) {
 	cudaError_t e;
 	DeviceMemory *d = p ? DeviceMemory::of_device(e) : nullptr;
-	if (d) cudaFreeAsync(p, d->stream);
+	if (d && !d->retire(p)) cudaFreeAsync(p, d->stream);
 }
-// Bytes that the pool holds and nothing uses.
+// Bytes that the library holds and nothing uses.
 inline size_t mem_unused() {
 	cudaError_t e;
 	DeviceMemory *d             = DeviceMemory::of_device(e);
@@ -116,15 +168,19 @@ inline size_t mem_unused() {
 	if (!d || cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
 	    cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
 		return 0;
-	return reserved > used ? (size_t) (reserved - used) : 0;
+	std::lock_guard<std::mutex> l(DeviceMemory::lock());
+	return (reserved > used ? (size_t) (reserved - used) : 0) + d->retired_bytes;
 }
 // Whether more than half of the device's memory is in use by solvers.
 inline bool mem_tight() {
 	cudaError_t e;
 	DeviceMemory *d = DeviceMemory::of_device(e);
-	return !d || d->in_use() > d->total / 2;
+	if (!d) return true;
+	const size_t used = d->pool_in_use();
+	std::lock_guard<std::mutex> l(DeviceMemory::lock());
+	return used + d->large_bytes > d->total / 2;
 }
-// A user of the current device's pool, as long as it lives.
+// A user of the current device's memory, as long as it lives.
 class MemoryUser {
 	DeviceMemory *d_;
 
@@ -139,7 +195,8 @@ public:
 	MemoryUser &operator=(const MemoryUser &) = delete;
 	~MemoryUser() {
 		if (!d_) return;
-		// what the user held has been given back on `stream` (mem_free_idle)
+		// what the user held has been given back (mem_free_idle)
+		d_->reclaim();
 		cudaStreamSynchronize(d_->stream);
 		d_->follow();
 		std::lock_guard<std::mutex> l(DeviceMemory::lock());
