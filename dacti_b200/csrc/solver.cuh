@@ -321,10 +321,11 @@ public:
 
 	// The spare buffer of the re-sort and gc holds the largest field of the pool (the reconstruction records,
 	// in practice), or a second pool where that is small and fits: a re-sort then writes every field once, in
-	// three launches, and the two change places. Launches are what a re-sort of a small pool consists of (some seventy field
-	// by field, 0.2 ms); above SECOND_POOL_MAX the copies are, a thousandth of a step, and the memory is worth more. A solver
-	// gives the second pool up again once more than half of the device's memory is in use.
-	static constexpr size_t SECOND_POOL_MAX = size_t(256) << 20;
+	// three launches, and the two change places. Field by field it is some seventy launches (0.2 ms, which small trees
+	// notice) and every field is written twice (nine trees of a million cells on one level, 0.9 GB of pool each, 35 ms a
+	// step against 32). A larger pool's memory is worth more. A solver gives the second pool up again once more than half
+	// of the device's memory is in use.
+	static constexpr size_t SECOND_POOL_MAX = size_t(1) << 30;
 	bool spare_dirty_ = true;   // the spare buffer holds something else than an earlier state of the pool
 	bool spare_small_ = false;  // a second pool of this size did not fit
 	size_t pool_bytes(Pool &P) {
@@ -846,13 +847,13 @@ private:
 	// ---- device-resident runs (run.cuh) ---------------------------------------------------------
 
 	// Largest cluster a run takes. Above it a substep's launches fill the GPU, and each of them has the
-	// registers and block size of its own stage, where a run has one for all. Between 32768 and 98304 cells the
-	// two are even (drop3d of perf/cases.py, clusters of 17 thousand cells on average, steps in 137 to 133 ms, the
-	// larger drop3d_large in 664 to 675); at 16384 the runs lose (the cylinder 109 ms against 80).
+	// registers and block size of its own stage, where a run has one for all. With the limit between 32768 and 98304
+	// cells steps take the same (a 32x16x16 + 3-level shock-drop, clusters of 17 thousand cells on average, 137 to 133 ms
+	// for two steps; 64x16x16 + 4 levels 664 to 675 for one); with 16384 a 128x64 + 5-level cylinder loses, 109 ms against 80.
 	static constexpr int RUN_CELLS = 1 << 16;
 	// Largest cluster for which a run is one thread-block cluster (its barrier is 0.35 us, the grid's 1.3):
-	// up to about here the run of sixteen SMs is as fast as the one of all (drop2d 107 ms against 118,
-	// lax_tiny 23 against 27).
+	// up to about here the run of sixteen SMs is as fast as the one of all (three steps of a 64x32 + 3-level shock-drop
+	// 107 ms against 118, twelve of a 16^2 + 2-level quadrant problem 23 against 27).
 	static constexpr int RUN_CLUSTER_CELLS = 2048;
 	// Solvers side by side from which each takes one thread-block cluster, whatever its size.
 	static constexpr int RUN_PEERS = 9;
