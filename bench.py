@@ -68,7 +68,7 @@ def parse_args():
     ap.add_argument("--batched-only", action="store_true", help="run only the batched section and print it")
     ap.add_argument("--no-pregrow", action="store_true", help="batched section: grow pools only at the capacity check")
     ap.add_argument("--batch-groups", type=int, default=0,
-                    help="batched section: also time this many lockstep groups stepped concurrently (0: not)")
+                    help="batched section: also time this many batches of a share of the trees stepped concurrently (0: not)")
     ap.add_argument("--learned-shock", action="store_true",
                     help="also run the forecast-driven regrid on the shock-drop of the bench workload")
     ap.add_argument("--forms", default="fp64,mixed",
@@ -432,11 +432,10 @@ def learned_shock_run(args, local_rank: int) -> dict:
 
 def batched_run(args, rank: int, local_rank: int, world: int) -> dict:
     """Batched 2D Euler quadtree Riemann problems (seeded, see cases.riemann_batch), mixed form. The
-    lockstep batch (dg_batch: merged ACTI schedules, one launch per stage for all trees of a level, the
-    global step planned on the host and issued with no synchronisation, device guards stopping a run
-    where the live counts leave the plan) is timed around its steps, beside dg_step_many (host threads,
-    one stream per tree, one synchronisation per tree and substep) and the same trees stepped one after
-    another. One more step with per-stage CUDA-event timing gives the device time per stage kind. With N
+    batch (dg_batch: each tree's global step one device-resident run, side by side; the keys named `lockstep` are
+    its times) is timed around its steps, beside dg_step_many (host threads, one stream and run per tree)
+    and the same trees stepped one after another. One more step with per-stage CUDA-event timing, which steps
+    in lockstep, gives the device time per stage kind. With N
     ranks the trees are split among them (dacti_b200.batch, no exchange): the batch's total work is fixed
     (strong scaling)."""
     import torch
@@ -457,7 +456,7 @@ def batched_run(args, rank: int, local_rank: int, world: int) -> dict:
     def updates(solvers):
         return float(sum(s.stats().cell_updates for s in solvers))
 
-    # lockstep batch: W warm-up steps, K timed steps between events on the batch's stream
+    # the batch: W warm-up steps, K timed steps on the host's clock, synchronised on both sides
     solvers = make()
     b = Batch(solvers)
     b.set_pregrow(not args.no_pregrow)
@@ -488,8 +487,7 @@ def batched_run(args, rank: int, local_rank: int, world: int) -> dict:
     for s in solvers:
         s.close()
 
-    # the trees in work-balanced groups, one lockstep batch and host thread each: merged launches within a
-    # group, concurrent streams across groups
+    # the trees in work-balanced groups, one batch and host thread each
     from dacti_b200.batch import partition
     from dacti_b200.solver import step_batches
     groups = args.batch_groups
@@ -552,7 +550,7 @@ def batched_run(args, rank: int, local_rank: int, world: int) -> dict:
                     f"+2..4 levels, seeded quadrant states (seed 3), LTS, mixed form{split}",
         "scaling": "strong", "trees_rank0": len(mine), "unit": UNIT, "steps": args.steps,
         "value": l_u / (l_ms * 1e-3), "ms_per_step": l_ms / args.steps,
-        "timing": "host wall clock around K lockstep batch steps (dg_batch_step), synchronised before and after",
+        "timing": "host wall clock around K batch steps (dg_batch_step), synchronised before and after",
         "planned_runs": runs,
         "pregrow": not args.no_pregrow,
         "force_breaks": int(breaks),

@@ -1,8 +1,13 @@
-// Batched trees: many independent solvers of one model advanced in lockstep by one host thread, with
-// one launch per stage for all trees that run a level and no host synchronisation inside a global step.
+// Batched trees: many independent solvers of one model advanced by one host thread, in one of two ways. Every tree
+// keeps its own node pool, lists, counters and ACTI schedule state, so in both each tree computes exactly what it
+// computes alone (impl/integrate.hpp:26-87 per tree).
 //
-// Every tree keeps its own node pool, lists, counters and ACTI schedule state, so each tree computes
-// exactly what it computes alone (impl/integrate.hpp:26-87 per tree). The trees' schedules are merged:
+// Side by side (Batch::step_side_by_side): each tree's global step is a device-resident run of its own (run.cuh), one
+// thread-block cluster, on one of 32 streams. For nine trees or more, and for fewer where no cluster has more than
+// 2048 cells.
+//
+// In lockstep, for few large trees and where the timing of stages or other stage options are asked for: one launch per
+// stage for all trees that run a level and no host synchronisation inside a global step. The trees' schedules are merged:
 // the global-step sequence counter advances with the stride of the finest level of any tree, and at
 // each sequence value a level substep runs for the trees whose schedule contains it. A tree whose
 // finest level is coarser simply has no substep at sequence values that only finer levels use, which
@@ -524,8 +529,8 @@ public:
 		}
 	}
 
-	// Planned runs, runs a check stopped, substeps planned and substeps the host completed after a stop,
-	// since the batch was made.
+	// Runs, runs that ended before the global step did, substeps planned (in lockstep) or stepped, and substeps that the
+	// host completed after a stop or issued itself, since the batch was made.
 	void run_stats(long long *out, int n) override {
 		const long long v[4] = {runs_, stops_, planned_, completed_};
 		for (int k = 0; k < n && k < 4; ++k) out[k] = v[k];
@@ -866,8 +871,8 @@ private:
 	// their own: no merged schedule, and a tree's substeps wait for no other tree's. The GPU holds nine such
 	// clusters, so this is for batches of nine trees on (24 trees of 2 to 11 thousand cells: three steps in 24 ms,
 	// in lockstep 55; 64 of up to 25 thousand: a step in 45 ms, in lockstep 190 to 390), and for fewer trees where
-	// one cluster is the shape of their runs anyway. A cluster above SIDE_CELLS is the host's, stage by stage: of 64
-	// trees with up to 256^2 base cells and 4 levels a first step took 750 ms with this limit at 2^17.
+	// one cluster is the shape of their runs anyway. A cluster above SIDE_CELLS is the host's, stage by stage, one tree after
+	// the other: ten trees of 274 thousand cells take 12 ms a step (in lockstep 24), nine of a million 35 (82).
 	static constexpr int SIDE_STREAMS = 32;
 	static constexpr int SIDE_CELLS   = Solver<M>::RUN_CELLS;
 

@@ -6,7 +6,8 @@
 // twenty stage kernels and one host synchronisation, 100 to 200 us on this GPU whatever the cluster's
 // size, while the stages' own work on a few thousand cells is a microsecond or two each. Here a barrier
 // takes the place of a launch, stages that do not read one another's results share one (six to nine
-// barriers a substep), and the host is not asked until the global step ends or something needs it.
+// barriers a substep), and the host is not asked until the global step ends or something needs it. A step with a
+// substep callback, with stage timing or with other stage options takes the launches.
 #pragma once
 
 #include "stages.cuh"
@@ -64,7 +65,7 @@ constexpr int RUN_THREADS = 512;
 
 // The warp items of a run: dealt out over the blocks one by one, so that few items spread over all SMs and the
 // cells with long walks (hanging faces, subtree means), which lie side by side in the list, do not meet in one
-// block: the slowest block ends a stage (2 to 3% on the small cases against contiguous chunks). `rev` hands
+// block: the slowest block ends a stage (2 to 3% on clusters below ten thousand cells against contiguous chunks). `rev` hands
 // the items to the blocks' warps from the last one on, for the second of two stages that share a barrier: with
 // few items the two then run on different warps instead of one after the other.
 struct DealtGrid {

@@ -241,7 +241,7 @@ __device__ __noinline__ bool mean_two_levels(const Pool &P, int n, int epoch, do
 
 // Mean primitive state and time of node n ({p[E], t} in out); `epoch` is the calling kernel's.
 // `DEEP` tries the two-level form before the general walk: shorter for the slowest lane of a run's stage, but the
-// call costs the stage launches occupancy (the indicator of drop3d_large 104 ms a step with it, 54 without).
+// call costs the stage launches occupancy (the indicator of a 64x16x16 + 4-level shock-drop 104 ms a step with it, 54 without).
 template<class M, bool DEEP>
 __device__ void interp_pt(const Pool &P, uint32_t *status, int n, int epoch, double *out) {
 	constexpr int E = M::E, NC = 1 << M::D, AW = Avg<M>::W;

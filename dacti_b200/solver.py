@@ -401,8 +401,8 @@ BATCH_STAGES = ("face_sum", "receive", "update", "slope", "aux", "estimate", "re
 
 
 def step_batches(batches) -> list:
-    """One global step of several lockstep batches at once, one host thread each (every batch has its own
-    stream, and ctypes releases the GIL during the call), so the batches' kernels overlap on the GPU.
+    """One global step of several batches at once, one host thread each (every batch has its own
+    streams, and ctypes releases the GIL during the call), so the batches' kernels overlap on the GPU.
     Returns the force_break flags of every batch's trees, batch by batch."""
     from concurrent.futures import ThreadPoolExecutor
     if len(batches) == 1:
@@ -412,11 +412,13 @@ def step_batches(batches) -> list:
 
 
 class Batch:
-    """dg_batch: independent solvers of one model stepped in lockstep, one launch per stage for all trees
-    that run a level (merged ACTI schedules). Per tree the results equal Solver.integrate's bit for bit.
-    The solvers stay usable for read-backs; step them through the batch only, and close the batch before
-    closing them. `launch` (blocks per SM per stage kind) defaults to the autotuned table of the model
-    when dacti_b200/launch_table.json has one."""
+    """dg_batch: independent solvers of one model stepped by one host thread. Nine trees or more, and fewer small
+    ones, step side by side, each tree's global step one launch; few large trees, and any batch with profiling on,
+    in lockstep, one launch per stage for all trees that run a level (merged ACTI schedules). Per tree the results
+    equal Solver.integrate's bit for bit, and side by side a tree that fails leaves the others' steps complete. The
+    solvers stay usable for read-backs; step them through the batch only, and close the batch before
+    closing them. `launch` (blocks per SM per stage kind of the lockstep) defaults to the autotuned table of the
+    model when dacti_b200/launch_table.json has one."""
 
     def __init__(self, solvers, launch=None):
         self._lib = load_library()
@@ -445,7 +447,7 @@ class Batch:
         self._bcheck(self._lib.dg_batch_set_profiling(self._h, 1 if on else 0))
 
     def stage_times(self) -> dict:
-        """{stage: (device ms, work items)} since the previous call (profiling on)."""
+        """{stage: (device ms, work items)} since the previous call (profiling on, which steps in lockstep)."""
         n = len(BATCH_STAGES)
         ms = (ctypes.c_double * n)()
         it = (ctypes.c_longlong * n)()
@@ -453,13 +455,13 @@ class Batch:
         return {k: (ms[i], it[i]) for i, k in enumerate(BATCH_STAGES)}
 
     def set_pregrow(self, on: bool = True) -> None:
-        """Grow pools ahead of each planned run (default) or only where a run stops at the capacity check."""
+        """Grow pools ahead of a step (default) or only where a run stops at the capacity check."""
         self._bcheck(self._lib.dg_batch_set_pregrow(self._h, 1 if on else 0))
 
     def run_stats(self) -> dict:
-        """Planned runs (one per global step once warmed up, unless a check stopped one), runs a check
-        stopped, substeps planned, and substeps the host completed after a stop at the capacity check,
-        since the batch was made."""
+        """Since the batch was made: runs (per tree and step side by side, for all trees in lockstep, and one more after
+        every stop), runs that ended before the global step did, substeps (`planned`: planned in lockstep, stepped
+        side by side), and substeps that the host completed after a stop at the capacity check or issued itself."""
         v = (ctypes.c_longlong * 4)()
         self._bcheck(self._lib.dg_batch_run_stats(self._h, v, 4))
         return {"runs": v[0], "stops": v[1], "planned": v[2], "completed": v[3]}

@@ -142,21 +142,26 @@ int dg_step(dg_solver *s, int signal, int *force_break, double *global_dt, dg_su
 int dg_step_many(dg_solver **solvers, int n, int threads, int signal, int *force_break, double *global_dt,
                  int *status);
 
-/* A batch of independent trees of one model, numeric form and set of viscous/tension terms, stepped in
- * lockstep by one host thread (the chosen form's batched path; no counterpart in the reference, where
- * every tree is an Integrator stepped on its own, impl/integrate.hpp:12-87). The trees' ACTI schedules
- * are merged; each substep of level L launches every stage once for all trees that run L, over block
- * ranges split among them by work. The host plans the global step and issues it with no
+/* A batch of independent trees of one model, numeric form and set of viscous/tension terms, stepped by one
+ * host thread (the chosen form's batched path; no counterpart in the reference, where every tree is an
+ * Integrator stepped on its own, impl/integrate.hpp:12-87).
+ * Nine trees or more, and fewer where no tree has a cluster above 2048 cells, step side by side: each tree's
+ * global step is one launch of one thread-block cluster on one of 32 streams, and a tree's clusters above
+ * 65536 cells are stepped stage by stage from the host.
+ * Few large trees, solvers with other stage options, and a batch with stage timing step in lockstep: the trees'
+ * ACTI schedules are merged; each substep of level L launches every stage once for all trees that run L, over
+ * block ranges split among them by work. The host plans the global step and issues it with no
  * synchronisation; each tree's schedule state lives on the device, which applies the reference's level
  * rule per tree and halts a tree with a NaN there. Device-side checks stop a run only where the live
  * counts leave the plan (a tree populating a level beyond its headroom, a pool that must grow), and the
  * host resumes from there.
- * Per tree the results are dg_step's, bit for bit. While in the batch, the solvers run on the batch's stream and keep their
- * counters in the batch's array: step them through dg_batch_step only, and destroy the batch before
+ * Per tree the results are dg_step's, bit for bit. While in the batch, the solvers run on the batch's streams and
+ * keep their counters in the batch's array: step them through dg_batch_step only, and destroy the batch before
  * its solvers. */
 typedef struct dg_batch dg_batch;
 int dg_batch_create(dg_solver **solvers, int n, dg_batch **out);
-/* One global step of every tree: force_break[k] and global_dt[k] per tree, as dg_step's. */
+/* One global step of every tree: force_break[k] and global_dt[k] per tree, as dg_step's. Side by side, an error in
+ * one tree ends that tree's step only; the others complete theirs, and the first error is returned then. */
 int dg_batch_step(dg_batch *b, int signal, int *force_break, double *global_dt);
 const char *dg_batch_last_error(dg_batch *b);
 void dg_batch_destroy(dg_batch *b);
@@ -165,17 +170,19 @@ void dg_batch_destroy(dg_batch *b);
  * multiphase auxiliary sweeps, indicator, per-cell regrid, regrid of new cells, neighbour repair,
  * buffer flush. */
 enum { DG_BATCH_STAGES = 10 };
-/* Launch budget of each stage kind in blocks per SM (1..64, default 16): a launch splits that many blocks
+/* Launch budget of each stage kind of the lockstep in blocks per SM (1..64, default 16): a launch splits that many blocks
  * among the trees in proportion to their work. What the autotuner (dacti_b200/autotune.py) sets. */
 int dg_batch_set_launch(dg_batch *b, const int *blocks_per_sm, int n_stages);
-/* Per-stage device timing with CUDA events (off by default). */
+/* Per-stage device timing with CUDA events (off by default). Steps are in lockstep while it is on. */
 int dg_batch_set_profiling(dg_batch *b, int on);
 /* Device milliseconds and work items per stage kind since the previous call. */
 int dg_batch_stage_times(dg_batch *b, double *ms, long long *items, int n_stages);
-/* Since the batch was made: out[0] planned runs, out[1] runs a check stopped, out[2] substeps planned,
- * out[3] substeps the host completed after a stop at the capacity check (n <= 4 values). */
+/* Since the batch was made (n <= 4 values): out[0] runs (one per tree and step side by side, one for all trees in
+ * lockstep, and one more after every stop), out[1] runs that ended before the global step did (a check, a cluster above
+ * the run's limit; side by side also a tree that reached a NaN), out[2] substeps, planned ones in lockstep, out[3]
+ * substeps that the host completed after a stop at the capacity check or, side by side, issued itself. */
 int dg_batch_run_stats(dg_batch *b, long long *out, int n);
-/* Pools grown ahead of each planned run when less than a fifth of the tree is free, to half the tree
+/* Pools grown ahead of each global step (each planned run in lockstep) when less than a fifth of the tree is free, to half the tree
  * again (on by default; capacity never changes a result). Off, a pool grows only where a run stops at
  * the capacity check. */
 int dg_batch_set_pregrow(dg_batch *b, int on);
