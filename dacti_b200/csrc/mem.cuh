@@ -171,14 +171,15 @@ inline size_t mem_unused() {
 	std::lock_guard<std::mutex> l(DeviceMemory::lock());
 	return (reserved > used ? (size_t) (reserved - used) : 0) + d->retired_bytes;
 }
-// Whether more than half of the device's memory is in use by solvers.
-inline bool mem_tight() {
+// Whether more than half of the device's memory is in use by solvers, or would nearly be (45%) with `more`: what is taken
+// below the one line is not given up again at once above the other.
+inline bool mem_tight(size_t more = 0) {
 	cudaError_t e;
 	DeviceMemory *d = DeviceMemory::of_device(e);
 	if (!d) return true;
 	const size_t used = d->pool_in_use();
 	std::lock_guard<std::mutex> l(DeviceMemory::lock());
-	return used + d->large_bytes > d->total / 2;
+	return used + d->large_bytes + more > (more > 0 ? d->total / 20 * 9 : d->total / 2);
 }
 // A user of the current device's memory, as long as it lives.
 class MemoryUser {

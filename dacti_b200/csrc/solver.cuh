@@ -338,7 +338,7 @@ public:
 		size_t field = 0;
 		for (auto &f: fields(P_)) field = std::max(field, field_bytes(f, P_.cap));
 		const size_t whole = pool_bytes(P_);
-		const bool two     = whole <= SECOND_POOL_MAX && !spare_small_ && !mem_tight();
+		const bool two     = whole <= SECOND_POOL_MAX && !spare_small_ && !mem_tight(spare_bytes_ >= whole ? 0 : whole);
 		if (spare_mem_ && spare_bytes_ >= (two ? whole : field) && (two || spare_bytes_ < whole)) return;
 		mem_free(spare_mem_, st_);
 		spare_mem_    = nullptr;
